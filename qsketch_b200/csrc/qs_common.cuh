@@ -22,33 +22,28 @@ constexpr uint32_t ST_TIMEOUT = 2u;
 constexpr uint32_t ST_CAPACITY = 4u;
 constexpr uint32_t ST_BAD_OFFSETS = 8u;  // batched streams: offsets not non-decreasing from 0
 
-// Lemire-Kaser-Kurz direct remainder ("Faster Remainder by Direct Computation", 2019):
-// for d < 2^32 and M = ceil(2^64 / d), a % d == mulhi64(M * a mod 2^64, d) for all
-// 32-bit a.  Replaces the two run-time `%` of device_sketch_v3.h:42-44 per key.
+// a % d by a 32-bit reciprocal (in place of the two run-time `%` of device_sketch_v3.h:42-44 per
+// key).  With M = floor(2^32 / d), q = (a * M) >> 32 is floor(a / d) or one less for every 32-bit
+// a: a / d - a * M / 2^32 = a * (2^32 / d - M) / 2^32 < 1.  So r = a - q * d lies in [0, 2d) and
+// one conditional subtraction (min(r, r - d) in unsigned arithmetic: r - d wraps when r < d)
+// finishes: a high multiply, a multiply-add, an add and a min, where the 64-bit direct
+// remainder (Lemire, Kaser, Kurz 2019) takes two 32-bit wide and two high multiplies.
 struct FastMod {
-    uint64_t M;
-    uint32_t d;
-    uint32_t pad;
+    uint32_t M, d;
 };
 
 inline FastMod make_fastmod(uint32_t d) {
     FastMod f;
-    f.M = (d == 0) ? 0 : (~0ull / d + 1ull);  // d == 1 wraps to 0: a % 1 == 0 below too
+    f.M = d < 2 ? 0xffffffffu : (uint32_t)((1ull << 32) / d);  // d = 1: q = a - 1 (a > 0), r = 1 -> 0
     f.d = d;
-    f.pad = 0;
     return f;
 }
 
 __host__ __device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 
-// a % d as Lemire's direct remainder: low = M * a mod 2^64, a % d = (low * d) >> 64.  With d
-// below 2^32 the 128-bit product's high word is (hi * d + mulhi(lo, d)) >> 32 for the 32-bit
-// halves hi, lo of low (the fractional part lo * d mod 2^32 cannot carry into it): two
-// 32-bit wide multiplies and one high multiply instead of a 64 x 64 product.
 __device__ __forceinline__ uint32_t fast_mod(const FastMod& f, uint32_t a) {
-    const uint64_t low = f.M * (uint64_t)a;
-    const uint32_t lo = (uint32_t)low, hi = (uint32_t)(low >> 32);
-    return (uint32_t)(((uint64_t)hi * f.d + __umulhi(lo, f.d)) >> 32);
+    const uint32_t r = a - __umulhi(a, f.M) * f.d;
+    return min(r, r - f.d);
 }
 
 // Per-sketch device control block.

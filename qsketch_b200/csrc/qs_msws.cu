@@ -690,7 +690,7 @@ struct KeyMap {
         }
         const StreamDesc* sd = B.desc + s;
         hv = key * __ldg(&sd->seed);
-        const FastMod fm{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d), 0u};
+        const FastMod fm{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d)};
         return __ldg(&sd->low_base) + fast_mod(fm, hv);
     }
 };
@@ -2003,7 +2003,7 @@ __global__ void __launch_bounds__(INS_THREADS, INS_MIN_CTAS) k_batch_insert(cons
         const uint32_t it_local = s_item;
         const StreamDesc* sd = B.desc + s;
         const uint32_t seed = __ldg(&sd->seed), base = __ldg(&sd->low_base);
-        const FastMod fm{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d), 0u};
+        const FastMod fm{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d)};
         const uint64_t t0 = __ldcg(B.lo + s) + (uint64_t)it_local * INS_TILE;
         const int cnt = (int)umin64(INS_TILE, __ldcg(B.hi + s) - t0);
         const int route = (int)S.misc[2];
@@ -2040,7 +2040,7 @@ __global__ void __launch_bounds__(QRY_THREADS) k_batch_query(const uint32_t* __r
         __syncthreads();
         const StreamDesc* sd = B.desc + s;
         const uint32_t seed = __ldg(&sd->seed), base = __ldg(&sd->low_base);
-        const FastMod fm{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d), 0u};
+        const FastMod fm{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d)};
         const uint64_t t0 = __ldcg(B.lo + s) + (uint64_t)(it - __ldcg(B.item_off + s)) * INS_TILE;
         const uint32_t cnt = (uint32_t)umin64(INS_TILE, __ldcg(B.hi + s) - t0);
         constexpr int PER = INS_TILE / QRY_THREADS;
