@@ -100,7 +100,10 @@ typedef struct qs_params {
     uint64_t max_batch;          /* keys per internal insert chunk (scratch sizing);
                                     a multiple of 32, at most 2^26; 0 = 1<<22 */
     int32_t device;              /* CUDA device ordinal; -1 = current */
-    /* Insert-kernel knobs; none changes any result.  When lanes_per_key, aggregate, route
+    /* Insert-kernel knobs; none changes any result.  They shape pass 1, which takes the calls
+     * that are small against the table; with all of them (and QS_FLAG_NO_CHUNK_RAMP) left at 0,
+     * calls of at least max(2^18, 1.5 n_low) keys are partitioned by bucket range and applied in
+     * shared memory instead, in chunks of up to 4 * max_batch keys.  When lanes_per_key, aggregate, route
      * and ctas_per_sm are all 0, qs_create takes them (and max_batch, if 0) from the
      * autotuner's entry for the sketch's size class (qs_autotune), else the defaults
      * 4 / 3 / 1 / 0. */

@@ -101,6 +101,10 @@ struct qs_sketch {
     std::vector<void*> allocs;
     MswsDev D{};
     MswsLaunch L{};
+    PartDev P{};              // partitioned insert: its scratch (P.parts == 0: not used)
+    PartLaunch PL{};
+    uint64_t part_cap = 0;    // keys a partitioned chunk takes
+    uint64_t part_min = 0;    // and the fewest it pays for
     CmDev C{};
     int cm_grid = 0;
     // host-buffer pipeline
@@ -229,6 +233,18 @@ qs_status setup_io(qs_sketch* sk) {
     return QS_OK;
 }
 
+// Keys of the next partitioned chunk when `rest` remain: even chunks of at most part_cap keys, in
+// whole tiles; after a create or clear a short one first, so that the buckets of heavy keys
+// are linked before their keys come in large runs to one block (2^27 Zipf 1.1 keys without it:
+// one block applies a tenth of a 2^24-key chunk in order, 1.3 ms where the others take 0.15).
+uint64_t part_chunk(const qs_sketch* sk, uint64_t rest) {
+    const uint64_t first = std::min<uint64_t>(1ull << 18, sk->part_cap);
+    if (sk->fresh < first && rest >= 3 * first) return first;
+    const uint64_t k = (rest + sk->part_cap - 1) / sk->part_cap;
+    const uint64_t c = ((rest + k - 1) / k + PART_TILE - 1) / PART_TILE * PART_TILE;
+    return std::min(rest, c);
+}
+
 // skip: optional bitmap over the keys (bit set = the key is not for this sketch); chunk
 // offsets are multiples of max_batch, itself a multiple of 32.
 // table (learned split, optional): pass 1 looks keys up in this exact table itself, counts the
@@ -237,7 +253,25 @@ qs_status setup_io(qs_sketch* sk) {
 qs_status insert_device(qs_sketch* sk, const uint32_t* d_keys, size_t n, cudaStream_t st,
                         const uint32_t* skip = nullptr, const TableDev* table = nullptr, uint32_t* skipbuf = nullptr) {
     if (sk->kind == QS_KIND_MSWS) {
+        bool hot = false;  // the call's heavy keys are sampled
         for (size_t off = 0; off < n;) {
+            if (sk->P.parts && !table && n >= sk->part_min) {
+                const uint64_t c = part_chunk(sk, n - off);
+                MswsDev D = sk->D;
+                D.skip = skip ? skip + off / 32 : nullptr;
+                CK(sk->prof_begin(0, st), "profile");
+                if (!hot && sk->fresh && n - off >= PART_HOT_MIN) {
+                    CK(part_hot(d_keys + off, n - off, sk->P, st), "heavy keys");
+                    ++sk->launches[0];
+                    hot = true;
+                }
+                CK(part_insert(d_keys + off, c, D, sk->P, sk->PL, hot, st), "partitioned insert");
+                CK(sk->prof_end(0, st), "profile");
+                sk->launches[0] += 2;  // three kernels, one timed interval
+                off += c;
+                sk->fresh += c;
+                continue;
+            }
             uint64_t c = std::min<uint64_t>(sk->max_batch, n - off);
             // after a create or clear the chunks grow geometrically from ramp_first keys, so
             // the buckets of heavy keys link in a small first chunk (sizes stay multiples of 32)
@@ -450,7 +484,26 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         D.compat_v3 = (p.flags & QS_FLAG_COMPAT_V3) ? 1u : 0u;
         D.route = route == 3 ? 0u : route;  // 0 in the kernel = adaptive per tile
         const uint64_t B = sk->max_batch;
-        const uint64_t cap = std::min<uint64_t>(n_low, B);
+        // the partitioned insert (qs_part.cu) takes the large chunks of a sketch whose pass-1
+        // knobs are left to the library
+        const bool own_knobs = p.lanes_per_key || p.aggregate || p.route || p.ctas_per_sm || p.keys_per_tile ||
+                               (p.flags & QS_FLAG_NO_CHUNK_RAMP);
+        PartDev& P = sk->P;
+        P.shift = PART_MIN_SHIFT;
+        while (P.shift < PART_MAX_SHIFT && (n_low >> P.shift) >= 640) ++P.shift;
+        const uint64_t parts = (n_low + (1ull << P.shift) - 1) >> P.shift;
+        if (!own_knobs && B >= PART_TILE && parts >= 8 && parts <= PART_MAX_PARTS && H <= PART_MAX_MASKS &&
+            p.n_high < (1ull << 28))
+            P.parts = (uint32_t)parts;
+        sk->part_cap = std::min<uint64_t>(B * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE;
+        // A partitioned chunk streams the whole table through shared memory (64 MB: 45 us), pass 1
+        // touches the buckets of its keys only.  Per call, measured: 2^18 Zipf 1.1 keys into a 4 MB
+        // table 48 us against 80 (uniform 22 against 19), 2^20 117 against 137 (38 / 45), 2^22 136
+        // against 269 (85 / 139); 2^22 keys into 64 MB 168 against 273 (124 / 145), but 2^20 174
+        // against 141 (73 / 49).
+        sk->part_min = std::max<uint64_t>(1ull << 18, n_low + n_low / 2);
+        const uint64_t reach = P.parts ? std::max(B, sk->part_cap) : B;  // keys of the largest chunk
+        const uint64_t cap = std::min<uint64_t>(n_low, reach);
         D.flag_cap = (uint32_t)cap;
         D.max_tiles = (uint32_t)((B + REPAIR_TILE - 1) / REPAIR_TILE);
         D.long_cap = (uint32_t)std::min<uint64_t>(cap, 1ull << 16);  // slots with grid-computed totals
@@ -462,23 +515,41 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         CKB(sk->alloc(&D.ctl, 1), "alloc control");
         CKB(sk->alloc(&D.flag_list, cap), "alloc flag list");
         CKB(sk->alloc(&D.tile_counts, D.max_tiles), "alloc tile counts");
-        CKB(sk->alloc(&D.rec[0], B), "alloc records");
-        CKB(sk->alloc(&D.rec[1], B), "alloc records");
+        // one block: the replay's records and their positions (24 B per key of max_batch), or a
+        // partitioned chunk's entries and key indices (6 B per key of up to 4 max_batch)
+        uint32_t* rb = nullptr;
+        CKB(sk->alloc(&rb, B * 6), "alloc records");
+        D.rec[0] = reinterpret_cast<uint2*>(rb);
+        D.rec[1] = reinterpret_cast<uint2*>(rb + 2 * B);
+        D.rpos[0] = rb + 4 * B;
+        D.rpos[1] = rb + 5 * B;
+        if (P.parts) {
+            P.ent = rb;
+            P.idx = reinterpret_cast<uint16_t*>(rb + sk->part_cap);
+            // tiles of a chunk: whole ones, or the small ones of a chunk below PART_SMALL_MAX keys
+            P.stride = (uint32_t)std::max(sk->part_cap / PART_TILE,
+                                          std::min(sk->part_cap, PART_SMALL_MAX) / PART_TILE_SMALL);
+            CKB(sk->alloc(&P.hot, PART_HOT), "alloc heavy keys");
+            CKB(sk->alloc(&P.off, (uint64_t)(P.parts + 1) * P.stride), "alloc run bounds");
+        }
         CKB(sk->alloc(&D.hist, (uint64_t)256 * D.max_tiles + 256), "alloc histograms");  // + digit totals
         CKB(sk->alloc(&D.seg_beg, cap), "alloc segments");
         CKB(sk->alloc(&D.totals, (uint64_t)D.long_cap * LOW_COUNTERS), "alloc totals");
-        CKB(sk->alloc(&D.rpos[0], B), "alloc record positions");
-        CKB(sk->alloc(&D.rpos[1], B), "alloc record positions");
         CKB(sk->alloc(&D.sw, cap), "alloc link order");
         CKB(sk->alloc(&D.sw_base, cap), "alloc link order");
-        CKB(sk->alloc(&D.sw_bits, (B + 31) / 32), "alloc link order");
-        CKB(sk->alloc(&D.sw_cnt, (B + SW_BLOCK - 1) / SW_BLOCK), "alloc link order");
+        CKB(sk->alloc(&D.sw_bits, (reach + 31) / 32), "alloc link order");
+        CKB(sk->alloc(&D.sw_cnt, (reach + SW_BLOCK - 1) / SW_BLOCK), "alloc link order");
         CKB(cudaMemcpy(masks_d, sk->masks.data(), (size_t)H * 4, cudaMemcpyHostToDevice), "upload masks");
         qs_status s = ctl_reset(sk, 0);
         if (s != QS_OK) return bail(s);
         CKB(cudaStreamSynchronize(0), "create sync");
         e = msws_configure(dev, H, &sk->L);
         if (e != cudaSuccess) return bail(cuda_fail(e, "configure kernels"));
+        if (P.parts) {
+            e = part_configure(&sk->PL, P.shift, P.parts, H, sk->L.num_sms);
+            if (e != cudaSuccess) return bail(cuda_fail(e, "configure partitioned insert"));
+            for (uint32_t m : sk->masks) sk->PL.wide |= __builtin_popcount(m) != 3;
+        }
         sk->L.lanes_per_key = (int)lpk;
         sk->L.tile_keys = (int)tile;
         sk->L.ctas_per_sm = tuned ? (int)tc.ctas_per_sm : (int)p.ctas_per_sm;

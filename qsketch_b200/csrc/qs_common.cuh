@@ -56,6 +56,8 @@ struct Ctl {
     uint32_t bar_count;    // blocks that finished the current repair (its last block resets)
     uint32_t link_gen;     // repairs that linked buckets since the create/clear (never reset
                            // otherwise): tags the per-stream link ranks of batched streams
+    uint32_t n_switch;     // partitioned insert: buckets that switched in the current chunk
+    uint32_t link_base;    // and the allocator when the chunk began
     unsigned long long bar_arrive;  // grid barrier arrivals (a barrier ends at the next multiple
                                     // of the grid size)
     unsigned long long dropped;
@@ -111,6 +113,28 @@ struct MswsDev {
     uint32_t* sw_cnt;        // switches per SW_BLOCK positions
 };
 constexpr uint32_t SW_BLOCK = 4096;  // positions per switch count (128 bit words)
+
+// Scratch of the partitioned insert (qs_part.cu); its tiles share the memory of the ordered
+// replay's records.
+struct PartDev {
+    uint32_t* ent;    // entries, each tile's at its own place, ordered by partition
+    uint16_t* idx;    // each entry's key: its index in the tile
+    uint16_t* off;    // [parts + 1][stride] first entry of each partition's run in each tile
+    uint32_t* hot;    // [PART_HOT] the current call's heavy keys, two per set
+    uint32_t stride;  // tiles a chunk can have
+    uint32_t shift;   // a partition is 2^shift consecutive buckets
+    uint32_t parts;
+    uint32_t tiles;   // this chunk's tiles, of `tile` keys
+    uint32_t tile;
+    uint32_t mean;    // entries per run when they spread evenly
+};
+constexpr uint32_t PART_TILE = 16384, PART_TILE_SMALL = 2048;
+constexpr uint64_t PART_SMALL_MAX = 148ull * PART_TILE;  // chunks below this many keys take small tiles
+constexpr uint32_t PART_MAX_PARTS = 2048, PART_MIN_SHIFT = 6, PART_MAX_SHIFT = 11;
+constexpr uint32_t PART_MAX_MASKS = 2048;         // mask tables the apply step keeps in shared memory
+constexpr uint64_t PART_MAX_CHUNK = 1ull << 26;
+constexpr uint32_t PART_HOT = 2048;               // heavy keys of a call
+constexpr uint64_t PART_HOT_MIN = 1ull << 21;      // calls of at least this many keys are sampled for them
 
 // Batched streams: many per-stream MSWS sketches share one low-table arena and one high
 // pool arena.  A stream's sketch is the bucket range [low_base, low_base + fm_low.d) of the

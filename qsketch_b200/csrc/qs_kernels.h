@@ -40,6 +40,18 @@ cudaError_t msws_repair(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
 cudaError_t msws_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, const MswsDev& D, const MswsLaunch& L,
                        cudaStream_t st);
 
+// Partitioned insert (qs_part.cu) of one chunk: split, apply, link.
+struct PartLaunch {
+    int num_sms = 0;
+    size_t apply_smem = 0;
+    bool wide = false;  // some mask does not select exactly three counters
+};
+// The call's heavy keys (a sample of its n keys) into part.hot, for part_insert's `hot`.
+cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cudaStream_t st);
+cudaError_t part_configure(PartLaunch* L, uint32_t shift, uint32_t parts, uint32_t n_masks, int num_sms);
+cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
+                        bool hot, cudaStream_t st);
+
 cudaError_t cm_insert(const uint32_t* d_keys, uint64_t n, const CmDev& D, int agg, int grid, cudaStream_t st);
 // REMOVE (qs_remove.cu): one occurrence of each key out, counters floored at 0.
 cudaError_t msws_remove(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const MswsLaunch& L, cudaStream_t st);

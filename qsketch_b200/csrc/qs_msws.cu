@@ -20,6 +20,7 @@
 //      moves the increments of that key and all later ones to the new high bucket.
 #include "qs_device.cuh"
 #include "qs_kernels.h"
+#include "qs_replay.cuh"
 
 namespace qsb {
 
@@ -111,10 +112,6 @@ __device__ __forceinline__ void flag_bucket(const MswsDev& D, uint32_t b) {
     }
 }
 
-__device__ __forceinline__ bool is_linked(const MswsDev& D, uint32_t w7) {
-    return w7 > START && (uint64_t)(w7 - START) < D.n_high;
-}
-
 __device__ __forceinline__ bool agg_insert(const InsShared& S, uint32_t key, uint32_t c, uint32_t id) {
     if (key == AGG_EMPTY) return false;
     const uint32_t h = (key * 0x9E3779B1u) >> 22;  // 10 bits
@@ -140,18 +137,6 @@ __device__ __forceinline__ bool agg_insert(const InsShared& S, uint32_t key, uin
         }
     }
     return false;
-}
-
-// Does a selected byte (nibble bit k selects byte k) of the pre-add word `old` reach CROSS
-// once c is added: byte + c >= CROSS, i.e. byte >= CROSS - c, four bytes at a time.
-// Selected bytes all below 64 with c below 64 cannot reach CROSS: a two-operation test
-// settles the common case before the four-byte comparison.
-__device__ __forceinline__ bool crosses(uint32_t old, uint32_t nib, uint32_t c) {
-    if (!nib) return false;
-    if (c >= CROSS) return true;
-    const uint32_t sel = expand_nibble(nib) * 0xffu;
-    if (c < 64u && !(old & sel & 0xC0C0C0C0u)) return false;
-    return (__vcmpgeu4(old, (CROSS - c) * 0x01010101u) & sel) != 0u;
 }
 
 // One lane, one key (or merged count c of one key) of an unlinked bucket: the selected 8-bit
@@ -572,7 +557,6 @@ constexpr uint32_t SEMI_TILES = 4;  // radix tiles per block kept as offsets and
 static_assert(SEMI_TILES * (REPAIR_THREADS / 32) * 256 * 2 + SEMI_TILES * REPAIR_TILE <= SET_SLOTS * 4,
               "the offsets and ranks of SEMI_TILES tiles fit the shared space");
 constexpr uint32_t SCAN_CAP = SET_SLOTS / 2;  // records replayed without a sort (64 KiB of uint2)
-constexpr uint32_t NONE = 0xffffffffu;
 
 __device__ __forceinline__ int radix_passes(uint32_t F) {
     if (F <= 1) return 0;
@@ -751,19 +735,6 @@ __device__ __forceinline__ void tile_count(RadixSmem& rs, const uint2 (&rec)[TIL
 // selected counter above LIMIT is found (the low->high switch of :160-190), the bucket is
 // linked there (atomic_malloc, :69-85) and that key and all later ones count high.
 
-// Occurrences of counter c (lane c) among the 32 masks of the warp: seven warp sums of the
-// masks expanded to one byte per counter (a byte counts at most 32, so no carries).
-__device__ __forceinline__ uint32_t group_counts(uint32_t m) {
-    const int lane = threadIdx.x & 31;
-    uint32_t mine = 0;
-#pragma unroll
-    for (int w = 0; w < 7; ++w) {
-        const uint32_t t = __reduce_add_sync(0xffffffffu, expand_nibble((m >> (4 * w)) & 0xfu));
-        if ((lane >> 2) == w) mine = t;
-    }
-    return lane < LOW_COUNTERS ? (mine >> (8 * (lane & 3))) & 0xffu : 0u;
-}
-
 // Lane c accumulates the occurrences of counter c among the 32 masks of the warp.
 __device__ __forceinline__ void count_counters(uint32_t m, uint32_t& T) { T += group_counts(m); }
 
@@ -776,67 +747,6 @@ __device__ __forceinline__ uint32_t pre_counters(const uint32_t* wp, uint32_t T)
     for (int k = 0; k < 4; ++k) sw += __shfl_sync(0xffffffffu, T, (4 * (lane & 7) + k) & 31) << (8 * k);
     const uint32_t pwi = __shfl_sync(0xffffffffu, fw - sw, (lane >> 2) & 7);
     return lane < LOW_COUNTERS ? (pwi >> (8 * (lane & 3))) & 0xffu : 0u;
-}
-
-// 32 consecutive records (mask m, 0 for lanes that are not this bucket's): returns the lane
-// of the first record that sees a selected counter above LIMIT, or -1; `cur` advances over
-// the records before it (all 32 when none triggers).
-__device__ __forceinline__ int link_step(uint32_t m, uint32_t& cur) {
-    const int lane = threadIdx.x & 31;
-    // The last record with counter c sees cur + (occurrences - 1): when that stays within
-    // LIMIT for every counter, no record of the group switches.
-    const uint32_t tot = group_counts(m);
-    if (!__any_sync(0xffffffffu, tot && cur + tot > LIMIT + 1)) {
-        cur += tot;
-        return -1;
-    }
-    const uint32_t lt = lanemask_lt();
-    bool trig = false;
-    uint32_t inc = 0;
-#pragma unroll
-    for (int c = 0; c < LOW_COUNTERS; ++c) {
-        const uint32_t bal = __ballot_sync(0xffffffffu, (m >> c) & 1u);
-        const uint32_t cc = __shfl_sync(0xffffffffu, cur, c);
-        if (((m >> c) & 1u) && cc + __popc(bal & lt) > LIMIT) trig = true;
-        if (lane == c) inc = __popc(bal);
-    }
-    const uint32_t tb = __ballot_sync(0xffffffffu, trig);
-    if (!tb) {
-        cur += inc;
-        return -1;
-    }
-    const int j = __ffs(tb) - 1;
-    const uint32_t before = (1u << j) - 1u;
-#pragma unroll
-    for (int c = 0; c < LOW_COUNTERS; ++c) {
-        const uint32_t bal = __ballot_sync(0xffffffffu, (m >> c) & 1u);
-        if (lane == c) cur += __popc(bal & before);
-    }
-    return j;
-}
-
-// Where the replay of one flagged bucket ended (per lane c: counter c).
-struct ReplayOut {
-    bool found;        // a key switched the bucket to the high level
-    uint32_t L;        // that key's record: index into the records the replay read
-    uint32_t n_after;  // the bucket's keys at or after the switch
-    uint32_t n_total;  // the bucket's keys in the chunk
-    uint32_t T;        // the chunk's increments of counter c
-    uint32_t P;        // counter c before the chunk
-    uint32_t cur;      // counter c when the switch happens (final low value)
-    uint32_t mL;       // the switching key's mask
-};
-
-// Increments of high counter `lane` in the new high bucket: the switching key's and all
-// later keys'.
-__device__ __forceinline__ uint32_t high_increments(const MswsDev& D, const ReplayOut& o) {
-    const int lane = threadIdx.x & 31;
-    uint32_t H = o.T - (o.cur - o.P);
-    if (D.compat_v3) {  // device_sketch_v3.h:187: the switching key lands on bit % 8
-        if (lane < LOW_COUNTERS && ((o.mL >> lane) & 1u)) H -= 1u;
-        if (lane < 8) H += __popc(o.mL & (0x01010101u << lane));
-    }
-    return H;
 }
 
 // The low counters at the switch, packed back into words 0..6 of bucket b.
@@ -975,36 +885,6 @@ __device__ __forceinline__ void settle_bucket(const MswsDev& D, const BatchDev& 
         atomicAdd(&D.ctl->repaired_buckets, 1ull);
         atomicAdd(&D.ctl->repaired_keys, (unsigned long long)o.n_total);
     }
-}
-
-// Link bucket b to high id `id` (global; ok: inside the pool) with high increments H, or
-// saturate it when the pool has run out (its n_after keys are dropped).
-__device__ __forceinline__ void link_bucket(const MswsDev& D, uint32_t b, uint32_t id, bool ok, uint32_t H,
-                                            uint32_t n_after) {
-    const int lane = threadIdx.x & 31;
-    if (ok) {
-        __stcg(D.high + (uint64_t)(id - START) * HIGH_WORDS + lane, H);
-    } else if (lane == 0) {
-        atomicOr(&D.ctl->status, ST_POOL_FULL);
-        atomicAdd(&D.ctl->dropped, (unsigned long long)n_after);
-    }
-    if (lane == 7) __stcg(D.low + (uint64_t)b * LOW_WORDS + 7, ok ? id : SATURATED);
-}
-
-// Rank of switch position p among all switch positions of the chunk (the result in every
-// lane): the exclusive prefix `spre` of the per-SW_BLOCK counts, plus the set bits before p
-// in its block of 128 words.
-__device__ __forceinline__ uint32_t switch_rank(const MswsDev& D, const uint32_t* spre, uint32_t p) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t q = p / SW_BLOCK, w = p >> 5;
-    uint32_t c = 0;
-#pragma unroll
-    for (int k = 0; k < (int)(SW_BLOCK / 32 / 32); ++k) {
-        const uint32_t wi = q * (SW_BLOCK / 32) + k * 32 + lane;
-        if (wi < w) c += __popc(__ldcg(D.sw_bits + wi));
-    }
-    if (lane == 0) c += __popc(__ldcg(D.sw_bits + w) & ((1u << (p & 31)) - 1u));
-    return spre[q] + __reduce_add_sync(0xffffffffu, c);
 }
 
 // The same rank in a chunk of at most SCAN_CAP records: the set bits of all switch words

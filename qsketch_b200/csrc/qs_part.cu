@@ -1,0 +1,960 @@
+// qs_part.cu — the partitioned MSWS insert: large chunks, bucket by bucket in shared memory.
+//
+// Pass 1 of qs_msws.cu sends every key to its bucket in L2 with returning atomics and merges
+// equal keys of a warp first (__match_any_sync: 64 SM cycles for 32 distinct values); the
+// ordered replay then reads the whole chunk again to find the keys of the buckets that
+// crossed.  A chunk with enough keys per bucket is instead split by bucket range:
+//   1. k_part_split: tiles of the chunk are ordered by partition (2^shift consecutive buckets)
+//      in shared memory and written out with each key's index in its tile.  An entry is the
+//      bucket within the partition and the number of the key's mask; nothing is hashed again.
+//   2. k_part_apply: one block per partition holds the partition's 32-byte buckets in shared
+//      memory and applies the entries tile by tile with shared-memory atomics.  A bucket whose
+//      selected counter would pass the threshold is replayed on the spot: the entries of the
+//      flagged buckets in the current run of tiles are sorted by array position and the exact
+//      sequential rule of qs_replay.cuh finds the switching key.  The new high bucket is a
+//      temporary row; the index word names it until the link order is known.
+//   3. k_part_link: high ids in the array order of the switching keys, as one-key-at-a-time
+//      insertion hands them out; rows move to their high buckets.
+// Nothing waits across blocks: the order between the steps is the order of the launches.
+//
+// What bounds it (2^24-key chunks): the split, instruction issue (84 warp instructions and 11
+// shared-memory passes per 32 keys; 82 us); the apply step, the latency of a unit's dependent
+// shared-memory steps with 32 warps an SM (95 us for uniform keys, 155 us for Zipf 1.1 with the
+// heavy keys counted in the split).  Against pass 1 and the replay: 2^24 uniform keys into 8 MB
+// 0.55 -> 0.22 ms, 2^27 Zipf 1.1 keys into 64 MB 6.4 -> 2.2 ms (both with default knobs).
+#include "qs_kernels.h"
+#include "qs_replay.cuh"
+
+namespace qsb {
+
+constexpr int AP_THREADS = 512;
+constexpr int AP_WARPS = AP_THREADS / 32;
+constexpr uint32_t AP_TILES = AP_THREADS;   // tiles whose run bounds are staged at a time
+// A unit: the entries applied between two looks at the flagged buckets (whole runs; a longer run is
+// a unit of its own).  A thread holds its share of the unit in registers, so the records of the
+// flagged buckets are gathered without reading the entries again, and always fit the
+// shared memory they are sorted in.  Half the size beside the 2048-bucket partitions of the
+// largest tables, so that two blocks fit an SM.
+__host__ __device__ constexpr uint32_t ap_unit(uint32_t shift) { return shift > 10 ? 2048u : 4096u; }
+// A partition that gets far more than its share starts with short units, doubling: the buckets of
+// its heavy keys link in them, with few records each.
+constexpr uint32_t AP_FIRST = 256;
+constexpr uint32_t ENT_MASK_BITS = 14;      // entry = bucket in partition << 14 | mask number
+constexpr uint32_t ENT_MASK = (1u << ENT_MASK_BITS) - 1u;
+// Index words while a partition is in shared memory, beside 0, FLAG | slot and real ids (below
+// ACC: the path takes pools of less than 2^28 buckets):
+//   ACC | a        linked; its high increments collect in row a of the block's accumulators
+//   ACC | NEW | a  the same for a bucket linked in this chunk, whose id is not known yet
+//   TEMP | row     linked in this chunk with no accumulator left: a row in global memory
+//                  (TEMP_NOROW: no row left either, counted again when the id is known)
+constexpr uint32_t ACC = 0x20000000u, NEW = 0x10000000u, TEMP = 0x40000000u;
+constexpr uint32_t TEMP_NOROW = 0x7fffffffu;
+constexpr uint32_t ACC_WORDS = LOW_COUNTERS + 1;  // 28 counters and the keys of a NEW bucket
+// Accumulator rows of a block: the linked buckets of a partition, a few per cent of its buckets.
+__host__ __device__ constexpr uint32_t ap_accs(uint32_t shift) { return shift > 10 ? 80u : 192u; }
+// ---- 0: the heavy keys of a call ---------------------------------------------------------
+
+constexpr uint32_t HOT_SETS = PART_HOT / 2;  // two keys per set
+constexpr uint32_t HOT_BLOCKS = 16, HOT_THREADS = 512;
+constexpr uint32_t HOT_SAMPLES = 16384, HOT_SLOTS = 2048, HOT_MIN = 3;
+constexpr uint32_t HOT_EMPTY = 0xffffffffu;
+
+__device__ __forceinline__ uint32_t hot_set(uint32_t key) { return (key * 0x9E3779B1u) >> 22; }
+static_assert(HOT_SETS == 1024, "hot_set yields 10 bits");
+
+// Keys seen at least HOT_MIN times among HOT_SAMPLES evenly spaced ones (a share of about 2e-4).
+// Every block reads the whole sample and counts the keys of its own sets: one block's atomics on
+// one SM take 28 us, sixteen blocks' a quarter of it.  Which keys the table keeps when a set
+// overflows (the heaviest go first) does not change any result.
+__global__ void __launch_bounds__(HOT_THREADS) k_part_hot(const uint32_t* __restrict__ keys, uint64_t n, uint32_t* hot) {
+    __shared__ uint32_t s_key[HOT_SLOTS], s_cnt[HOT_SLOTS];
+    constexpr uint32_t SETS = HOT_SETS / HOT_BLOCKS;  // this block's sets
+    __shared__ uint32_t s_hot[2 * SETS];
+    const uint32_t tid = threadIdx.x, set0 = blockIdx.x * SETS;
+    for (uint32_t i = tid; i < HOT_SLOTS; i += HOT_THREADS) s_key[i] = HOT_EMPTY, s_cnt[i] = 0u;
+    for (uint32_t i = tid; i < 2 * SETS; i += HOT_THREADS) s_hot[i] = HOT_EMPTY;
+    const uint64_t step = n / HOT_SAMPLES;
+    uint32_t k[HOT_SAMPLES / HOT_THREADS];
+#pragma unroll
+    for (uint32_t j = 0; j < HOT_SAMPLES / HOT_THREADS; ++j)
+        k[j] = __ldg(keys + step * (uint64_t)(j * HOT_THREADS + tid));
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < HOT_SAMPLES / HOT_THREADS; ++j) {
+        if (k[j] == HOT_EMPTY || hot_set(k[j]) - set0 >= SETS) continue;
+        const uint32_t h = mix32(k[j]);
+        for (uint32_t q = 0; q < 8; ++q) {  // a heavy key finds a slot early; a lone one may be left out
+            const uint32_t s = (h + q) & (HOT_SLOTS - 1);
+            uint32_t seen = reinterpret_cast<volatile uint32_t*>(s_key)[s];
+            if (seen == HOT_EMPTY) seen = atomicCAS(s_key + s, HOT_EMPTY, k[j]);
+            if (seen == HOT_EMPTY || seen == k[j]) {
+                atomicAdd(s_cnt + s, 1u);
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    uint32_t hi = 0xffffffffu;
+    for (uint32_t lo : {64u, 8u, HOT_MIN}) {  // the heaviest first
+        for (uint32_t i = tid; i < HOT_SLOTS; i += HOT_THREADS) {
+            if (s_cnt[i] < lo || s_cnt[i] >= hi) continue;
+            const uint32_t s = 2 * (hot_set(s_key[i]) - set0);
+            if (atomicCAS(s_hot + s, HOT_EMPTY, s_key[i]) != HOT_EMPTY) atomicCAS(s_hot + s + 1, HOT_EMPTY, s_key[i]);
+        }
+        hi = lo;
+        __syncthreads();
+    }
+    for (uint32_t i = tid; i < 2 * SETS; i += HOT_THREADS) hot[2 * set0 + i] = s_hot[i];
+}
+
+// ---- 1: tiles ordered by partition ---------------------------------------------------------
+
+// HOT: keys of the call's hot table whose bucket is linked when the chunk begins are counted in
+// shared memory (high-level additions commute) and never become entries.
+template <int PT_THREADS, int KPT, bool HOT>
+__global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(const uint32_t* __restrict__ keys, uint64_t n, MswsDev D,
+                                                              PartDev Q) {
+    constexpr uint32_t R = PT_THREADS * KPT;
+    extern __shared__ __align__(16) uint32_t sm[];
+    uint32_t* s_ent = sm;                                          // [R]
+    uint16_t* s_idx = reinterpret_cast<uint16_t*>(sm + R);         // [R]
+    uint32_t* s_hkey = sm + R + R / 2;                             // HOT: [PART_HOT] keys, counts, high ids
+    uint32_t* s_hcnt = s_hkey + PART_HOT;
+    uint32_t* s_hid = s_hcnt + PART_HOT;
+    uint32_t* s_hist = HOT ? s_hid + PART_HOT : s_hkey;            // [parts] counts, then first positions
+    const int tid = threadIdx.x;
+    const uint32_t parts = Q.parts, per = (parts + PT_THREADS - 1) / PT_THREADS;
+    const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
+    if (blockIdx.x == 0 && tid == 0) {
+        D.ctl->n_switch = 0;
+        D.ctl->link_base = D.ctl->next_id;
+    }
+    if (HOT) {
+        for (uint32_t i = tid; i < PART_HOT; i += PT_THREADS) {
+            uint32_t key = __ldcg(Q.hot + i), id = 0;
+            if (key != HOT_EMPTY) {
+                id = __ldcg(D.low + (uint64_t)fast_mod(D.fm_low, key * D.seed) * LOW_WORDS + 7);
+                if (!is_linked(D, id)) key = HOT_EMPTY;
+            }
+            s_hkey[i] = key;
+            s_hcnt[i] = 0u;
+            s_hid[i] = id;
+        }
+    }
+    for (uint32_t t = blockIdx.x; t < Q.tiles; t += gridDim.x) {
+        const uint64_t k0 = (uint64_t)t * R;
+        const uint32_t cnt = (uint32_t)umin64(R, n - k0);
+        for (uint32_t i = tid; i < parts; i += PT_THREADS) s_hist[i] = 0u;
+        // the link order's switch bits and counts of this tile's positions
+        for (uint32_t i = tid; i < R / 32; i += PT_THREADS) __stcg(D.sw_bits + (k0 >> 5) + i, 0u);
+        if (R >= SW_BLOCK) {
+            if (tid < (int)(R / SW_BLOCK)) __stcg(D.sw_cnt + k0 / SW_BLOCK + tid, 0u);
+        } else if (tid == 0 && (k0 % SW_BLOCK) == 0) {
+            __stcg(D.sw_cnt + k0 / SW_BLOCK, 0u);
+        }
+        uint32_t e[KPT], pr[KPT];  // the key, then its entry; partition << 16 | rank
+        // thread's keys: vector v of 4 at tile index v * 4 * PT_THREADS + 4 * tid
+        if (vec && cnt == R) {
+#pragma unroll
+            for (int v = 0; v < KPT / 4; ++v) {
+                const uint4 q = __ldcs(reinterpret_cast<const uint4*>(keys + k0) + v * PT_THREADS + tid);
+                e[4 * v] = q.x, e[4 * v + 1] = q.y, e[4 * v + 2] = q.z, e[4 * v + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) {
+                const uint32_t i = (j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3);
+                e[j] = i < cnt ? __ldg(keys + k0 + i) : 0u;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+            const uint32_t i = (j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3);
+            bool live = i < cnt;
+            if (D.skip && live) live = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
+            if (HOT && live) {
+                const uint32_t s = 2 * hot_set(e[j]);
+                const uint2 hk = *reinterpret_cast<const uint2*>(s_hkey + s);
+                if (e[j] != HOT_EMPTY && (hk.x == e[j] || hk.y == e[j])) {
+                    atomicAdd(s_hcnt + s + (hk.x != e[j]), 1u);
+                    live = false;
+                }
+            }
+            const uint32_t hv = e[j] * D.seed;
+            const uint32_t b = fast_mod(D.fm_low, hv), p = b >> Q.shift;
+            e[j] = ((b & ((1u << Q.shift) - 1u)) << ENT_MASK_BITS) | fast_mod(D.fm_mask, hv);
+            pr[j] = live ? (p << 16) | atomicAdd(s_hist + p, 1u) : NONE;
+        }
+        __syncthreads();
+        {  // first position of each partition; its row of the run bounds
+            constexpr uint32_t PER = PART_MAX_PARTS / PT_THREADS;
+            uint32_t c[PER], sum = 0, total;
+#pragma unroll
+            for (uint32_t j = 0; j < PER; ++j) {
+                const uint32_t p = tid * per + j;
+                c[j] = j < per && p < parts ? s_hist[p] : 0u;
+                sum += c[j];
+            }
+            uint32_t run = block_exclusive_scan(sum, &total);
+#pragma unroll
+            for (uint32_t j = 0; j < PER; ++j) {
+                const uint32_t p = tid * per + j;
+                if (j < per && p < parts) {
+                    s_hist[p] = run;
+                    Q.off[(uint64_t)p * Q.stride + t] = (uint16_t)run;
+                    run += c[j];
+                }
+            }
+            if (tid == 0) Q.off[(uint64_t)parts * Q.stride + t] = (uint16_t)total;
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) {
+                if (pr[j] == NONE) continue;
+                const uint32_t pos = s_hist[pr[j] >> 16] + (pr[j] & 0xffffu);
+                s_ent[pos] = e[j];
+                s_idx[pos] = (uint16_t)((j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3));
+            }
+            __syncthreads();
+            uint4* ge = reinterpret_cast<uint4*>(Q.ent + k0);
+            uint4* gi = reinterpret_cast<uint4*>(Q.idx + k0);
+            for (uint32_t i = tid; i * 4 < total; i += PT_THREADS) __stcg(ge + i, reinterpret_cast<const uint4*>(s_ent)[i]);
+            for (uint32_t i = tid; i * 8 < total; i += PT_THREADS) __stcg(gi + i, reinterpret_cast<const uint4*>(s_idx)[i]);
+        }
+        __syncthreads();
+    }
+    if (HOT) {  // the counts of the hot keys: one add per counter and block
+        for (uint32_t i = tid; i < PART_HOT; i += PT_THREADS) {
+            const uint32_t c = s_hcnt[i];
+            if (!c) continue;
+            uint32_t* hb = D.high + (uint64_t)(s_hid[i] - START) * HIGH_WORDS;
+            for (uint32_t m = __ldg(D.masks + fast_mod(D.fm_mask, s_hkey[i] * D.seed)); m; m &= m - 1)
+                atomicAdd(hb + (__ffs(m) - 1), c);
+        }
+    }
+}
+
+// ---- 2: one partition per block ------------------------------------------------------------
+
+// A mask table of three counters per mask (the default) is kept as the counters' numbers, 5 bits
+// each; any other (WIDE) as the masks.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t mask_code(uint32_t m) {
+    if (WIDE) return m;
+    const uint32_t a = __ffs(m) - 1, m1 = m & (m - 1), b = __ffs(m1) - 1, c = __ffs(m1 & (m1 - 1)) - 1;
+    return a | b << 5 | c << 10;
+}
+template <bool WIDE>
+__device__ __forceinline__ uint32_t code_mask(uint32_t q) {
+    return WIDE ? q : (1u << (q & 31u)) | (1u << ((q >> 5) & 31u)) | (1u << (q >> 10));
+}
+
+struct ApShared {
+    uint32_t* tab;             // [2^shift][8] the partition's buckets (word 7: flagged buckets by slot)
+    uint32_t* w7;              // [2^shift] their index words
+    uint32_t* mk;              // [n_masks] mask_code
+    uint32_t* acc;             // [ap_accs][ACC_WORDS]
+    uint32_t* accid;           // [ap_accs] a row's high id, or (NEW) its switch position
+    uint16_t* accb;            // [ap_accs] and its bucket
+    unsigned long long* recs;  // [ap_unit]
+    uint32_t* before;          // [AP_TILES + 1] entries of the staged runs before run r
+    uint32_t* dlt;             // [AP_TILES] run r: its first entry minus before[r]
+    uint16_t* map;             // [ap_unit] the run of each entry of the unit
+};
+
+__host__ __device__ inline size_t apply_smem(uint32_t shift, uint32_t n_masks) {
+    const size_t pb = (size_t)1 << shift;
+    return (size_t)ap_unit(shift) * 10 + pb * 36 + (size_t)((n_masks + 1) & ~1u) * 4 + AP_TILES * 8 + 8 +
+           ap_accs(shift) * (ACC_WORDS * 4 + 6);
+}
+
+__device__ __forceinline__ ApShared ap_carve(uint8_t* p, uint32_t shift, uint32_t n_masks) {
+    const size_t pb = (size_t)1 << shift;
+    ApShared S;
+    S.recs = reinterpret_cast<unsigned long long*>(p);
+    p += ap_unit(shift) * 8;
+    S.tab = reinterpret_cast<uint32_t*>(p);
+    p += pb * 32;
+    S.mk = reinterpret_cast<uint32_t*>(p);
+    p += (size_t)((n_masks + 1) & ~1u) * 4;  // what follows stays 8-byte aligned (replay_few uses the run map's memory)
+    S.acc = reinterpret_cast<uint32_t*>(p);
+    p += ap_accs(shift) * ACC_WORDS * 4;
+    S.accid = reinterpret_cast<uint32_t*>(p);
+    p += ap_accs(shift) * 4;
+    S.w7 = reinterpret_cast<uint32_t*>(p);
+    p += pb * 4;
+    S.dlt = reinterpret_cast<uint32_t*>(p);
+    p += AP_TILES * 4;
+    S.before = reinterpret_cast<uint32_t*>(p);
+    p += AP_TILES * 4 + 8;
+    S.map = reinterpret_cast<uint16_t*>(p);
+    p += ap_unit(shift) * 2;
+    S.accb = reinterpret_cast<uint16_t*>(p);
+    return S;
+}
+
+// c occurrences to the selected low counters of a bucket, any mask; whether one crosses.
+__device__ __forceinline__ bool part_low_add(uint32_t* bw, uint32_t mm, uint32_t c) {
+    bool cross = false;
+    while (mm) {
+        const uint32_t w = (uint32_t)(__ffs(mm) - 1) >> 2, nib = (mm >> (4u * w)) & 0xfu;
+        mm &= ~(nib << (4u * w));
+        cross |= crosses(atomicAdd(bw + w, expand_nibble(nib) * c), nib, c);
+    }
+    return cross;
+}
+
+// One entry (MANY: c merged occurrences; else c = 1) of the chunk.
+template <bool MANY, bool WIDE>
+__device__ __forceinline__ void part_apply_entry(const MswsDev& D, const ApShared& S, uint32_t e, uint32_t c,
+                                                 uint32_t* s_nflag, uint32_t* s_drop) {
+    const uint32_t lb = e >> ENT_MASK_BITS;
+    const uint32_t q = S.mk[e & ENT_MASK];
+    const uint32_t w7 = S.w7[lb];
+    if ((int32_t)w7 <= 0) {  // not linked, or flagged in this run of tiles
+        bool cross;
+        uint32_t* bw = S.tab + lb * LOW_WORDS;
+        if (MANY || WIDE) {
+            cross = part_low_add(bw, code_mask<WIDE>(q), c);
+        } else {
+            // counter i: byte i & 3 of word i >> 2.  One more makes 130 of 129, so no byte below
+            // 128 can cross; counters that share a word see each other's additions only in the
+            // other's byte.
+            const uint32_t sx = (q & 3u) * 8u, sy = ((q >> 5) & 3u) * 8u, sz = ((q >> 10) & 3u) * 8u;
+            const uint32_t ox = atomicAdd(bw + ((q >> 2) & 7u), 1u << sx);
+            const uint32_t oy = atomicAdd(bw + ((q >> 7) & 7u), 1u << sy);
+            const uint32_t oz = atomicAdd(bw + (q >> 12), 1u << sz);
+            cross = ((ox & (0x80u << sx)) | (oy & (0x80u << sy)) | (oz & (0x80u << sz))) != 0u;
+            if (cross)
+                cross = ((ox >> sx) & 0xffu) >= CROSS - 1u || ((oy >> sy) & 0xffu) >= CROSS - 1u ||
+                        ((oz >> sz) & 0xffu) >= CROSS - 1u;
+        }
+        if (cross && !(atomicOr(S.w7 + lb, FLAG) & FLAG)) {
+            const uint32_t slot = atomicAdd(s_nflag, 1u);
+            S.tab[slot * LOW_WORDS + 7] = lb;
+            atomicExch(S.w7 + lb, FLAG | slot);
+        }
+        return;
+    }
+    if ((w7 & (ACC | TEMP)) == ACC) {
+        uint32_t* row = S.acc + (w7 & 0xffffu) * ACC_WORDS;
+        if (WIDE) {
+            for (uint32_t mm = q; mm; mm &= mm - 1) atomicAdd(row + (__ffs(mm) - 1), c);
+        } else {
+            atomicAdd(row + (q & 31u), c);
+            atomicAdd(row + ((q >> 5) & 31u), c);
+            atomicAdd(row + (q >> 10), c);
+        }
+        if (w7 & NEW) atomicAdd(row + LOW_COUNTERS, c);
+        return;
+    }
+    uint32_t* hb;
+    if (w7 & TEMP) {
+        if (w7 == TEMP_NOROW) return;
+        const uint32_t r = w7 & ~TEMP;
+        hb = D.totals + (uint64_t)r * LOW_COUNTERS;
+        atomicAdd(&D.sw[r].y, c);
+    } else if (is_linked(D, w7)) {
+        hb = D.high + (uint64_t)(w7 - START) * HIGH_WORDS;
+    } else {  // saturated: the pool ran out
+        atomicAdd(s_drop, c);
+        return;
+    }
+    for (uint32_t mm = code_mask<WIDE>(q); mm; mm &= mm - 1) atomicAdd(hb + (__ffs(mm) - 1), c);
+}
+
+// A thread's share of up to U * AP_THREADS entries: entry u * AP_THREADS + tid for u < U, `sub` in
+// all.  Heavy: one key fills most of the partition, so a warp counts the entries equal to one of
+// its first ones and adds them at once.
+template <bool WIDE, int U>
+__device__ __forceinline__ void part_apply_batch(const MswsDev& D, const ApShared& S, const uint32_t (&e)[U], uint32_t sub,
+                                                 bool heavy, uint32_t* s_nflag, uint32_t* s_drop) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    uint32_t skip = HOT_EMPTY;  // no entry
+    if (heavy && tid - lane < sub) {  // warp-uniform
+        const uint32_t have = __ballot_sync(0xffffffffu, tid < sub);
+        uint32_t x = __shfl_sync(0xffffffffu, e[0], 0);
+        const uint32_t other = __ballot_sync(0xffffffffu, tid < sub && e[0] != x);
+        if (__popc(other) > 16) x = __shfl_sync(0xffffffffu, e[0], __ffs(other) - 1);
+        uint32_t c = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) c += e[u] == x && u * AP_THREADS + tid < sub;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c >= 2) {
+            skip = x;
+            if (lane == (uint32_t)__ffs(have) - 1) part_apply_entry<true, WIDE>(D, S, x, c, s_nflag, s_drop);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const uint32_t k = u * AP_THREADS + tid;
+        if (k - lane >= sub) break;  // warp-uniform
+        if (k < sub && e[u] != skip) part_apply_entry<false, WIDE>(D, S, e[u], 1u, s_nflag, s_drop);
+    }
+}
+
+// A bucket that switched at array position pos, with n_after keys from there on: its increments
+// collect in an accumulator (or a row) until the link order is known.  Called by a whole warp,
+// lane c with counter c's high increment H.
+__device__ __forceinline__ void put_row(const MswsDev& D, uint32_t r, uint32_t bucket, uint32_t pos, uint32_t n_after,
+                                        uint32_t H) {
+    const int lane = threadIdx.x & 31;
+    if (r < D.long_cap && lane < LOW_COUNTERS) __stcg(D.totals + (uint64_t)r * LOW_COUNTERS + lane, H);
+    if (lane == 0) {
+        __stcg(D.flag_list + r, bucket);  // flag_cap covers every bucket a chunk can link
+        __stcg(D.sw + r, make_uint2(pos, n_after));
+        atomicOr(D.sw_bits + (pos >> 5), 1u << (pos & 31));
+        atomicAdd(D.sw_cnt + pos / SW_BLOCK, 1u);
+    }
+}
+__device__ __forceinline__ void open_row(const MswsDev& D, const ApShared& S, uint32_t accs, uint32_t* s_nacc, uint32_t lb,
+                                         uint32_t b0, uint32_t pos, uint32_t n_after, uint32_t H) {
+    const int lane = threadIdx.x & 31;
+    uint32_t a = 0;
+    if (lane == 0) a = atomicAdd(s_nacc, 1u);
+    a = __shfl_sync(0xffffffffu, a, 0);
+    if (a < accs) {
+        if (lane < LOW_COUNTERS) S.acc[a * ACC_WORDS + lane] = H;
+        if (lane == 0) {
+            S.acc[a * ACC_WORDS + LOW_COUNTERS] = n_after;
+            S.accid[a] = pos;
+            S.accb[a] = (uint16_t)lb;
+            S.w7[lb] = ACC | NEW | a;
+        }
+        return;
+    }
+    uint32_t r = 0;
+    if (lane == 0) r = atomicAdd(&D.ctl->n_switch, 1u);
+    r = __shfl_sync(0xffffffffu, r, 0);
+    put_row(D, r, b0 + lb, pos, n_after, H);
+    if (lane == 0) S.w7[lb] = r < D.long_cap ? (TEMP | r) : TEMP_NOROW;
+}
+
+// Pre-chunk counter of lane i: the bucket's words minus the packed increments T (counter c in
+// lane c), as pre_counters of the grid-wide replay.
+__device__ __forceinline__ uint32_t part_pre(const uint32_t* bw, uint32_t T) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t fw = lane < 7 ? bw[lane] : 0u;
+    uint32_t sw = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sw += __shfl_sync(0xffffffffu, T, (4 * (lane & 7) + k) & 31) << (8 * k);
+    const uint32_t pwi = __shfl_sync(0xffffffffu, fw - sw, (lane >> 2) & 7);
+    return lane < LOW_COUNTERS ? (pwi >> (8 * (lane & 3))) & 0xffu : 0u;
+}
+
+__device__ __forceinline__ void part_write_low(uint32_t* bw, uint32_t cur) {
+    const int lane = threadIdx.x & 31;
+    uint32_t word = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) word |= __shfl_sync(0xffffffffu, cur, (4 * (lane & 7) + k) & 31) << (8 * k);
+    if (lane < 7) bw[lane] = word;
+}
+
+// Ascending sort of recs[0, K) (at most ap_recs) by the whole block: bitonic over the next power
+// of two, padded with all ones.
+__device__ __forceinline__ void block_sort(unsigned long long* recs, uint32_t K) {
+    uint32_t N = 32;
+    while (N < K) N <<= 1;
+    for (uint32_t i = K + threadIdx.x; i < N; i += AP_THREADS) recs[i] = ~0ull;
+    __syncthreads();
+    for (uint32_t k = 2; k <= N; k <<= 1)
+        for (uint32_t j = k >> 1; j; j >>= 1) {
+            for (uint32_t i = threadIdx.x; i < N / 2; i += AP_THREADS) {
+                const uint32_t a = ((i & ~(j - 1)) << 1) | (i & (j - 1)), b = a | j;
+                const unsigned long long x = recs[a], y = recs[b];
+                if ((x > y) == ((a & k) == 0)) {
+                    recs[a] = y;
+                    recs[b] = x;
+                }
+            }
+            __syncthreads();
+        }
+}
+
+// Flagged bucket `s`, if it has at most 32 records among recs[0, K) (else false), replayed by one warp (buf: 32
+// words of its own; the run map's memory, which is done with by then): lane i takes
+// the i-th record in array order; counter c's occurrences are one ballot (kept by lane c), so a
+// record sees P + the bits before its lane in each counter it selects.
+static_assert(ap_unit(11) * 2 >= AP_WARPS * 32 * 8, "the run map holds every warp's 32 records");
+template <bool WIDE>
+__device__ __forceinline__ bool replay_few(const MswsDev& D, const ApShared& S, unsigned long long* buf, uint32_t accs,
+                                           uint32_t* s_nacc, uint32_t s, uint32_t K, uint32_t b0, uint32_t* s_rb,
+                                           uint32_t* s_rk) {
+    const int lane = threadIdx.x & 31;
+    uint32_t n = 0;
+    for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+        const unsigned long long r = k0 + lane < K ? S.recs[k0 + lane] : ~0ull;
+        const bool mine = (uint32_t)(r >> 46) == s;
+        const uint32_t bal = __ballot_sync(0xffffffffu, mine);
+        n += __popc(bal);
+        if (n > 32) return false;
+        if (mine) buf[n - __popc(bal) + __popc(bal & lanemask_lt())] = r;
+    }
+    __syncwarp();
+    unsigned long long r = lane < (int)n ? buf[lane] : ~0ull;
+    uint32_t rank = 0;
+    for (uint32_t k = 0; k < n; ++k) rank += buf[k] < r;
+    __syncwarp();
+    if (lane < (int)n) buf[rank] = r;  // positions are distinct
+    __syncwarp();
+    r = buf[lane];
+    const uint32_t m = lane < (int)n ? code_mask<WIDE>(S.mk[(uint32_t)r & ENT_MASK]) : 0u;
+    uint32_t occ = 0;  // lane c: the records that select counter c
+#pragma unroll
+    for (int c = 0; c < LOW_COUNTERS; ++c) {
+        const uint32_t bal = __ballot_sync(0xffffffffu, (m >> c) & 1u);
+        if (lane == c) occ = bal;
+    }
+    const uint32_t lb = S.tab[s * LOW_WORDS + 7];
+    uint32_t* bw = S.tab + lb * LOW_WORDS;
+    ReplayOut o;
+    o.T = __popc(occ);
+    o.P = part_pre(bw, o.T);
+    bool trig = false;
+    for (uint32_t mm = m; __any_sync(0xffffffffu, mm != 0); mm &= mm - 1) {
+        const int c = mm ? __ffs(mm) - 1 : 0;
+        const uint32_t bal = __shfl_sync(0xffffffffu, occ, c), P = __shfl_sync(0xffffffffu, o.P, c);
+        trig |= mm && P + __popc(bal & lanemask_lt()) > LIMIT;
+    }
+    const uint32_t tb = __ballot_sync(0xffffffffu, trig);
+    if (tb) {
+        const int j = __ffs(tb) - 1;
+        o.cur = o.P + __popc(occ & ((1u << j) - 1u));
+        o.mL = __shfl_sync(0xffffffffu, m, j);
+        const uint32_t pos = __shfl_sync(0xffffffffu, (uint32_t)(r >> ENT_MASK_BITS), j);
+        const uint32_t H = high_increments(D, o);
+        __syncwarp();
+        part_write_low(bw, o.cur);
+        open_row(D, S, accs, s_nacc, lb, b0, pos, n - j, H);
+    } else if (lane == 0) {
+        S.w7[lb] = 0u;  // every key added low
+    }
+    if (lane == 0) {
+        atomicAdd(s_rb, 1u);
+        atomicAdd(s_rk, n);
+    }
+    __syncwarp();
+    return true;
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev Q) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const ApShared S = ap_carve(smem, Q.shift, D.n_masks);
+    __shared__ uint32_t s_nflag, s_nrec, s_many, s_drop, s_rb, s_rk, s_nacc, s_new, s_row;
+    __shared__ uint32_t s_cnt[LOW_COUNTERS + 2];  // bisection: counts per counter, keys, mask
+    __shared__ uint32_t s_pre[LOW_COUNTERS];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t p = blockIdx.x;
+    for (uint32_t i = tid; i < D.n_masks; i += AP_THREADS) S.mk[i] = mask_code<WIDE>(__ldg(D.masks + i));  // the host's
+    const uint32_t accs = ap_accs(Q.shift);
+    for (uint32_t i = tid; i < accs * ACC_WORDS; i += AP_THREADS) S.acc[i] = 0u;
+    if (tid == 0) s_nflag = s_nrec = s_many = s_drop = s_rb = s_rk = s_nacc = s_new = 0;
+    __syncthreads();
+    const uint64_t b0 = (uint64_t)p << Q.shift;
+    const uint32_t nb = (uint32_t)umin64((uint64_t)1 << Q.shift, D.n_low - b0);
+    uint4* gt = reinterpret_cast<uint4*>(D.low + b0 * LOW_WORDS);
+    {
+        uint4* st = reinterpret_cast<uint4*>(S.tab);
+        for (uint32_t i0 = tid; i0 < nb * 2; i0 += 4 * AP_THREADS) {
+            uint4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * AP_THREADS < nb * 2) v[u] = __ldcg(gt + i0 + u * AP_THREADS);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t i = i0 + u * AP_THREADS;
+                if (i < nb * 2) {
+                    st[i] = v[u];
+                    if (i & 1u) {
+                        uint32_t w7 = v[u].w;
+                        if (is_linked(D, w7)) {
+                            const uint32_t a = atomicAdd(&s_nacc, 1u);
+                            if (a < accs) {
+                                S.accid[a] = w7;
+                                S.accb[a] = (uint16_t)(i >> 1);
+                                w7 = ACC | a;
+                            }
+                        }
+                        S.w7[i >> 1] = w7;
+                    }
+                }
+            }
+        }
+    }
+    const uint16_t* o0 = Q.off + (uint64_t)p * Q.stride;
+    const uint16_t* o1 = o0 + Q.stride;
+    const uint32_t tile = Q.tile, cap = ap_unit(Q.shift);
+    constexpr int U = 4096 / AP_THREADS;  // a thread's entries of a unit, at most
+    uint32_t units = 0;
+    for (uint32_t ts = 0; ts < Q.tiles; ts += AP_TILES) {
+        // the run bounds of the next AP_TILES tiles
+        __syncthreads();
+        const uint32_t nr = min(AP_TILES, Q.tiles - ts);
+        uint32_t a = 0, len = 0, total;
+        if (tid < nr) {
+            a = __ldcg(o0 + ts + tid);
+            len = __ldcg(o1 + ts + tid) - a;
+        }
+        const uint32_t before = block_exclusive_scan(len, &total);
+        S.dlt[tid] = (ts + tid) * tile + a - before;
+        S.before[tid] = before;
+        if (tid == 0) S.before[nr] = total;  // (entry nr < AP_TILES already holds it)
+        // far above an even share, a heavy key is likely, maybe of a bucket that is not linked yet
+        const bool heavy = total > 4u * Q.mean * nr;
+        for (uint32_t r0 = 0; r0 < nr;) {
+            __syncthreads();
+            const uint32_t base = S.before[r0];
+            const uint32_t most = heavy ? min(cap, AP_FIRST << min(units++, 4u)) : cap;
+            const uint32_t r1 =
+                r0 + __syncthreads_count(tid >= r0 && tid < nr && (tid == r0 || before + len - base <= most));
+            const uint32_t sub = S.before[r1] - base;
+            const uint32_t rb = r0;
+            r0 = r1;
+            if (sub == 0) continue;
+            const bool one_run = sub > cap;  // then r1 == rb + 1: no map needed
+            uint32_t e[U];
+            if (!one_run) {
+                for (uint32_t r = rb + wid * 4 + (lane >> 3); r < r1; r += AP_WARPS * 4) {  // eight lanes per run
+                    const uint32_t k1 = S.before[r + 1] - base;
+                    for (uint32_t k = S.before[r] - base + (lane & 7); k < k1; k += 8) S.map[k] = (uint16_t)r;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t k = u * AP_THREADS + tid;
+                    e[u] = k < sub ? __ldcg(Q.ent + S.dlt[S.map[k]] + base + k) : 0u;
+                }
+                part_apply_batch<WIDE, U>(D, S, e, sub, heavy, &s_nflag, &s_drop);
+            } else {
+                const uint32_t* run = Q.ent + S.dlt[rb] + base;
+                for (uint32_t k0 = 0; k0 < sub; k0 += U * AP_THREADS) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t k = k0 + u * AP_THREADS + tid;
+                        e[u] = k < sub ? __ldcg(run + k) : 0u;
+                    }
+                    part_apply_batch<WIDE, U>(D, S, e, sub - k0, true, &s_nflag, &s_drop);
+                }
+            }
+            __syncthreads();
+            const uint32_t F = s_nflag;
+            if (F == 0) continue;
+            // the records of the flagged buckets
+            auto record = [&](uint32_t x, uint32_t r, uint32_t at) {
+                const uint32_t w7 = S.w7[x >> ENT_MASK_BITS];
+                if (!(w7 & FLAG)) return;
+                const uint32_t k = atomicAdd(&s_nrec, 1u), pos = (ts + r) * tile + __ldcg(Q.idx + at);
+                if (k < cap)
+                    S.recs[k] = (unsigned long long)(w7 & ~FLAG) << 46 | (unsigned long long)pos << ENT_MASK_BITS |
+                                (x & ENT_MASK);
+            };
+            if (!one_run) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t k = u * AP_THREADS + tid;
+                    if (k < sub) record(e[u], S.map[k], S.dlt[S.map[k]] + base + k);
+                }
+            } else {
+                for (uint32_t k = tid; k < sub; k += AP_THREADS)
+                    record(__ldcg(Q.ent + S.dlt[rb] + base + k), rb, S.dlt[rb] + base + k);
+            }
+            __syncthreads();
+            const uint32_t K = s_nrec;
+            if (K <= cap) {
+                // a warp replays a bucket of up to 32 records on its own
+                for (uint32_t s = wid; s < F; s += AP_WARPS)
+                    if (!replay_few<WIDE>(D, S, reinterpret_cast<unsigned long long*>(S.map) + wid * 32, accs, &s_nacc, s,
+                                          K, (uint32_t)b0, &s_rb, &s_rk) && lane == 0)
+                        s_many = 1;
+                __syncthreads();
+            }
+            // longer ones: all records sorted (12 k cycles for 300 of them), then a warp each
+            if (K <= cap && s_many) {
+                block_sort(S.recs, K);
+                for (uint32_t s = wid; s < F; s += AP_WARPS) {
+                    const uint32_t lb = S.tab[s * LOW_WORDS + 7];
+                    if (S.w7[lb] != (FLAG | s)) continue;  // replayed above
+                    uint32_t beg = 0, end = 0;  // the slot's records
+                    {
+                        uint32_t lo = 0, hi = K;
+                        while (lo < hi) {
+                            const uint32_t mid = (lo + hi) >> 1;
+                            if ((uint32_t)(S.recs[mid] >> 46) < s) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        beg = lo, hi = K;
+                        while (lo < hi) {
+                            const uint32_t mid = (lo + hi) >> 1;
+                            if ((uint32_t)(S.recs[mid] >> 46) <= s) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        end = lo;
+                    }
+                    uint32_t* bw = S.tab + lb * LOW_WORDS;
+                    ReplayOut o;
+                    o.T = 0;
+                    for (uint32_t q = beg; q < end; q += 32)
+                        o.T += group_counts(q + lane < end ? code_mask<WIDE>(S.mk[(uint32_t)S.recs[q + lane] & ENT_MASK]) : 0u);
+                    o.P = part_pre(bw, o.T);
+                    o.cur = o.P;
+                    o.mL = 0;
+                    o.found = false;
+                    o.L = 0;
+                    for (uint32_t q = beg; q < end; q += 32) {
+                        const uint32_t m = q + lane < end ? code_mask<WIDE>(S.mk[(uint32_t)S.recs[q + lane] & ENT_MASK]) : 0u;
+                        const int j = link_step(m, o.cur);
+                        if (j >= 0) {
+                            o.found = true;
+                            o.L = q + j;
+                            o.mL = __shfl_sync(0xffffffffu, m, j);
+                            break;
+                        }
+                    }
+                    if (o.found) {
+                        const uint32_t pos = (uint32_t)(S.recs[o.L] >> ENT_MASK_BITS);
+                        const uint32_t H = high_increments(D, o);
+                        __syncwarp();
+                        part_write_low(bw, o.cur);
+                        open_row(D, S, accs, &s_nacc, lb, (uint32_t)b0, pos, end - o.L, H);
+                    } else if (lane == 0) {
+                        S.w7[lb] = 0u;  // every key added low
+                    }
+                    if (lane == 0) {
+                        atomicAdd(&s_rb, 1u);
+                        atomicAdd(&s_rk, end - beg);
+                    }
+                }
+            } else if (K > cap) {
+                // More records than fit, all of one tile (a very heavy key that is not linked
+                // yet): per flagged bucket, bisect the array position of the switching key, the
+                // first position x such that some counter has 130 - P occurrences up to x (the key
+                // that sees 129 = P + its earlier occurrences).
+                const uint32_t plo = (ts + rb) * tile, phi = plo + tile - 1;
+                for (uint32_t s = 0; s < F; ++s) {
+                    const uint32_t lb = S.tab[s * LOW_WORDS + 7];
+                    uint32_t* bw = S.tab + lb * LOW_WORDS;
+                    auto count = [&](uint32_t upto) {  // occurrences per counter (and keys) at positions <= upto
+                        __syncthreads();
+                        if (tid < LOW_COUNTERS + 2) s_cnt[tid] = 0u;
+                        __syncthreads();
+                        for (uint32_t k = tid; k < sub; k += AP_THREADS) {
+                            const uint32_t at = S.dlt[rb] + base + k, x = __ldcg(Q.ent + at);
+                            if ((x >> ENT_MASK_BITS) != lb) continue;
+                            const uint32_t pos = plo + __ldcg(Q.idx + at);
+                            if (pos > upto) continue;
+                            const uint32_t m = code_mask<WIDE>(S.mk[x & ENT_MASK]);
+                            for (uint32_t mm = m; mm; mm &= mm - 1) atomicAdd(s_cnt + (__ffs(mm) - 1), 1u);
+                            atomicAdd(s_cnt + LOW_COUNTERS, 1u);
+                            if (pos == upto) s_cnt[LOW_COUNTERS + 1] = m;
+                        }
+                        __syncthreads();
+                    };
+                    count(phi);
+                    const uint32_t n_total = s_cnt[LOW_COUNTERS];
+                    uint32_t T = lane < LOW_COUNTERS ? s_cnt[lane] : 0u;
+                    if (wid == 0) {
+                        const uint32_t P = part_pre(bw, T);
+                        if (lane < LOW_COUNTERS) s_pre[lane] = P;
+                    }
+                    __syncthreads();
+                    const uint32_t P = lane < LOW_COUNTERS ? s_pre[lane] : 0u;
+                    auto reached = [&](uint32_t c) { return __any_sync(0xffffffffu, c && P + c > LIMIT + 1); };
+                    const bool found = reached(T);
+                    uint32_t lo = plo, hi = phi;  // uniform over the block
+                    while (found && lo < hi) {
+                        const uint32_t mid = lo + (hi - lo) / 2;
+                        count(mid);
+                        if (reached(lane < LOW_COUNTERS ? s_cnt[lane] : 0u)) hi = mid;
+                        else lo = mid + 1;
+                    }
+                    if (found) count(lo);
+                    if (wid == 0) {
+                        if (found) {
+                            ReplayOut o;
+                            o.T = T;
+                            o.P = P;
+                            o.mL = s_cnt[LOW_COUNTERS + 1];
+                            const uint32_t upto = lane < LOW_COUNTERS ? s_cnt[lane] : 0u;
+                            o.cur = P + upto - (lane < LOW_COUNTERS ? (o.mL >> lane) & 1u : 0u);
+                            const uint32_t n_after = n_total - s_cnt[LOW_COUNTERS] + 1u;
+                            const uint32_t H = high_increments(D, o);
+                            part_write_low(bw, o.cur);
+                            open_row(D, S, accs, &s_nacc, lb, (uint32_t)b0, lo, n_after, H);
+                        } else if (lane == 0) {
+                            S.w7[lb] = 0u;
+                        }
+                        if (lane == 0) {
+                            s_rb += 1u;
+                            s_rk += n_total;
+                        }
+                    }
+                    __syncthreads();
+                }
+            }
+            __syncthreads();
+            if (tid == 0) s_nflag = s_nrec = s_many = 0;
+        }
+    }
+    __syncthreads();
+    // the accumulators: linked buckets' counts to their high buckets, new ones to rows
+    const uint32_t na = min(s_nacc, accs);
+    for (uint32_t a = tid; a < na; a += AP_THREADS)
+        if (S.w7[S.accb[a]] & NEW) atomicAdd(&s_new, 1u);
+    __syncthreads();
+    if (tid == 0 && s_new) s_row = atomicAdd(&D.ctl->n_switch, s_new);
+    __syncthreads();
+    for (uint32_t a = wid; a < na; a += AP_WARPS) {
+        const uint32_t lb = S.accb[a], id = S.accid[a];
+        const uint32_t v = lane < LOW_COUNTERS ? S.acc[a * ACC_WORDS + lane] : 0u;
+        if (S.w7[lb] & NEW) {
+            uint32_t r = 0;
+            if (lane == 0) r = atomicAdd(&s_row, 1u);
+            r = __shfl_sync(0xffffffffu, r, 0);
+            put_row(D, r, (uint32_t)b0 + lb, id, S.acc[a * ACC_WORDS + LOW_COUNTERS], v);
+        } else {
+            if (v) atomicAdd(D.high + (uint64_t)(id - START) * HIGH_WORDS + lane, v);
+            if (lane == 0) S.w7[lb] = id;
+        }
+    }
+    __syncthreads();
+    {
+        const uint4* st = reinterpret_cast<const uint4*>(S.tab);
+        for (uint32_t i = tid; i < nb * 2; i += AP_THREADS) {
+            uint4 v = st[i];
+            if (i & 1u) v.w = S.w7[i >> 1];  // a new bucket's is set with its id
+            __stcg(gt + i, v);
+        }
+    }
+    if (tid == 0) {
+        if (s_drop) atomicAdd(&D.ctl->dropped, (unsigned long long)s_drop);
+        if (s_rb) {
+            atomicAdd(&D.ctl->repaired_buckets, (unsigned long long)s_rb);
+            atomicAdd(&D.ctl->repaired_keys, (unsigned long long)s_rk);
+        }
+    }
+}
+
+// ---- 3: high ids in the array order of the switching keys -----------------------------------
+
+__global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev Q) {
+    extern __shared__ __align__(16) uint32_t spre[];  // switches per SW_BLOCK positions, then their prefix
+    Ctl* ctl = D.ctl;
+    const uint32_t ns = __ldcg(&ctl->n_switch);
+    if (ns == 0) return;
+    const uint32_t base = __ldcg(&ctl->link_base);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (blockIdx.x == 0 && tid == 0)  // the allocator stops at the pool's end, as the oracle's
+        ctl->next_id = (uint32_t)min((unsigned long long)base + ns, (unsigned long long)START + D.n_high);
+    if (blockIdx.x * AP_WARPS >= ns) return;
+    const uint32_t nq = (uint32_t)(((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK);
+    for (uint32_t i = tid; i < nq; i += AP_THREADS) spre[i] = __ldcg(D.sw_cnt + i);
+    __syncthreads();
+    block_scan_smem(spre, nq);
+    for (uint32_t r = blockIdx.x * AP_WARPS + wid; r < ns; r += gridDim.x * AP_WARPS) {
+        const uint32_t b = __ldcg(D.flag_list + r);
+        const uint2 w = __ldcg(D.sw + r);
+        const uint32_t id = base + switch_rank(D, spre, w.x);
+        const bool ok = (uint64_t)(id - START) < D.n_high;
+        uint32_t H = 0, n_after = w.y;
+        if (r < D.long_cap) {
+            if (lane < LOW_COUNTERS) H = __ldcg(D.totals + (uint64_t)r * LOW_COUNTERS + lane);
+        } else {
+            // no row was left: count the bucket's entries from the switch on again
+            const uint32_t part = b >> Q.shift, lb = b & ((1u << Q.shift) - 1u);
+            const uint16_t* o0 = Q.off + (uint64_t)part * Q.stride;
+            uint32_t keys = 0;
+            for (uint32_t t = w.x / Q.tile; t < Q.tiles; ++t) {
+                const uint32_t e1 = t * Q.tile + __ldcg(o0 + Q.stride + t);
+                for (uint32_t i0 = t * Q.tile + __ldcg(o0 + t); i0 < e1; i0 += 32) {
+                    const uint32_t i = i0 + lane;
+                    uint32_t m = 0;
+                    bool first = false;
+                    if (i < e1) {
+                        const uint32_t e = __ldcg(Q.ent + i);
+                        if ((e >> ENT_MASK_BITS) == lb) {
+                            const uint32_t pos = t * Q.tile + __ldcg(Q.idx + i);
+                            if (pos >= w.x) m = __ldg(D.masks + (e & ENT_MASK));
+                            first = pos == w.x;
+                        }
+                    }
+                    keys += __popc(__ballot_sync(0xffffffffu, m != 0));
+                    if (!__any_sync(0xffffffffu, m != 0)) continue;
+                    H += group_counts(m);
+                    if (D.compat_v3) {  // the switching key lands on bit % 8
+                        const uint32_t fb = __ballot_sync(0xffffffffu, first);
+                        if (fb) {
+                            ReplayOut o;
+                            o.T = H;
+                            o.cur = o.P = 0;
+                            o.mL = __shfl_sync(0xffffffffu, m, __ffs(fb) - 1);
+                            H = high_increments(D, o);
+                        }
+                    }
+                }
+            }
+            n_after = keys;
+        }
+        link_bucket(D, b, id, ok, H, n_after);
+    }
+}
+
+// ---- launchers ------------------------------------------------------------------------------
+
+static size_t split_smem(uint32_t tile, uint32_t parts, bool hot) {
+    return (size_t)tile * 6 + parts * 4 + (hot ? PART_HOT * 12 : 0);
+}
+
+cudaError_t part_configure(PartLaunch* L, uint32_t shift, uint32_t parts, uint32_t n_masks, int num_sms) {
+    cudaError_t e = cudaSuccess;
+    // the dynamic shared-memory cap is a per-kernel attribute shared by every sketch of the
+    // process: the largest any of them may ask for; a launch passes its own size
+    const size_t split_max = split_smem(PART_TILE, PART_MAX_PARTS, true);
+    const size_t apply_max = std::max(apply_smem(PART_MAX_SHIFT, PART_MAX_MASKS), apply_smem(PART_MAX_SHIFT - 1, PART_MAX_MASKS));
+    const size_t link_max = PART_MAX_CHUNK / SW_BLOCK * 4;
+    const void* fns[] = {(const void*)k_part_split<1024, 16, false>, (const void*)k_part_split<512, 4, false>,
+                         (const void*)k_part_split<1024, 16, true>,  (const void*)k_part_split<512, 4, true>,
+                         (const void*)k_part_apply<false>,     (const void*)k_part_apply<true>,
+                         (const void*)k_part_link};
+    const size_t most[] = {split_max, split_max, split_max, split_max, apply_max, apply_max, link_max};
+    for (int i = 0; i < 7 && e == cudaSuccess; ++i)
+        e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most[i]);
+    L->num_sms = num_sms;
+    L->apply_smem = apply_smem(shift, n_masks);
+    return e;
+}
+
+cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cudaStream_t st) {
+    uint32_t* hot = part.hot;
+    void* args[] = {(void*)&d_keys, (void*)&n, (void*)&hot};
+    return cudaLaunchKernel((const void*)k_part_hot, dim3(HOT_BLOCKS), dim3(HOT_THREADS), args, 0, st);
+}
+
+cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
+                        bool hot, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    PartDev Q = part;
+    MswsDev Dc = D;
+    // tiles of 2048 keys while 8192-key tiles would leave SMs idle (two blocks on each of 148)
+    const bool small = n < PART_SMALL_MAX;
+    Q.tile = small ? PART_TILE_SMALL : PART_TILE;
+    Q.tiles = (uint32_t)((n + Q.tile - 1) / Q.tile);
+    Q.mean = std::max<uint32_t>(1u, (uint32_t)(Q.tile / Q.parts));
+    {
+        void* args[] = {(void*)&d_keys, (void*)&n, (void*)&Dc, (void*)&Q};
+        const void* fn = hot ? (small ? (const void*)k_part_split<512, 4, true> : (const void*)k_part_split<1024, 16, true>)
+                             : (small ? (const void*)k_part_split<512, 4, false> : (const void*)k_part_split<1024, 16, false>);
+        const int grid = (int)std::min<uint64_t>(Q.tiles, (uint64_t)(small ? 2 * L.num_sms : L.num_sms));
+        const cudaError_t e = cudaLaunchKernel(fn, dim3(grid), dim3(small ? 512 : 1024), args,
+                                               split_smem(Q.tile, Q.parts, hot), st);
+        if (e != cudaSuccess) return e;
+    }
+    void* args[] = {(void*)&Dc, (void*)&Q};
+    const void* fn = L.wide ? (const void*)k_part_apply<true> : (const void*)k_part_apply<false>;
+    cudaError_t e = cudaLaunchKernel(fn, dim3(Q.parts), dim3(AP_THREADS), args, L.apply_smem, st);
+    if (e != cudaSuccess) return e;
+    const uint64_t nq = ((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK;
+    return cudaLaunchKernel((const void*)k_part_link, dim3(L.num_sms), dim3(AP_THREADS), args, (size_t)nq * 4, st);
+}
+
+}  // namespace qsb
