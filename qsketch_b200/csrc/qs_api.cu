@@ -88,11 +88,16 @@ namespace qsb {
 void set_last_error(const char* text) { g_err = text; }
 }  // namespace qsb
 
+constexpr uint64_t SEEN_UNKNOWN = 1ull << 62;
+
 struct qs_sketch {
     qs_params p{};
     int device = 0;
     uint32_t kind = 0;
     uint64_t max_batch = 0;
+    uint64_t seen = 0;        // keys inserted since create / clear, or SEEN_UNKNOWN: bounds every
+                              // u32 counter (a key adds at most 4 to one, see high_increments)
+    bool arena = false;       // the tables of a batch
     uint64_t fresh = 0;       // keys inserted since create / clear (drives the chunk-size ramp)
     uint64_t ramp_first = 0;  // first chunk of the ramp, 0 = no ramp
     int agg = 1;
@@ -252,6 +257,7 @@ uint64_t part_chunk(const qs_sketch* sk, uint64_t rest) {
 // replay.
 qs_status insert_device(qs_sketch* sk, const uint32_t* d_keys, size_t n, cudaStream_t st,
                         const uint32_t* skip = nullptr, const TableDev* table = nullptr, uint32_t* skipbuf = nullptr) {
+    sk->seen = std::min(sk->seen + n, SEEN_UNKNOWN);
     if (sk->kind == QS_KIND_MSWS) {
         bool hot = false;  // the call's heavy keys are sampled
         for (size_t off = 0; off < n;) {
@@ -667,10 +673,11 @@ qs_status qs_remove(qs_sketch* sk, const uint32_t* d_keys, size_t n, void* strea
     if ((reinterpret_cast<uintptr_t>(d_keys) & 3u) != 0) return fail(QS_ERR_INVALID_ARG, "keys not 4-byte aligned");
     DeviceGuard guard(sk->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool low = sk->seen < (1ull << 29) && n < (1ull << 31);
     if (sk->kind == QS_KIND_MSWS)
-        CK(msws_remove(d_keys, n, sk->D, sk->L, st), "msws remove");
+        CK(msws_remove(d_keys, n, sk->D, sk->L, low, st), "msws remove");
     else
-        CK(cm_remove(d_keys, n, sk->C, sk->cm_grid, sk->D.ctl ? &sk->D.ctl->status : nullptr, st), "cm remove");
+        CK(cm_remove(d_keys, n, sk->C, sk->cm_grid, low, sk->D.ctl ? &sk->D.ctl->status : nullptr, st), "cm remove");
     return QS_OK;
 }
 
@@ -737,6 +744,7 @@ qs_status qs_clear(qs_sketch* sk, void* stream) {
     if (!sk) return fail(QS_ERR_INVALID_ARG, "null sketch");
     DeviceGuard guard(sk->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    sk->seen = sk->arena ? SEEN_UNKNOWN : 0;
     if (sk->kind == QS_KIND_MSWS) {
         CK(cudaMemsetAsync(sk->D.low, 0, sk->D.n_low * LOW_WORDS * 4, st), "clear low");
         CK(cudaMemsetAsync(sk->D.high, 0, sk->D.n_high * HIGH_WORDS * 4, st), "clear high");
@@ -1017,6 +1025,7 @@ qs_status qs_snapshot_load(const void* h_buf, uint64_t bytes, int32_t device, qs
         if (e == cudaSuccess) e = cudaMemcpy(sk->D.ctl, &c, sizeof c, cudaMemcpyHostToDevice);
         sk->fresh = sk->max_batch;  // a warm sketch: no chunk ramp
     }
+    sk->seen = SEEN_UNKNOWN;
     if (e != cudaSuccess) {
         qs_destroy(sk);
         return cuda_fail(e, "snapshot upload");
@@ -1887,6 +1896,8 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
         return st;
     };
     qs_sketch* sk = b->sk;
+    sk->arena = true;
+    sk->seen = SEEN_UNKNOWN;  // the batch's inserts do not go through the arena sketch's
     DeviceGuard guard(sk->device);
     b->seeds.resize(S);
     if (p->hash_seeds)

@@ -53,9 +53,11 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
                         bool hot, cudaStream_t st);
 
 cudaError_t cm_insert(const uint32_t* d_keys, uint64_t n, const CmDev& D, int agg, int grid, cudaStream_t st);
-// REMOVE (qs_remove.cu): one occurrence of each key out, counters floored at 0.
-cudaError_t msws_remove(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const MswsLaunch& L, cudaStream_t st);
-cudaError_t cm_remove(const uint32_t* d_keys, uint64_t n, const CmDev& D, int grid, uint32_t* d_status,
+// REMOVE (qs_remove.cu): one occurrence of each key out, counters floored at 0.  below_2_31: no u32
+// counter can hold 2^31 or more (and n is below 2^31).
+cudaError_t msws_remove(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const MswsLaunch& L, bool below_2_31,
+                        cudaStream_t st);
+cudaError_t cm_remove(const uint32_t* d_keys, uint64_t n, const CmDev& D, int grid, bool below_2_31, uint32_t* d_status,
                       cudaStream_t st);
 cudaError_t cm_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, const CmDev& D, int grid, cudaStream_t st);
 
