@@ -487,6 +487,7 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         D.fm_mask = make_fastmod(H);
         D.seed = sk->seeds[0];
         D.n_masks = H;
+        for (uint32_t m : sk->masks) D.wide |= __builtin_popcount(m) != 3 ? 1u : 0u;
         D.compat_v3 = (p.flags & QS_FLAG_COMPAT_V3) ? 1u : 0u;
         D.route = route == 3 ? 0u : route;  // 0 in the kernel = adaptive per tile
         const uint64_t B = sk->max_batch;
@@ -554,7 +555,6 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         if (P.parts) {
             e = part_configure(&sk->PL, P.shift, P.parts, H, sk->L.num_sms);
             if (e != cudaSuccess) return bail(cuda_fail(e, "configure partitioned insert"));
-            for (uint32_t m : sk->masks) sk->PL.wide |= __builtin_popcount(m) != 3;
         }
         sk->L.lanes_per_key = (int)lpk;
         sk->L.tile_keys = (int)tile;

@@ -82,6 +82,7 @@ struct MswsDev {
     uint32_t seed;
     uint32_t n_masks;
     uint32_t compat_v3;
+    uint32_t wide;           // some mask does not select exactly three counters
     uint32_t flag_cap;       // capacity of flag_list / per-slot arrays
     // ordered-replay scratch
     uint32_t* flag_list;     // slot -> bucket

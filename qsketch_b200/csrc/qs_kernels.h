@@ -44,7 +44,6 @@ cudaError_t msws_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, cons
 struct PartLaunch {
     int num_sms = 0;
     size_t apply_smem = 0;
-    bool wide = false;  // some mask does not select exactly three counters
 };
 // The call's heavy keys (a sample of its n keys) into part.hot, for part_insert's `hot`.
 cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cudaStream_t st);

@@ -1592,69 +1592,107 @@ __global__ void __launch_bounds__(REPAIR_THREADS, 2) k_msws_repair(const uint32_
 constexpr int QRY_THREADS = 256;
 constexpr int QRY_KPT = 4;
 
-// The estimate from a key's low bucket words u (word 7 the index) and mask m, h4 holding its
-// first four selected high counters when the bucket is linked (calculation_s2_search,
-// device_sketch_v3.h:340-357, 397-402; search_high :293-307, 364-395): min over the selected
-// 8-bit counters, plus the min over the selected high counters if linked.
-__device__ __forceinline__ uint32_t msws_estimate(const MswsDev& D, const uint32_t (&u)[8], uint32_t m,
+// Byte i of the 28 counter bytes in words u[0..6]: one byte permute per pair of words, then two
+// selections by the pair (the words are registers, so no indexed access).  Three of these cost half
+// of masking and byte-wise minima over all seven words, which any other mask still takes; the
+// query is issue bound as much as it waits for L2: 2^24 keys on 8 MB 141.6 -> 132.8 us, on
+// 64 MB 177 -> 154 us (126 Gkeys/s; random 32-byte loads alone reach 209).
+__device__ __forceinline__ uint32_t counter_byte(const uint32_t (&u)[8], uint32_t i) {
+    const uint32_t s = i & 7u;
+    const uint32_t a = (i & 8u) ? __byte_perm(u[2], u[3], s) : __byte_perm(u[0], u[1], s);
+    const uint32_t b = (i & 8u) ? u[6] >> (8u * (i & 3u)) : __byte_perm(u[4], u[5], s);
+    return ((i & 16u) ? b : a) & 0xffu;
+}
+
+// The estimate from a key's low bucket words u (word 7 the index) and mask code q
+// (calculation_s2_search, device_sketch_v3.h:340-357, 397-402; search_high :293-307, 364-395): min
+// over the selected 8-bit counters, plus, if linked, the min over the selected high counters, of
+// which hi4 holds the first four (WIDE) or all three.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t msws_estimate(const MswsDev& D, const uint32_t (&u)[8], uint32_t q,
                                                   const uint32_t (&h4)[4]) {
-    uint32_t acc = 0xffffffffu;
+    uint32_t lo;
+    if (WIDE) {
+        uint32_t acc = 0xffffffffu;
 #pragma unroll
-    for (int w = 0; w < 7; ++w) {
-        const uint32_t sel = expand_nibble((m >> (4 * w)) & 0xfu) * 0xffu;
-        acc = __vminu4(acc, u[w] | ~sel);
+        for (int w = 0; w < 7; ++w) {
+            const uint32_t sel = expand_nibble((q >> (4 * w)) & 0xfu) * 0xffu;
+            acc = __vminu4(acc, u[w] | ~sel);
+        }
+        acc = __vminu4(acc, acc >> 16);
+        lo = min(acc & 0xffu, (acc >> 8) & 0xffu);
+    } else {
+        lo = min(min(counter_byte(u, q & 31u), counter_byte(u, (q >> 5) & 31u)), counter_byte(u, q >> 10));
     }
-    acc = __vminu4(acc, acc >> 16);
-    const uint32_t lo = min(acc & 0xffu, (acc >> 8) & 0xffu);
     const uint32_t ptr = u[7];
-    if (!(ptr > START && (uint64_t)(ptr - START) < D.n_high)) return lo;
-    uint32_t hi = min(min(h4[0], h4[1]), min(h4[2], h4[3]));
-    uint32_t mm = m;
+    if (!is_linked(D, ptr)) return lo;
+    uint32_t hi = min(min(h4[0], h4[1]), h4[2]);
+    if (WIDE) {
+        hi = min(hi, h4[3]);
+        uint32_t mm = q;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) mm &= mm - 1;
-    const uint32_t* hb = D.high + (uint64_t)(ptr - START) * HIGH_WORDS;
-    for (; mm; mm &= mm - 1) hi = min(hi, __ldg(hb + (__ffs(mm) - 1)));  // masks of more than four counters
+        for (int i = 0; i < 4; ++i) mm &= mm - 1;
+        const uint32_t* hb = D.high + (uint64_t)(ptr - START) * HIGH_WORDS;
+        for (; mm; mm &= mm - 1) hi = min(hi, __ldg(hb + (__ffs(mm) - 1)));  // masks of more than four counters
+    }
     return lo + hi;
 }
 
-__device__ __forceinline__ uint32_t msws_lookup(const MswsDev& D, const uint32_t* s_masks, uint32_t key,
-                                                uint32_t seed, const FastMod& fm_low, uint32_t base) {
-    const uint32_t hv = key * seed;
-    const uint32_t b = base + fast_mod(fm_low, hv);
-    const uint32_t m = s_masks[fast_mod(D.fm_mask, hv)];
-    const uint4* bp = reinterpret_cast<const uint4*>(D.low + (uint64_t)b * LOW_WORDS);
-    const uint4 a = __ldg(bp), c = __ldg(bp + 1);
-    const uint32_t u[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-    // min over the selected bytes (calculation_s2_search, device_sketch_v3.h:340-357,397-402)
-    uint32_t acc = 0xffffffffu;
-#pragma unroll
-    for (int w = 0; w < 7; ++w) {
-        const uint32_t sel = expand_nibble((m >> (4 * w)) & 0xfu) * 0xffu;
-        acc = __vminu4(acc, u[w] | ~sel);
-    }
-    acc = __vminu4(acc, acc >> 16);
-    const uint32_t lo = min(acc & 0xffu, (acc >> 8) & 0xffu);
-    const uint32_t ptr = u[7];
-    uint32_t hi = 0;
-    if (ptr > START && (uint64_t)(ptr - START) < D.n_high) {  // search_high, device_sketch_v3.h:293-307, 364-395
-        // the first four selected counters as independent loads (no loop: the lookups of a
-        // thread's keys interleave), the rest of a wider mask after them
-        const uint32_t* hb = D.high + (uint64_t)(ptr - START) * HIGH_WORDS;
-        uint32_t mm = m, h4[4];
+// The first four (WIDE) or the three selected high counters of a linked bucket, as independent
+// loads; all ones where there is none.
+template <bool WIDE>
+__device__ __forceinline__ void high_counters(const MswsDev& D, uint32_t ptr, uint32_t q, uint32_t (&h4)[4]) {
+    const bool linked = is_linked(D, ptr);
+    const uint32_t* hb = D.high + (uint64_t)(linked ? ptr - START : 0u) * HIGH_WORDS;
+    if (WIDE) {
+        uint32_t mm = q;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            h4[i] = mm ? __ldg(hb + (__ffs(mm) - 1)) : 0xffffffffu;
+            h4[i] = (linked && mm) ? __ldg(hb + (__ffs(mm) - 1)) : 0xffffffffu;
             mm &= mm - 1;
         }
-        hi = min(min(h4[0], h4[1]), min(h4[2], h4[3]));
-        for (; mm; mm &= mm - 1) hi = min(hi, __ldg(hb + (__ffs(mm) - 1)));
+    } else {
+        h4[0] = linked ? __ldg(hb + (q & 31u)) : 0xffffffffu;
+        h4[1] = linked ? __ldg(hb + ((q >> 5) & 31u)) : 0xffffffffu;
+        h4[2] = linked ? __ldg(hb + (q >> 10)) : 0xffffffffu;
+        h4[3] = 0xffffffffu;
     }
-    return lo + hi;
 }
 
+template <bool WIDE>
+__device__ __forceinline__ void stage_codes(const MswsDev& D, uint32_t* s_codes) {
+    for (uint32_t i = threadIdx.x; i < D.n_masks; i += blockDim.x) s_codes[i] = mask_code<WIDE>(__ldg(D.masks + i));
+}
+
+// K keys of a thread, all of one sketch: the low buckets of all of them first, then the high
+// counters of the linked ones, so that the loads are in flight together at each level.
+template <bool WIDE, int K>
+__device__ __forceinline__ void msws_lookup(const MswsDev& D, const uint32_t* s_codes, const uint32_t (&k)[K],
+                                            uint32_t seed, const FastMod& fm_low, uint32_t base, uint32_t (&r)[K]) {
+    uint4 la[K], lc[K];
+    uint32_t q[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const uint32_t hv = k[j] * seed;
+        const uint4* bp = reinterpret_cast<const uint4*>(D.low + (uint64_t)(base + fast_mod(fm_low, hv)) * LOW_WORDS);
+        q[j] = s_codes[fast_mod(D.fm_mask, hv)];
+        la[j] = __ldg(bp);
+        lc[j] = __ldg(bp + 1);
+    }
+    uint32_t h4[K][4];
+#pragma unroll
+    for (int j = 0; j < K; ++j) high_counters<WIDE>(D, lc[j].w, q[j], h4[j]);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const uint32_t u[8] = {la[j].x, la[j].y, la[j].z, la[j].w, lc[j].x, lc[j].y, lc[j].z, lc[j].w};
+        r[j] = msws_estimate<WIDE>(D, u, q[j], h4[j]);
+    }
+}
+
+template <bool WIDE>
 __global__ void __launch_bounds__(QRY_THREADS) k_msws_query(const uint32_t* __restrict__ keys, uint64_t n,
                                                             uint32_t* __restrict__ out, MswsDev D) {
-    extern __shared__ __align__(16) uint32_t s_masks[];
+    extern __shared__ __align__(16) uint32_t s_codes[];
     griddep_wait();  // the previous kernel (an insert or its replay) has ended
     griddep_launch_dependents();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -1666,7 +1704,7 @@ __global__ void __launch_bounds__(QRY_THREADS) k_msws_query(const uint32_t* __re
         const uint64_t i = base + j * stride;
         k[j] = i < n ? __ldcs(keys + i) : 0u;
     }
-    for (uint32_t i = threadIdx.x; i < D.n_masks; i += blockDim.x) s_masks[i] = __ldg(D.masks + i);
+    stage_codes<WIDE>(D, s_codes);
     __syncthreads();
     for (; base < n; base += stride * QRY_KPT) {
         if (base != (uint64_t)blockIdx.x * blockDim.x + threadIdx.x) {
@@ -1676,36 +1714,7 @@ __global__ void __launch_bounds__(QRY_THREADS) k_msws_query(const uint32_t* __re
                 k[j] = i < n ? __ldcs(keys + i) : 0u;
             }
         }
-        // the low buckets of all QRY_KPT keys first, then the high counters of the linked ones,
-        // so the loads of the thread's keys are in flight together at each level
-        uint4 la[QRY_KPT], lc[QRY_KPT];
-        uint32_t m[QRY_KPT];
-#pragma unroll
-        for (int j = 0; j < QRY_KPT; ++j) {
-            const uint32_t hv = k[j] * D.seed;
-            const uint4* bp = reinterpret_cast<const uint4*>(D.low + (uint64_t)fast_mod(D.fm_low, hv) * LOW_WORDS);
-            m[j] = s_masks[fast_mod(D.fm_mask, hv)];
-            la[j] = __ldg(bp);
-            lc[j] = __ldg(bp + 1);
-        }
-        uint32_t h4[QRY_KPT][4];
-#pragma unroll
-        for (int j = 0; j < QRY_KPT; ++j) {
-            const uint32_t ptr = lc[j].w;
-            const bool linked = ptr > START && (uint64_t)(ptr - START) < D.n_high;
-            const uint32_t* hb = D.high + (uint64_t)(linked ? ptr - START : 0u) * HIGH_WORDS;
-            uint32_t mm = m[j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                h4[j][i] = (linked && mm) ? __ldg(hb + (__ffs(mm) - 1)) : 0xffffffffu;
-                mm &= mm - 1;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < QRY_KPT; ++j) {
-            const uint32_t u[8] = {la[j].x, la[j].y, la[j].z, la[j].w, lc[j].x, lc[j].y, lc[j].z, lc[j].w};
-            r[j] = msws_estimate(D, u, m[j], h4[j]);
-        }
+        msws_lookup<WIDE, QRY_KPT>(D, s_codes, k, D.seed, D.fm_low, 0u, r);
 #pragma unroll
         for (int j = 0; j < QRY_KPT; ++j) {
             const uint64_t i = base + j * stride;
@@ -1716,18 +1725,20 @@ __global__ void __launch_bounds__(QRY_THREADS) k_msws_query(const uint32_t* __re
 
 // Learned split query: exact count of a key in the heavy table (if admitted) plus the MSWS
 // estimate (its occurrences before admission live in the sketch).
+template <bool WIDE>
 __global__ void __launch_bounds__(QRY_THREADS) k_learned_query(const uint32_t* __restrict__ keys, uint64_t n,
                                                                TableDev T, uint32_t* __restrict__ out, MswsDev D) {
-    extern __shared__ __align__(16) uint32_t s_masks[];
-    for (uint32_t i = threadIdx.x; i < D.n_masks; i += blockDim.x) s_masks[i] = __ldg(D.masks + i);
+    extern __shared__ __align__(16) uint32_t s_codes[];
+    stage_codes<WIDE>(D, s_codes);
     __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint32_t key = __ldcs(keys + i);
-        uint32_t r = msws_lookup(D, s_masks, key, D.seed, D.fm_low, 0u);
-        const int s = table_find(T.keys, T.slots, key);
-        if (s >= 0) r += __ldcg(T.counts + s);
-        __stcs(out + i, r);
+        const uint32_t key[1] = {__ldcs(keys + i)};
+        uint32_t r[1];
+        const int s = table_find(T.keys, T.slots, key[0]);
+        msws_lookup<WIDE, 1>(D, s_codes, key, D.seed, D.fm_low, 0u, r);
+        if (s >= 0) r[0] += __ldcg(T.counts + s);
+        __stcs(out + i, r[0]);
     }
 }
 
@@ -1736,7 +1747,10 @@ cudaError_t learned_query(const uint32_t* d_keys, uint64_t n, const TableDev& T,
     if (n == 0) return cudaSuccess;
     const uint64_t want = (n + QRY_THREADS - 1) / QRY_THREADS;
     const int grid = (int)std::min<uint64_t>((uint64_t)L.query_grid, std::max<uint64_t>(1ull, want));
-    k_learned_query<<<grid, QRY_THREADS, (size_t)D.n_masks * 4, st>>>(d_keys, n, T, d_out, D);
+    if (D.wide)
+        k_learned_query<true><<<grid, QRY_THREADS, (size_t)D.n_masks * 4, st>>>(d_keys, n, T, d_out, D);
+    else
+        k_learned_query<false><<<grid, QRY_THREADS, (size_t)D.n_masks * 4, st>>>(d_keys, n, T, d_out, D);
     return cudaGetLastError();
 }
 
@@ -1904,11 +1918,12 @@ __global__ void __launch_bounds__(INS_THREADS, INS_MIN_CTAS) k_batch_insert(cons
 }
 
 // Query over a batch: static tiles, each stream's keys with its own descriptor.
+template <bool WIDE>
 __global__ void __launch_bounds__(QRY_THREADS) k_batch_query(const uint32_t* __restrict__ keys,
                                                              uint32_t* __restrict__ out, MswsDev D, BatchDev B) {
-    extern __shared__ __align__(16) uint32_t s_masks[];
+    extern __shared__ __align__(16) uint32_t s_codes[];
     __shared__ uint32_t s_stream;
-    for (uint32_t i = threadIdx.x; i < D.n_masks; i += blockDim.x) s_masks[i] = __ldg(D.masks + i);
+    stage_codes<WIDE>(D, s_codes);
     const uint32_t n_items = __ldcg(B.item_off + B.n_streams);
     for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
         if (threadIdx.x < 32) {
@@ -1931,10 +1946,17 @@ __global__ void __launch_bounds__(QRY_THREADS) k_batch_query(const uint32_t* __r
             k[j] = i < cnt ? __ldcs(keys + t0 + i) : 0u;
         }
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const uint32_t i = threadIdx.x + j * QRY_THREADS;
-            const uint32_t r = msws_lookup(D, s_masks, k[j], seed, fm, base);
-            if (i < cnt) __stcs(out + t0 + i, r);
+        for (int h = 0; h < PER / QRY_KPT; ++h) {
+            uint32_t kk[QRY_KPT], r[QRY_KPT];
+#pragma unroll
+            for (int j = 0; j < QRY_KPT; ++j) kk[j] = k[h * QRY_KPT + j];
+            if (h * QRY_KPT * QRY_THREADS >= cnt) break;
+            msws_lookup<WIDE, QRY_KPT>(D, s_codes, kk, seed, fm, base, r);
+#pragma unroll
+            for (int j = 0; j < QRY_KPT; ++j) {
+                const uint32_t i = threadIdx.x + (h * QRY_KPT + j) * QRY_THREADS;
+                if (i < cnt) __stcs(out + t0 + i, r[j]);
+            }
         }
     }
 }
@@ -1991,12 +2013,12 @@ cudaError_t msws_configure(int device, uint32_t n_masks, MswsLaunch* L) {
                     if (e != cudaSuccess) return e;
                 }
             }
-    e = cudaFuncSetAttribute((const void*)k_msws_query, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute((const void*)k_learned_query, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute((const void*)k_batch_query, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4);
-    if (e != cudaSuccess) return e;
+    for (const void* fn : {(const void*)k_msws_query<false>, (const void*)k_msws_query<true>,
+                           (const void*)k_learned_query<false>, (const void*)k_learned_query<true>,
+                           (const void*)k_batch_query<false>, (const void*)k_batch_query<true>}) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4);
+        if (e != cudaSuccess) return e;
+    }
     int occ = 0;
     L->insert_grid = prop.multiProcessorCount * std::max(1, L->ins_occ[AGG_BLOCK][1]);
     for (const void* fn : {(const void*)k_msws_repair<false>, (const void*)k_msws_repair<true>}) {
@@ -2101,7 +2123,10 @@ cudaError_t batch_repair(const uint32_t* d_window, const MswsDev& D, const Batch
 
 cudaError_t batch_query(const uint32_t* d_keys, uint32_t* d_out, const MswsDev& D, const BatchDev& B,
                         const MswsLaunch& L, cudaStream_t st) {
-    k_batch_query<<<L.query_grid, QRY_THREADS, (size_t)D.n_masks * 4, st>>>(d_keys, d_out, D, B);
+    if (D.wide)
+        k_batch_query<true><<<L.query_grid, QRY_THREADS, (size_t)D.n_masks * 4, st>>>(d_keys, d_out, D, B);
+    else
+        k_batch_query<false><<<L.query_grid, QRY_THREADS, (size_t)D.n_masks * 4, st>>>(d_keys, d_out, D, B);
     return cudaGetLastError();
 }
 
@@ -2112,7 +2137,8 @@ cudaError_t msws_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, cons
     const int grid = (int)umin64((uint64_t)L.query_grid, std::max<uint64_t>(1ull, want));
     MswsDev Dc = D;
     void* args[] = {(void*)&d_keys, (void*)&n, (void*)&d_out, (void*)&Dc};
-    return launch_pdl((const void*)k_msws_query, dim3(grid), dim3(QRY_THREADS), (size_t)D.n_masks * 4, st, args, false);
+    const void* fn = D.wide ? (const void*)k_msws_query<true> : (const void*)k_msws_query<false>;
+    return launch_pdl(fn, dim3(grid), dim3(QRY_THREADS), (size_t)D.n_masks * 4, st, args, false);
 }
 
 }  // namespace qsb

@@ -236,19 +236,6 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
 
 // ---- 2: one partition per block ------------------------------------------------------------
 
-// A mask table of three counters per mask (the default) is kept as the counters' numbers, 5 bits
-// each; any other (WIDE) as the masks.
-template <bool WIDE>
-__device__ __forceinline__ uint32_t mask_code(uint32_t m) {
-    if (WIDE) return m;
-    const uint32_t a = __ffs(m) - 1, m1 = m & (m - 1), b = __ffs(m1) - 1, c = __ffs(m1 & (m1 - 1)) - 1;
-    return a | b << 5 | c << 10;
-}
-template <bool WIDE>
-__device__ __forceinline__ uint32_t code_mask(uint32_t q) {
-    return WIDE ? q : (1u << (q & 31u)) | (1u << ((q >> 5) & 31u)) | (1u << (q >> 10));
-}
-
 struct ApShared {
     uint32_t* tab;             // [2^shift][8] the partition's buckets (word 7: flagged buckets by slot)
     uint32_t* w7;              // [2^shift] their index words
@@ -950,7 +937,7 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
         if (e != cudaSuccess) return e;
     }
     void* args[] = {(void*)&Dc, (void*)&Q};
-    const void* fn = L.wide ? (const void*)k_part_apply<true> : (const void*)k_part_apply<false>;
+    const void* fn = D.wide ? (const void*)k_part_apply<true> : (const void*)k_part_apply<false>;
     cudaError_t e = cudaLaunchKernel(fn, dim3(Q.parts), dim3(AP_THREADS), args, L.apply_smem, st);
     if (e != cudaSuccess) return e;
     const uint64_t nq = ((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK;

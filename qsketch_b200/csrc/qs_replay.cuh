@@ -13,6 +13,19 @@ __device__ __forceinline__ bool is_linked(const MswsDev& D, uint32_t w7) {
     return w7 > START && (uint64_t)(w7 - START) < D.n_high;
 }
 
+// A mask table of three counters per mask (the default) is kept as the counters' numbers, 5 bits
+// each; any other (WIDE) as the masks.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t mask_code(uint32_t m) {
+    if (WIDE) return m;
+    const uint32_t a = __ffs(m) - 1, m1 = m & (m - 1), b = __ffs(m1) - 1, c = __ffs(m1 & (m1 - 1)) - 1;
+    return a | b << 5 | c << 10;
+}
+template <bool WIDE>
+__device__ __forceinline__ uint32_t code_mask(uint32_t q) {
+    return WIDE ? q : (1u << (q & 31u)) | (1u << ((q >> 5) & 31u)) | (1u << (q >> 10));
+}
+
 // Does a selected byte (nibble bit k selects byte k) of the pre-add word `old` reach CROSS
 // once c is added: byte + c >= CROSS, i.e. byte >= CROSS - c, four bytes at a time.
 // Selected bytes all below 64 with c below 64 cannot reach CROSS: a two-operation test
