@@ -384,7 +384,9 @@ qs_status qs_draw_seeds(uint32_t rng_seed, size_t count, uint32_t* out) {
     return QS_OK;
 }
 
-qs_status qs_create(const qs_params* params, qs_sketch** out) {
+// arena_chunk (batch arenas only, else 0): keys of the batch's partitioned windows; the arena's own
+// bucket ranges are not partitioned.
+static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_t arena_chunk) {
     if (!params || !out) return fail(QS_ERR_INVALID_ARG, "qs_create: null argument");
     *out = nullptr;
     const qs_params& p = *params;
@@ -509,8 +511,9 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         // against 269 (85 / 139); 2^22 keys into 64 MB 168 against 273 (124 / 145), but 2^20 174
         // against 141 (73 / 49).
         sk->part_min = std::max<uint64_t>(1ull << 18, n_low + n_low / 2);
-        const uint64_t reach = P.parts ? std::max(B, sk->part_cap) : B;  // keys of the largest chunk
-        const uint64_t cap = std::min<uint64_t>(n_low, reach);
+        if (arena_chunk) P.parts = 0;
+        const uint64_t reach = std::max(B, P.parts ? sk->part_cap : arena_chunk);  // keys of the largest chunk
+        const uint64_t cap = std::min<uint64_t>(n_low, B), links = std::min<uint64_t>(n_low, reach);
         D.flag_cap = (uint32_t)cap;
         D.max_tiles = (uint32_t)((B + REPAIR_TILE - 1) / REPAIR_TILE);
         D.long_cap = (uint32_t)std::min<uint64_t>(cap, 1ull << 16);  // slots with grid-computed totals
@@ -520,7 +523,7 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         CKB(sk->alloc(&masks_d, H), "alloc masks");
         D.masks = masks_d;
         CKB(sk->alloc(&D.ctl, 1), "alloc control");
-        CKB(sk->alloc(&D.flag_list, cap), "alloc flag list");
+        CKB(sk->alloc(&D.flag_list, links), "alloc flag list");
         CKB(sk->alloc(&D.tile_counts, D.max_tiles), "alloc tile counts");
         // one block: the replay's records and their positions (24 B per key of max_batch), or a
         // partitioned chunk's entries and key indices (6 B per key of up to 4 max_batch)
@@ -530,9 +533,9 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         D.rec[1] = reinterpret_cast<uint2*>(rb + 2 * B);
         D.rpos[0] = rb + 4 * B;
         D.rpos[1] = rb + 5 * B;
+        P.ent = rb;
+        P.idx = reinterpret_cast<uint16_t*>(rb + sk->part_cap);
         if (P.parts) {
-            P.ent = rb;
-            P.idx = reinterpret_cast<uint16_t*>(rb + sk->part_cap);
             // tiles of a chunk: whole ones, or the small ones of a chunk below PART_SMALL_MAX keys
             P.stride = (uint32_t)std::max(sk->part_cap / PART_TILE,
                                           std::min(sk->part_cap, PART_SMALL_MAX) / PART_TILE_SMALL);
@@ -542,7 +545,7 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         CKB(sk->alloc(&D.hist, (uint64_t)256 * D.max_tiles + 256), "alloc histograms");  // + digit totals
         CKB(sk->alloc(&D.seg_beg, cap), "alloc segments");
         CKB(sk->alloc(&D.totals, (uint64_t)D.long_cap * LOW_COUNTERS), "alloc totals");
-        CKB(sk->alloc(&D.sw, cap), "alloc link order");
+        CKB(sk->alloc(&D.sw, links), "alloc link order");
         CKB(sk->alloc(&D.sw_base, cap), "alloc link order");
         CKB(sk->alloc(&D.sw_bits, (reach + 31) / 32), "alloc link order");
         CKB(sk->alloc(&D.sw_cnt, (reach + SW_BLOCK - 1) / SW_BLOCK), "alloc link order");
@@ -552,9 +555,10 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
         CKB(cudaStreamSynchronize(0), "create sync");
         e = msws_configure(dev, H, &sk->L);
         if (e != cudaSuccess) return bail(cuda_fail(e, "configure kernels"));
-        if (P.parts) {
-            e = part_configure(&sk->PL, P.shift, P.parts, H, sk->L.num_sms);
+        if (P.parts || arena_chunk) {
+            e = part_configure(sk->L.num_sms, &sk->PL);
             if (e != cudaSuccess) return bail(cuda_fail(e, "configure partitioned insert"));
+            sk->PL.apply_smem = part_apply_smem(P.shift, H);
         }
         sk->L.lanes_per_key = (int)lpk;
         sk->L.tile_keys = (int)tile;
@@ -634,6 +638,8 @@ qs_status qs_create(const qs_params* params, qs_sketch** out) {
     *out = sk;
     return QS_OK;
 }
+
+qs_status qs_create(const qs_params* params, qs_sketch** out) { return create_sketch(params, out, 0); }
 
 qs_status qs_destroy(qs_sketch* sk) {
     if (!sk) return QS_OK;
@@ -1733,6 +1739,11 @@ struct qs_batch {
     // Pass 1 runs one launch per run of size classes with the same lanes per key; streams are
     // grouped by size class floor(log2 n_low) (the grouped order lives in B.cls_streams).
     std::vector<uint32_t> grp_class;   // size class of each grouped position
+    // partitioned insert of the streams with enough keys (batch_dense)
+    std::vector<uint32_t> part_off;    // [S + 1] prefix of the streams' partitions (empty: not used)
+    std::vector<uint32_t> n_low;       // [S]
+    PartDev P{};
+    uint64_t run_cap = 0;              // run bounds a window can have
     uint32_t class_lpk[MAX_SIZE_CLASSES] = {};
     struct Run {
         uint32_t k_lo, k_hi;
@@ -1780,6 +1791,78 @@ qs_status batch_insert_seq(qs_batch* b, const uint32_t* d_keys, const uint64_t* 
     CK(batch_repair(d_keys, sk->D, B, sk->L, st), "batch repair");
     if (timed) CK(sk->prof_end(1, st), "profile");
     b->info.launches += 3;
+    return QS_OK;
+}
+
+// The partitioned insert of the dense streams: windows of as many streams as the scratch holds.
+qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t* d_offsets,
+                             const std::vector<uint64_t>& off, const std::vector<char>& dense, cudaStream_t st) {
+    qs_sketch* sk = b->sk;
+    BatchDev B = b->B;
+    B.key_off = d_offsets;
+    const uint64_t first = 1ull << 14;
+    // one window: the streams [s_lo, s_hi), each stream's keys [r0, r1)
+    auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1, bool small) -> qs_status {
+        const uint64_t tile = small ? PART_TILE_SMALL : PART_TILE;
+        uint64_t tiles = 0;
+        for (uint32_t i = s_lo; i < s_hi; ++i) {
+            const uint64_t len = dense[i] ? off[i + 1] - off[i] : 0;
+            tiles += (std::min(len, r1) - std::min(len, r0) + tile - 1) / tile;
+        }
+        BatchWindow W{};
+        W.s_lo = s_lo;
+        W.s_hi = s_hi;
+        W.rel_lo = r0;
+        W.rel_hi = r1;
+        W.which = STREAMS_DENSE;
+        const bool hot = r0 > 0;
+        CK(sk->prof_begin(0, st), "profile");
+        CK(part_insert_batch(d_keys, sk->D, b->P, B, sk->PL, W, (uint32_t)tiles, b->part_off[s_lo], b->part_off[s_hi],
+                             small, hot, st),
+           "partitioned batch insert");
+        CK(sk->prof_end(0, st), "profile");
+        b->info.launches += hot ? 5 : 4;
+        return QS_OK;
+    };
+    for (int round = 0; round < 2; ++round) {
+        const uint64_t r0 = round ? first : 0, r1 = round ? ~0ull : first;
+        uint64_t slots = 0, keys = 0, runs = 0;
+        uint32_t lo = 0;
+        auto close = [&](uint32_t hi) -> qs_status {
+            qs_status s = QS_OK;
+            // tiles of 2048 keys in the first round (a heavy key's run of a tile stays within a
+            // unit), and while larger ones would leave SMs idle
+            if (keys) s = run(lo, hi, r0, r1, !round);
+            slots = keys = runs = 0;
+            lo = hi;
+            return s;
+        };
+        const uint64_t tile = round ? PART_TILE : PART_TILE_SMALL;
+        for (uint32_t i = 0; i < b->S; ++i) {
+            const uint64_t len = dense[i] ? off[i + 1] - off[i] : 0, part = std::min(len, r1) - std::min(len, r0);
+            const uint64_t parts = b->part_off[i + 1] - b->part_off[i];
+            if (part > sk->part_cap) {  // one stream's slice alone exceeds a window: split it
+                qs_status s = close(i);
+                if (s != QS_OK) return s;
+                for (uint64_t a = r0; a < len; a += sk->part_cap) {
+                    s = run(i, i + 1, a, std::min(len, a + sk->part_cap), false);
+                    if (s != QS_OK) return s;
+                }
+                lo = i + 1;
+                continue;
+            }
+            const uint64_t t = (part + tile - 1) / tile;
+            if (slots + t * tile > sk->part_cap || runs + t * (parts + 1) > b->run_cap) {
+                const qs_status s = close(i);
+                if (s != QS_OK) return s;
+            }
+            slots += t * tile;
+            keys += part;
+            runs += t * (parts + 1);
+        }
+        const qs_status s = close(b->S);
+        if (s != QS_OK) return s;
+    }
     return QS_OK;
 }
 
@@ -1885,7 +1968,12 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
     ap.lanes_per_key = p->lanes_per_key;
     ap.ctas_per_sm = p->ctas_per_sm;
     qs_batch* b = new qs_batch();
-    qs_status s = qs_create(&ap, &b->sk);
+    const bool own_knobs = p->lanes_per_key || p->aggregate || p->route || p->ctas_per_sm || p->class_lanes_per_key ||
+                           p->first_chunk || (p->flags & QS_FLAG_NO_CHUNK_RAMP);
+    const uint64_t mb = p->max_batch ? p->max_batch : (1ull << 22);
+    const bool part = !own_knobs && mb >= PART_TILE && th < (1ull << 28) && p->hash_mask_table_sz <= PART_MAX_MASKS;
+    const uint64_t part_cap = part ? std::min<uint64_t>(mb * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE : 0;
+    qs_status s = create_sketch(&ap, &b->sk, part_cap);
     if (s != QS_OK) {
         delete b;
         return s;
@@ -1916,8 +2004,40 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
         lb += p->n_low[i];
         hb += p->n_high[i];
     }
+    if (part) {
+        // 64 partitions of a stream's sketch where that leaves 16 buckets to each (several
+        // blocks then share even a small sketch's keys), 2048 buckets to each of a large one
+        b->part_off.assign(S + 1, 0);
+        b->n_low.resize(S);
+        size_t smem = 0;
+        for (uint32_t i = 0; i < S; ++i) {
+            uint32_t sh = 4;
+            while (sh < PART_MAX_SHIFT && (p->n_low[i] >> sh) >= 64) ++sh;
+            const uint64_t parts = (p->n_low[i] + (1ull << sh) - 1) >> sh;
+            desc[i].shift = sh;
+            desc[i].parts = parts >= 4 && parts <= PART_MAX_PARTS ? (uint32_t)parts : 0u;
+            b->n_low[i] = (uint32_t)p->n_low[i];
+            b->part_off[i + 1] = b->part_off[i] + desc[i].parts;
+            if (desc[i].parts) smem = std::max(smem, part_apply_smem(sh, p->hash_mask_table_sz));
+        }
+        sk->PL.apply_smem = smem;
+        sk->part_cap = part_cap;
+        b->P = sk->P;
+        for (uint32_t i = 0; i < S; ++i) b->P.parts = std::max(b->P.parts, desc[i].parts);  // sizes the split's counts
+        b->run_cap = part_cap / PART_TILE_SMALL * 520;
+        CKB(sk->alloc(&b->P.off, b->run_cap), "alloc run bounds");
+    }
     BatchDev& B = b->B;
     B.n_streams = S;
+    if (part) {
+        uint32_t* d_off = nullptr;
+        CKB(sk->alloc(&d_off, (uint64_t)S + 1), "alloc partitions");
+        CKB(cudaMemcpy(d_off, b->part_off.data(), ((size_t)S + 1) * 4, cudaMemcpyHostToDevice), "upload partitions");
+        B.part_off = d_off;
+        CKB(sk->alloc(&B.run_off, (uint64_t)S + 1), "alloc run prefix");
+        CKB(sk->alloc(&B.base_id, S), "alloc allocators");
+        CKB(sk->alloc(&B.hot, (uint64_t)S * BATCH_HOT), "alloc heavy keys");
+    }
     StreamDesc* d_desc = nullptr;
     CKB(sk->alloc(&d_desc, S), "alloc stream descriptors");
     B.desc = d_desc;
@@ -2018,8 +2138,26 @@ qs_status qs_batch_insert(qs_batch* b, const uint32_t* d_keys, const uint64_t* d
         ++b->info.inserts;
         return QS_OK;
     }
+    // streams with enough keys: partitioned, their first keys in a round of their own (heavy keys
+    // link in it), then the rest; the others below
+    std::vector<char> dense(S, 0);
+    bool any_dense = false, any_sparse = false;
+    for (uint32_t i = 0; i < S; ++i) {
+        dense[i] = !b->part_off.empty() &&
+                   batch_dense(off[i + 1] - off[i], b->n_low[i], b->part_off[i + 1] - b->part_off[i]);
+        (dense[i] ? any_dense : any_sparse) = true;
+    }
+    if (any_dense) {
+        s = batch_insert_dense(b, d_keys, d_offsets, off, dense, st);
+        if (s != QS_OK) return s;
+        if (!any_sparse) {
+            ++b->info.inserts;
+            return QS_OK;
+        }
+    }
     uint64_t longest = 0;
-    for (uint32_t i = 0; i < S; ++i) longest = std::max(longest, off[i + 1] - off[i]);
+    for (uint32_t i = 0; i < S; ++i)
+        if (!dense[i]) longest = std::max(longest, off[i + 1] - off[i]);
     auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1) -> qs_status {
         BatchWindow W{};
         W.s_lo = s_lo;
@@ -2027,13 +2165,14 @@ qs_status qs_batch_insert(qs_batch* b, const uint32_t* d_keys, const uint64_t* d
         W.rel_lo = r0;
         W.rel_hi = r1;
         W.flat = 0;
+        W.which = any_dense ? STREAMS_SPARSE : STREAMS_ALL;
         return batch_insert_seq(b, d_keys, d_offsets, W, false, st);
     };
     for (uint64_t r0 = 0, r1 = b->ramp_first; r0 < longest; r0 = r1, r1 = std::max(r1 * 2, r1 + 1)) {
         uint64_t acc = 0;
         uint32_t first = 0;
         for (uint32_t i = 0; i <= S; ++i) {
-            const uint64_t len = i < S ? off[i + 1] - off[i] : 0;
+            const uint64_t len = i < S && !dense[i] ? off[i + 1] - off[i] : 0;
             const uint64_t part = i < S ? std::min(len, r1) - std::min(len, r0) : 0;
             if (i == S || acc + part > mb) {  // close the window [first, i)
                 if (acc) {

@@ -127,7 +127,7 @@ struct PartDev {
     uint32_t parts;
     uint32_t tiles;   // this chunk's tiles, of `tile` keys
     uint32_t tile;
-    uint32_t mean;    // entries per run when they spread evenly
+    uint32_t part0;   // batch: the window's first partition among all streams'
 };
 constexpr uint32_t PART_TILE = 16384, PART_TILE_SMALL = 2048;
 constexpr uint64_t PART_SMALL_MAX = 148ull * PART_TILE;  // chunks below this many keys take small tiles
@@ -148,6 +148,8 @@ struct StreamDesc {
     uint32_t low_base;   // first bucket of the stream's sketch in the low arena
     uint32_t high_base;  // global high id = high_base + the stream's own id (from FIRST_ID)
     uint32_t n_high;     // the stream's pool size in buckets (own ids < START + n_high)
+    uint32_t shift;      // partitioned insert: 2^shift buckets to a partition
+    uint32_t parts;      // and the stream's partitions
 };
 
 struct BatchDev {
@@ -166,9 +168,15 @@ struct BatchDev {
     uint32_t* status;         // [n_streams] latched ST_* bits per stream
     unsigned long long* first;// [n_streams] (repair generation << 32) | ~(lowest rank of the
                               // stream's links in that repair): ranks within each stream
+    // partitioned insert (its plan fills item_off with its own tiles)
+    const uint32_t* part_off; // [n_streams + 1] prefix of the streams' partitions
+    uint32_t* run_off;        // [n_streams + 1] prefix of the streams' run bounds in PartDev::off
+    uint32_t* base_id;        // [n_streams] next_id when the window began
+    uint32_t* hot;            // [n_streams][BATCH_HOT] heavy keys of the window
     uint32_t n_streams;       // 0: not a batch
     uint32_t pad;
 };
+constexpr uint32_t BATCH_HOT = 128;
 
 // Which keys one batched launch sequence covers: flat mode, the keys [c0, c1) of the caller's
 // flat array; else, for the streams [s_lo, s_hi), each stream's keys [rel_lo, rel_hi) counted
@@ -178,8 +186,14 @@ struct BatchWindow {
     uint64_t rel_lo, rel_hi;
     uint32_t s_lo, s_hi;
     uint32_t flat;
-    uint32_t pad;
+    uint32_t which;  // all streams, or only the dense or the sparse ones (batch_dense)
 };
+enum { STREAMS_ALL = 0, STREAMS_DENSE = 1, STREAMS_SPARSE = 2 };
+// Streams whose keys go through the partitioned insert: at least two keys to a bucket and 2^15 keys
+// in the call.
+__host__ __device__ __forceinline__ bool batch_dense(uint64_t keys, uint32_t n_low, uint32_t parts) {
+    return parts && keys >= (1ull << 15) && keys >= n_low;
+}
 
 // Plain count-min (rows x n counters, one seed per row) or, when `masks` is set, a one-level
 // bucket sketch: n buckets of `rows` u32 counters, a key's mask (of rows bits) selecting its

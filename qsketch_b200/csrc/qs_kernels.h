@@ -45,11 +45,17 @@ struct PartLaunch {
     int num_sms = 0;
     size_t apply_smem = 0;
 };
+cudaError_t part_configure(int num_sms, PartLaunch* L);
+size_t part_apply_smem(uint32_t shift, uint32_t n_masks);
 // The call's heavy keys (a sample of its n keys) into part.hot, for part_insert's `hot`.
 cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cudaStream_t st);
-cudaError_t part_configure(PartLaunch* L, uint32_t shift, uint32_t parts, uint32_t n_masks, int num_sms);
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
                         bool hot, cudaStream_t st);
+// The same for a window of a batch: `tiles` tiles (small or large) of the streams W names, whose
+// partitions are [part_lo, part_hi) of all streams'; hot: each stream's heavy keys are sampled.
+cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const PartDev& part, const BatchDev& B,
+                              const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t part_lo,
+                              uint32_t part_hi, bool small, bool hot, cudaStream_t st);
 
 cudaError_t cm_insert(const uint32_t* d_keys, uint64_t n, const CmDev& D, int agg, int grid, cudaStream_t st);
 // REMOVE (qs_remove.cu): one occurrence of each key out, counters floored at 0.  below_2_31: no u32

@@ -632,19 +632,6 @@ __device__ __forceinline__ uint32_t stream_of_window_key(const BatchDev& B, uint
     return lo;
 }
 
-// The stream whose bucket range holds global bucket g (bases strictly increase).
-__device__ __forceinline__ uint32_t stream_of_bucket(const BatchDev& B, uint32_t g) {
-    uint32_t lo = 0, hi = B.n_streams;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&B.desc[mid].low_base) <= g)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
 // The repair's key passes: one sketch whose chunk is `keys[0, n)`, or a batch window whose key
 // i lies in stream s at flat index lo[s] + i - wpre[s]; a thread walks window keys in
 // increasing order, so the stream cursor only moves forward.
@@ -1782,7 +1769,7 @@ __global__ void __launch_bounds__(1024) k_batch_plan(BatchDev B, BatchWindow W, 
         } else if (W.flat) {
             lo = umin64(e, max(o0, b0));
             hi = umin64(e, max(o1, lo));
-        } else if (s >= W.s_lo && s < W.s_hi) {
+        } else if (s >= W.s_lo && s < W.s_hi && in_window(B, W, s, o1 - o0)) {
             const uint64_t len = o1 - o0;
             lo = o0 + umin64(W.rel_lo, len);
             hi = o0 + umin64(W.rel_hi, len);
@@ -1814,24 +1801,6 @@ __global__ void __launch_bounds__(1024) k_batch_plan(BatchDev B, BatchWindow W, 
         if (bad) atomicOr(&ctl->status, ST_BAD_OFFSETS);
         if (strict && !bad && total > W.c1) atomicOr(&ctl->status, ST_CAPACITY);
     }
-}
-
-// The stream of work item `it` (< item_off[n_streams]): the last s with item_off[s] <= it.
-// Called by a whole warp: each step probes 32 evenly spaced offsets, so 512 streams take two
-// dependent loads instead of nine.
-__device__ __forceinline__ uint32_t stream_of_item_warp(const BatchDev& B, uint32_t it) {
-    const int lane = threadIdx.x & 31;
-    uint32_t lo = 0, hi = B.n_streams;  // item_off[lo] <= it; the answer lies in [lo, hi)
-    while (hi - lo > 1) {
-        const uint32_t step = (hi - lo + 31) / 32;
-        const uint32_t idx = lo + lane * step;
-        const bool le = idx < hi && __ldcg(B.item_off + idx) <= it;
-        const uint32_t bal = __ballot_sync(0xffffffffu, le);  // lane 0 always holds
-        const uint32_t last = 31 - __clz(bal);
-        lo += last * step;
-        hi = min(hi, lo + step);
-    }
-    return lo;
 }
 
 // The grouped index k in [k_lo, k_hi) whose items hold work item `it` (cls_item_off[k] <=

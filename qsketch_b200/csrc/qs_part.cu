@@ -107,50 +107,178 @@ __global__ void __launch_bounds__(HOT_THREADS) k_part_hot(const uint32_t* __rest
     for (uint32_t i = tid; i < 2 * SETS; i += HOT_THREADS) hot[2 * set0 + i] = s_hot[i];
 }
 
+// ---- the sketch a tile or a partition belongs to ----------------------------------------------
+
+// One sketch, or stream s of a batch: the window's slices are cut into tiles stream after stream,
+// each stream with its own partitions and run bounds; everything else is the single-sketch path.
+struct PartView {
+    FastMod fm;
+    uint32_t seed, low_base, shift, parts;
+    uint32_t tile0, tiles;  // its tiles in the chunk
+    uint16_t* off;          // [parts + 1][tiles of `stride`]
+    uint32_t stride;
+};
+template <bool BATCH>
+__device__ __forceinline__ PartView part_view(const MswsDev& D, const PartDev& Q, const BatchDev& B, uint32_t s) {
+    PartView V;
+    if (!BATCH) {
+        V.fm = D.fm_low, V.seed = D.seed, V.low_base = 0, V.shift = Q.shift, V.parts = Q.parts;
+        V.tile0 = 0, V.tiles = Q.tiles, V.off = Q.off, V.stride = Q.stride;
+        return V;
+    }
+    const StreamDesc* sd = B.desc + s;
+    V.fm = FastMod{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d)};
+    V.seed = __ldg(&sd->seed), V.low_base = __ldg(&sd->low_base);
+    V.shift = __ldg(&sd->shift), V.parts = __ldg(&sd->parts);
+    V.tile0 = __ldcg(B.item_off + s), V.tiles = __ldcg(B.item_off + s + 1) - V.tile0;
+    V.off = Q.off + __ldcg(B.run_off + s), V.stride = V.tiles;
+    return V;
+}
+
+// One block: the slices of the window's streams (offsets checked by the host), their tiles of
+// `tile` keys and run bounds, and the allocators as the window begins.
+__global__ void __launch_bounds__(1024) k_part_plan(BatchDev B, BatchWindow W, uint32_t tile, Ctl* ctl) {
+    const uint32_t S = B.n_streams;
+    for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
+        const uint64_t o0 = __ldcg(B.key_off + s), len = __ldcg(B.key_off + s + 1) - o0;
+        const bool in = s >= W.s_lo && s < W.s_hi && in_window(B, W, s, len);
+        const uint64_t lo = in ? o0 + umin64(W.rel_lo, len) : o0, hi = in ? o0 + umin64(W.rel_hi, len) : o0;
+        const uint32_t t = (uint32_t)((hi - lo + tile - 1) / tile);
+        B.lo[s] = lo;
+        B.hi[s] = hi;
+        B.item_off[s] = t;
+        B.run_off[s] = t * (B.desc[s].parts + 1u);
+        B.base_id[s] = __ldcg(B.next_id + s);
+    }
+    __syncthreads();
+    const uint32_t tiles = block_scan_array(B.item_off, S), runs = block_scan_array(B.run_off, S);
+    if (threadIdx.x == 0) {
+        B.item_off[S] = tiles;
+        B.run_off[S] = runs;
+        ctl->n_switch = 0;
+    }
+}
+
+__device__ __forceinline__ uint32_t batch_hot_set(uint32_t key) { return (key * 0x9E3779B1u) >> 26; }
+static_assert(BATCH_HOT == 2 * 64, "batch_hot_set yields 6 bits, two keys per set");
+
+// A block per stream of the window: keys seen at least four times in 4096 samples of its slice
+// (short slices: none), the heaviest first, as k_part_hot.
+__global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restrict__ keys, BatchDev B, uint32_t s_lo) {
+    constexpr uint32_t N = 4096, SLOTS = 4096;
+    __shared__ uint32_t s_key[SLOTS], s_cnt[SLOTS], s_hot[BATCH_HOT];
+    const uint32_t tid = threadIdx.x, s = s_lo + blockIdx.x;
+    const uint64_t lo = __ldcg(B.lo + s), len = __ldcg(B.hi + s) - lo;
+    if (len == 0) return;
+    for (uint32_t i = tid; i < BATCH_HOT; i += 256) s_hot[i] = HOT_EMPTY;
+    if (len >= 8 * N) {
+        for (uint32_t i = tid; i < SLOTS; i += 256) s_key[i] = HOT_EMPTY, s_cnt[i] = 0u;
+        const uint64_t step = len / N;
+        uint32_t k[N / 256];
+#pragma unroll
+        for (uint32_t j = 0; j < N / 256; ++j) k[j] = __ldg(keys + lo + step * (uint64_t)(j * 256 + tid));
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < N / 256; ++j) {
+            if (k[j] == HOT_EMPTY) continue;
+            const uint32_t h = mix32(k[j]);
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t i = (h + q) & (SLOTS - 1);
+                uint32_t seen = reinterpret_cast<volatile uint32_t*>(s_key)[i];
+                if (seen == HOT_EMPTY) seen = atomicCAS(s_key + i, HOT_EMPTY, k[j]);
+                if (seen == HOT_EMPTY || seen == k[j]) {
+                    atomicAdd(s_cnt + i, 1u);
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        uint32_t hi = 0xffffffffu;
+        for (uint32_t least : {64u, 16u, 4u}) {
+            for (uint32_t i = tid; i < SLOTS; i += 256) {
+                if (s_cnt[i] < least || s_cnt[i] >= hi) continue;
+                const uint32_t h = 2 * batch_hot_set(s_key[i]);
+                if (atomicCAS(s_hot + h, HOT_EMPTY, s_key[i]) != HOT_EMPTY) atomicCAS(s_hot + h + 1, HOT_EMPTY, s_key[i]);
+            }
+            hi = least;
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < BATCH_HOT; i += 256) B.hot[(uint64_t)s * BATCH_HOT + i] = s_hot[i];
+}
+
 // ---- 1: tiles ordered by partition ---------------------------------------------------------
 
 // HOT: keys of the call's hot table whose bucket is linked when the chunk begins are counted in
 // shared memory (high-level additions commute) and never become entries.
-template <int PT_THREADS, int KPT, bool HOT>
+template <int PT_THREADS, int KPT, bool HOT, bool BATCH>
 __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(const uint32_t* __restrict__ keys, uint64_t n, MswsDev D,
-                                                              PartDev Q) {
-    constexpr uint32_t R = PT_THREADS * KPT;
+                                                              PartDev Q, BatchDev B) {
+    constexpr uint32_t R = PT_THREADS * KPT, HOTS = BATCH ? BATCH_HOT : PART_HOT;
     extern __shared__ __align__(16) uint32_t sm[];
     uint32_t* s_ent = sm;                                          // [R]
     uint16_t* s_idx = reinterpret_cast<uint16_t*>(sm + R);         // [R]
-    uint32_t* s_hkey = sm + R + R / 2;                             // HOT: [PART_HOT] keys, counts, high ids
-    uint32_t* s_hcnt = s_hkey + PART_HOT;
-    uint32_t* s_hid = s_hcnt + PART_HOT;
-    uint32_t* s_hist = HOT ? s_hid + PART_HOT : s_hkey;            // [parts] counts, then first positions
+    uint32_t* s_hkey = sm + R + R / 2;                             // HOT: [HOTS] keys, counts, high ids
+    uint32_t* s_hcnt = s_hkey + HOTS;
+    uint32_t* s_hid = s_hcnt + HOTS;
+    uint32_t* s_hist = HOT ? s_hid + HOTS : s_hkey;                // [parts] counts, then first positions
     const int tid = threadIdx.x;
-    const uint32_t parts = Q.parts, per = (parts + PT_THREADS - 1) / PT_THREADS;
-    const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
-    if (blockIdx.x == 0 && tid == 0) {
+    if (!BATCH && blockIdx.x == 0 && tid == 0) {
         D.ctl->n_switch = 0;
         D.ctl->link_base = D.ctl->next_id;
     }
-    if (HOT) {
-        for (uint32_t i = tid; i < PART_HOT; i += PT_THREADS) {
-            uint32_t key = __ldcg(Q.hot + i), id = 0;
+    uint32_t stream = 0;
+    PartView V = part_view<false>(D, Q, B, 0);
+    auto load_hot = [&] {  // the hot keys whose buckets are linked
+        const uint32_t* hot = BATCH ? B.hot + (uint64_t)stream * BATCH_HOT : Q.hot;
+        for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
+            uint32_t key = __ldcg(hot + i), id = 0;
             if (key != HOT_EMPTY) {
-                id = __ldcg(D.low + (uint64_t)fast_mod(D.fm_low, key * D.seed) * LOW_WORDS + 7);
+                id = __ldcg(D.low + (uint64_t)(V.low_base + fast_mod(V.fm, key * V.seed)) * LOW_WORDS + 7);
                 if (!is_linked(D, id)) key = HOT_EMPTY;
             }
             s_hkey[i] = key;
             s_hcnt[i] = 0u;
             s_hid[i] = id;
         }
-    }
+    };
+    auto flush_hot = [&] {  // their counts: one add per counter
+        for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
+            const uint32_t c = s_hcnt[i];
+            if (!c) continue;
+            uint32_t* hb = D.high + (uint64_t)(s_hid[i] - START) * HIGH_WORDS;
+            for (uint32_t m = __ldg(D.masks + fast_mod(D.fm_mask, s_hkey[i] * V.seed)); m; m &= m - 1)
+                atomicAdd(hb + (__ffs(m) - 1), c);
+        }
+    };
+    if (HOT && !BATCH) load_hot();
+    if (BATCH) stream = NONE;
     for (uint32_t t = blockIdx.x; t < Q.tiles; t += gridDim.x) {
-        const uint64_t k0 = (uint64_t)t * R;
-        const uint32_t cnt = (uint32_t)umin64(R, n - k0);
+        if (BATCH) {
+            const uint32_t s = stream_of_item_warp(B, t);
+            if (s != stream) {  // uniform over the block
+                if (HOT && stream != NONE) {
+                    flush_hot();
+                    __syncthreads();
+                }
+                stream = s;
+                V = part_view<true>(D, Q, B, s);
+                if (HOT) load_hot();
+            }
+        }
+        const uint32_t parts = V.parts, per = (parts + PT_THREADS - 1) / PT_THREADS, lt = t - V.tile0;
+        const uint64_t p0 = (uint64_t)t * R;                                             // its place and positions
+        const uint64_t k0 = BATCH ? __ldcg(B.lo + stream) + (uint64_t)lt * R : p0;       // its first key
+        const uint32_t cnt = (uint32_t)umin64(R, (BATCH ? __ldcg(B.hi + stream) : n) - k0);
+        const bool vec = (reinterpret_cast<uintptr_t>(keys + k0) & 15u) == 0;
         for (uint32_t i = tid; i < parts; i += PT_THREADS) s_hist[i] = 0u;
         // the link order's switch bits and counts of this tile's positions
-        for (uint32_t i = tid; i < R / 32; i += PT_THREADS) __stcg(D.sw_bits + (k0 >> 5) + i, 0u);
+        for (uint32_t i = tid; i < R / 32; i += PT_THREADS) __stcg(D.sw_bits + (p0 >> 5) + i, 0u);
         if (R >= SW_BLOCK) {
-            if (tid < (int)(R / SW_BLOCK)) __stcg(D.sw_cnt + k0 / SW_BLOCK + tid, 0u);
-        } else if (tid == 0 && (k0 % SW_BLOCK) == 0) {
-            __stcg(D.sw_cnt + k0 / SW_BLOCK, 0u);
+            if (tid < (int)(R / SW_BLOCK)) __stcg(D.sw_cnt + p0 / SW_BLOCK + tid, 0u);
+        } else if (tid == 0 && (p0 % SW_BLOCK) == 0) {
+            __stcg(D.sw_cnt + p0 / SW_BLOCK, 0u);
         }
         uint32_t e[KPT], pr[KPT];  // the key, then its entry; partition << 16 | rank
         // thread's keys: vector v of 4 at tile index v * 4 * PT_THREADS + 4 * tid
@@ -172,18 +300,18 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
         for (int j = 0; j < KPT; ++j) {
             const uint32_t i = (j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3);
             bool live = i < cnt;
-            if (D.skip && live) live = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
+            if (!BATCH && D.skip && live) live = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
             if (HOT && live) {
-                const uint32_t s = 2 * hot_set(e[j]);
+                const uint32_t s = 2 * (BATCH ? batch_hot_set(e[j]) : hot_set(e[j]));
                 const uint2 hk = *reinterpret_cast<const uint2*>(s_hkey + s);
                 if (e[j] != HOT_EMPTY && (hk.x == e[j] || hk.y == e[j])) {
                     atomicAdd(s_hcnt + s + (hk.x != e[j]), 1u);
                     live = false;
                 }
             }
-            const uint32_t hv = e[j] * D.seed;
-            const uint32_t b = fast_mod(D.fm_low, hv), p = b >> Q.shift;
-            e[j] = ((b & ((1u << Q.shift) - 1u)) << ENT_MASK_BITS) | fast_mod(D.fm_mask, hv);
+            const uint32_t hv = e[j] * V.seed;
+            const uint32_t b = fast_mod(V.fm, hv), p = b >> V.shift;
+            e[j] = ((b & ((1u << V.shift) - 1u)) << ENT_MASK_BITS) | fast_mod(D.fm_mask, hv);
             pr[j] = live ? (p << 16) | atomicAdd(s_hist + p, 1u) : NONE;
         }
         __syncthreads();
@@ -202,11 +330,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
                 const uint32_t p = tid * per + j;
                 if (j < per && p < parts) {
                     s_hist[p] = run;
-                    Q.off[(uint64_t)p * Q.stride + t] = (uint16_t)run;
+                    V.off[(uint64_t)p * V.stride + lt] = (uint16_t)run;
                     run += c[j];
                 }
             }
-            if (tid == 0) Q.off[(uint64_t)parts * Q.stride + t] = (uint16_t)total;
+            if (tid == 0) V.off[(uint64_t)parts * V.stride + lt] = (uint16_t)total;
             __syncthreads();
 #pragma unroll
             for (int j = 0; j < KPT; ++j) {
@@ -216,22 +344,14 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
                 s_idx[pos] = (uint16_t)((j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3));
             }
             __syncthreads();
-            uint4* ge = reinterpret_cast<uint4*>(Q.ent + k0);
-            uint4* gi = reinterpret_cast<uint4*>(Q.idx + k0);
+            uint4* ge = reinterpret_cast<uint4*>(Q.ent + p0);
+            uint4* gi = reinterpret_cast<uint4*>(Q.idx + p0);
             for (uint32_t i = tid; i * 4 < total; i += PT_THREADS) __stcg(ge + i, reinterpret_cast<const uint4*>(s_ent)[i]);
             for (uint32_t i = tid; i * 8 < total; i += PT_THREADS) __stcg(gi + i, reinterpret_cast<const uint4*>(s_idx)[i]);
         }
         __syncthreads();
     }
-    if (HOT) {  // the counts of the hot keys: one add per counter and block
-        for (uint32_t i = tid; i < PART_HOT; i += PT_THREADS) {
-            const uint32_t c = s_hcnt[i];
-            if (!c) continue;
-            uint32_t* hb = D.high + (uint64_t)(s_hid[i] - START) * HIGH_WORDS;
-            for (uint32_t m = __ldg(D.masks + fast_mod(D.fm_mask, s_hkey[i] * D.seed)); m; m &= m - 1)
-                atomicAdd(hb + (__ffs(m) - 1), c);
-        }
-    }
+    if (HOT && (!BATCH || stream != NONE)) flush_hot();
 }
 
 // ---- 2: one partition per block ------------------------------------------------------------
@@ -524,22 +644,35 @@ __device__ __forceinline__ bool replay_few(const MswsDev& D, const ApShared& S, 
     return true;
 }
 
-template <bool WIDE>
-__global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev Q) {
+template <bool WIDE, bool BATCH>
+__global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev Q, BatchDev B) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const ApShared S = ap_carve(smem, Q.shift, D.n_masks);
+    uint32_t p = blockIdx.x, stream = 0;
+    if (BATCH) {  // block: partition `part0 + blockIdx.x` of all streams'
+        p += Q.part0;
+        uint32_t lo = 0, hi = B.n_streams;  // part_off[lo] <= p < part_off[hi]
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (__ldg(B.part_off + mid) <= p) lo = mid;
+            else hi = mid;
+        }
+        stream = lo;
+        p -= __ldg(B.part_off + lo);
+    }
+    const PartView V = part_view<BATCH>(D, Q, B, stream);
+    if (V.tiles == 0) return;
+    const ApShared S = ap_carve(smem, V.shift, D.n_masks);
     __shared__ uint32_t s_nflag, s_nrec, s_many, s_drop, s_rb, s_rk, s_nacc, s_new, s_row;
     __shared__ uint32_t s_cnt[LOW_COUNTERS + 2];  // bisection: counts per counter, keys, mask
     __shared__ uint32_t s_pre[LOW_COUNTERS];
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const uint32_t p = blockIdx.x;
     for (uint32_t i = tid; i < D.n_masks; i += AP_THREADS) S.mk[i] = mask_code<WIDE>(__ldg(D.masks + i));  // the host's
-    const uint32_t accs = ap_accs(Q.shift);
+    const uint32_t accs = ap_accs(V.shift);
     for (uint32_t i = tid; i < accs * ACC_WORDS; i += AP_THREADS) S.acc[i] = 0u;
     if (tid == 0) s_nflag = s_nrec = s_many = s_drop = s_rb = s_rk = s_nacc = s_new = 0;
     __syncthreads();
-    const uint64_t b0 = (uint64_t)p << Q.shift;
-    const uint32_t nb = (uint32_t)umin64((uint64_t)1 << Q.shift, D.n_low - b0);
+    const uint64_t b0 = V.low_base + ((uint64_t)p << V.shift);
+    const uint32_t nb = (uint32_t)umin64((uint64_t)1 << V.shift, V.fm.d - ((uint64_t)p << V.shift));
     uint4* gt = reinterpret_cast<uint4*>(D.low + b0 * LOW_WORDS);
     {
         uint4* st = reinterpret_cast<uint4*>(S.tab);
@@ -569,26 +702,26 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             }
         }
     }
-    const uint16_t* o0 = Q.off + (uint64_t)p * Q.stride;
-    const uint16_t* o1 = o0 + Q.stride;
-    const uint32_t tile = Q.tile, cap = ap_unit(Q.shift);
+    const uint16_t* o0 = V.off + (uint64_t)p * V.stride;
+    const uint16_t* o1 = o0 + V.stride;
+    const uint32_t tile = Q.tile, cap = ap_unit(V.shift), mean = max(1u, tile / V.parts);
     constexpr int U = 4096 / AP_THREADS;  // a thread's entries of a unit, at most
     uint32_t units = 0;
-    for (uint32_t ts = 0; ts < Q.tiles; ts += AP_TILES) {
+    for (uint32_t ts = 0; ts < V.tiles; ts += AP_TILES) {
         // the run bounds of the next AP_TILES tiles
         __syncthreads();
-        const uint32_t nr = min(AP_TILES, Q.tiles - ts);
+        const uint32_t nr = min(AP_TILES, V.tiles - ts), tile_s = V.tile0 + ts;
         uint32_t a = 0, len = 0, total;
         if (tid < nr) {
             a = __ldcg(o0 + ts + tid);
             len = __ldcg(o1 + ts + tid) - a;
         }
         const uint32_t before = block_exclusive_scan(len, &total);
-        S.dlt[tid] = (ts + tid) * tile + a - before;
+        S.dlt[tid] = (tile_s + tid) * tile + a - before;
         S.before[tid] = before;
         if (tid == 0) S.before[nr] = total;  // (entry nr < AP_TILES already holds it)
         // far above an even share, a heavy key is likely, maybe of a bucket that is not linked yet
-        const bool heavy = total > 4u * Q.mean * nr;
+        const bool heavy = total > 4u * mean * nr;
         for (uint32_t r0 = 0; r0 < nr;) {
             __syncthreads();
             const uint32_t base = S.before[r0];
@@ -631,7 +764,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             auto record = [&](uint32_t x, uint32_t r, uint32_t at) {
                 const uint32_t w7 = S.w7[x >> ENT_MASK_BITS];
                 if (!(w7 & FLAG)) return;
-                const uint32_t k = atomicAdd(&s_nrec, 1u), pos = (ts + r) * tile + __ldcg(Q.idx + at);
+                const uint32_t k = atomicAdd(&s_nrec, 1u), pos = (tile_s + r) * tile + __ldcg(Q.idx + at);
                 if (k < cap)
                     S.recs[k] = (unsigned long long)(w7 & ~FLAG) << 46 | (unsigned long long)pos << ENT_MASK_BITS |
                                 (x & ENT_MASK);
@@ -717,7 +850,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
                 // yet): per flagged bucket, bisect the array position of the switching key, the
                 // first position x such that some counter has 130 - P occurrences up to x (the key
                 // that sees 129 = P + its earlier occurrences).
-                const uint32_t plo = (ts + rb) * tile, phi = plo + tile - 1;
+                const uint32_t plo = (tile_s + rb) * tile, phi = plo + tile - 1;
                 for (uint32_t s = 0; s < F; ++s) {
                     const uint32_t lb = S.tab[s * LOW_WORDS + 7];
                     uint32_t* bw = S.tab + lb * LOW_WORDS;
@@ -824,14 +957,15 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
 
 // ---- 3: high ids in the array order of the switching keys -----------------------------------
 
-__global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev Q) {
+template <bool BATCH>
+__global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev Q, BatchDev B) {
     extern __shared__ __align__(16) uint32_t spre[];  // switches per SW_BLOCK positions, then their prefix
     Ctl* ctl = D.ctl;
     const uint32_t ns = __ldcg(&ctl->n_switch);
     if (ns == 0) return;
     const uint32_t base = __ldcg(&ctl->link_base);
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (blockIdx.x == 0 && tid == 0)  // the allocator stops at the pool's end, as the oracle's
+    if (!BATCH && blockIdx.x == 0 && tid == 0)  // the allocator stops at the pool's end, as the oracle's
         ctl->next_id = (uint32_t)min((unsigned long long)base + ns, (unsigned long long)START + D.n_high);
     if (blockIdx.x * AP_WARPS >= ns) return;
     const uint32_t nq = (uint32_t)(((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK);
@@ -841,18 +975,32 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev 
     for (uint32_t r = blockIdx.x * AP_WARPS + wid; r < ns; r += gridDim.x * AP_WARPS) {
         const uint32_t b = __ldcg(D.flag_list + r);
         const uint2 w = __ldcg(D.sw + r);
-        const uint32_t id = base + switch_rank(D, spre, w.x);
-        const bool ok = (uint64_t)(id - START) < D.n_high;
+        uint32_t id = base + switch_rank(D, spre, w.x), st = 0;
+        bool ok = (uint64_t)(id - START) < D.n_high;
+        if (BATCH) {  // ranked within the stream (its positions are contiguous) on its own allocator
+            if (lane == 0) st = stream_of_bucket(B, b);
+            st = __shfl_sync(0xffffffffu, st, 0);
+            const uint32_t own = __ldcg(B.base_id + st) + (id - base) -
+                                 switch_rank(D, spre, __ldcg(B.item_off + st) * Q.tile);
+            const uint32_t nh = __ldg(&B.desc[st].n_high);
+            ok = (uint64_t)(own - START) < nh;
+            id = own + __ldg(&B.desc[st].high_base);
+            if (lane == 0) {
+                atomicMax(B.next_id + st, (uint32_t)min((unsigned long long)own + 1ull, (unsigned long long)START + nh));
+                if (!ok) atomicOr(B.status + st, ST_POOL_FULL);
+            }
+        }
         uint32_t H = 0, n_after = w.y;
         if (r < D.long_cap) {
             if (lane < LOW_COUNTERS) H = __ldcg(D.totals + (uint64_t)r * LOW_COUNTERS + lane);
         } else {
             // no row was left: count the bucket's entries from the switch on again
-            const uint32_t part = b >> Q.shift, lb = b & ((1u << Q.shift) - 1u);
-            const uint16_t* o0 = Q.off + (uint64_t)part * Q.stride;
+            const PartView V = part_view<BATCH>(D, Q, B, st);
+            const uint32_t part = (b - V.low_base) >> V.shift, lb = (b - V.low_base) & ((1u << V.shift) - 1u);
+            const uint16_t* o0 = V.off + (uint64_t)part * V.stride - V.tile0;
             uint32_t keys = 0;
-            for (uint32_t t = w.x / Q.tile; t < Q.tiles; ++t) {
-                const uint32_t e1 = t * Q.tile + __ldcg(o0 + Q.stride + t);
+            for (uint32_t t = w.x / Q.tile; t < V.tile0 + V.tiles; ++t) {
+                const uint32_t e1 = t * Q.tile + __ldcg(o0 + V.stride + t);
                 for (uint32_t i0 = t * Q.tile + __ldcg(o0 + t); i0 < e1; i0 += 32) {
                     const uint32_t i = i0 + lane;
                     uint32_t m = 0;
@@ -888,26 +1036,44 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev 
 
 // ---- launchers ------------------------------------------------------------------------------
 
-static size_t split_smem(uint32_t tile, uint32_t parts, bool hot) {
-    return (size_t)tile * 6 + parts * 4 + (hot ? PART_HOT * 12 : 0);
+static size_t split_smem(uint32_t tile, uint32_t parts, uint32_t hot) {
+    return (size_t)tile * 6 + parts * 4 + hot * 12;
 }
 
-cudaError_t part_configure(PartLaunch* L, uint32_t shift, uint32_t parts, uint32_t n_masks, int num_sms) {
-    cudaError_t e = cudaSuccess;
+static const void* split_fn(bool small, bool hot, bool batch) {
+    if (batch)
+        return small ? (hot ? (const void*)k_part_split<512, 4, true, true> : (const void*)k_part_split<512, 4, false, true>)
+                     : (hot ? (const void*)k_part_split<1024, 16, true, true>
+                            : (const void*)k_part_split<1024, 16, false, true>);
+    return small ? (hot ? (const void*)k_part_split<512, 4, true, false> : (const void*)k_part_split<512, 4, false, false>)
+                 : (hot ? (const void*)k_part_split<1024, 16, true, false>
+                        : (const void*)k_part_split<1024, 16, false, false>);
+}
+
+static const void* apply_fn(bool wide, bool batch) {
+    return batch ? (wide ? (const void*)k_part_apply<true, true> : (const void*)k_part_apply<false, true>)
+                 : (wide ? (const void*)k_part_apply<true, false> : (const void*)k_part_apply<false, false>);
+}
+
+size_t part_apply_smem(uint32_t shift, uint32_t n_masks) { return apply_smem(shift, n_masks); }
+
+cudaError_t part_configure(int num_sms, PartLaunch* L) {
     // the dynamic shared-memory cap is a per-kernel attribute shared by every sketch of the
     // process: the largest any of them may ask for; a launch passes its own size
-    const size_t split_max = split_smem(PART_TILE, PART_MAX_PARTS, true);
+    const size_t split_max = split_smem(PART_TILE, PART_MAX_PARTS, PART_HOT);
     const size_t apply_max = std::max(apply_smem(PART_MAX_SHIFT, PART_MAX_MASKS), apply_smem(PART_MAX_SHIFT - 1, PART_MAX_MASKS));
     const size_t link_max = PART_MAX_CHUNK / SW_BLOCK * 4;
-    const void* fns[] = {(const void*)k_part_split<1024, 16, false>, (const void*)k_part_split<512, 4, false>,
-                         (const void*)k_part_split<1024, 16, true>,  (const void*)k_part_split<512, 4, true>,
-                         (const void*)k_part_apply<false>,     (const void*)k_part_apply<true>,
-                         (const void*)k_part_link};
-    const size_t most[] = {split_max, split_max, split_max, split_max, apply_max, apply_max, link_max};
-    for (int i = 0; i < 7 && e == cudaSuccess; ++i)
-        e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most[i]);
+    cudaError_t e = cudaSuccess;
+    auto cap = [&](const void* fn, size_t bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    for (int batch = 0; batch < 2; ++batch) {
+        for (int i = 0; i < 4; ++i) cap(split_fn(i & 1, i & 2, batch != 0), split_max);
+        for (int wide = 0; wide < 2; ++wide) cap(apply_fn(wide != 0, batch != 0), apply_max);
+    }
+    cap((const void*)k_part_link<false>, link_max);
+    cap((const void*)k_part_link<true>, link_max);
     L->num_sms = num_sms;
-    L->apply_smem = apply_smem(shift, n_masks);
     return e;
 }
 
@@ -917,31 +1083,52 @@ cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cu
     return cudaLaunchKernel((const void*)k_part_hot, dim3(HOT_BLOCKS), dim3(HOT_THREADS), args, 0, st);
 }
 
+// Split, apply and link of a chunk (or a batch's window) whose tiles Q names.
+static cudaError_t part_steps(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& Q, const BatchDev& B,
+                              const PartLaunch& L, bool small, bool hot, uint32_t blocks, cudaStream_t st) {
+    MswsDev Dc = D;
+    PartDev Qc = Q;
+    BatchDev Bc = B;
+    const bool batch = B.n_streams != 0;
+    {
+        void* args[] = {(void*)&d_keys, (void*)&n, (void*)&Dc, (void*)&Qc, (void*)&Bc};
+        const int grid = (int)std::min<uint64_t>(Q.tiles, (uint64_t)(small ? 2 * L.num_sms : L.num_sms));
+        const cudaError_t e = cudaLaunchKernel(split_fn(small, hot, batch), dim3(grid), dim3(small ? 512 : 1024), args,
+                                               split_smem(Q.tile, Q.parts, hot ? (batch ? BATCH_HOT : PART_HOT) : 0), st);
+        if (e != cudaSuccess) return e;
+    }
+    void* args[] = {(void*)&Dc, (void*)&Qc, (void*)&Bc};
+    const cudaError_t e = cudaLaunchKernel(apply_fn(D.wide != 0, batch), dim3(blocks), dim3(AP_THREADS), args, L.apply_smem, st);
+    if (e != cudaSuccess) return e;
+    const uint64_t nq = ((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK;
+    return cudaLaunchKernel(batch ? (const void*)k_part_link<true> : (const void*)k_part_link<false>, dim3(L.num_sms),
+                            dim3(AP_THREADS), args, (size_t)nq * 4, st);
+}
+
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
                         bool hot, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     PartDev Q = part;
-    MswsDev Dc = D;
-    // tiles of 2048 keys while 8192-key tiles would leave SMs idle (two blocks on each of 148)
+    // tiles of 2048 keys while larger ones would leave SMs idle
     const bool small = n < PART_SMALL_MAX;
     Q.tile = small ? PART_TILE_SMALL : PART_TILE;
     Q.tiles = (uint32_t)((n + Q.tile - 1) / Q.tile);
-    Q.mean = std::max<uint32_t>(1u, (uint32_t)(Q.tile / Q.parts));
-    {
-        void* args[] = {(void*)&d_keys, (void*)&n, (void*)&Dc, (void*)&Q};
-        const void* fn = hot ? (small ? (const void*)k_part_split<512, 4, true> : (const void*)k_part_split<1024, 16, true>)
-                             : (small ? (const void*)k_part_split<512, 4, false> : (const void*)k_part_split<1024, 16, false>);
-        const int grid = (int)std::min<uint64_t>(Q.tiles, (uint64_t)(small ? 2 * L.num_sms : L.num_sms));
-        const cudaError_t e = cudaLaunchKernel(fn, dim3(grid), dim3(small ? 512 : 1024), args,
-                                               split_smem(Q.tile, Q.parts, hot), st);
-        if (e != cudaSuccess) return e;
-    }
-    void* args[] = {(void*)&Dc, (void*)&Q};
-    const void* fn = D.wide ? (const void*)k_part_apply<true> : (const void*)k_part_apply<false>;
-    cudaError_t e = cudaLaunchKernel(fn, dim3(Q.parts), dim3(AP_THREADS), args, L.apply_smem, st);
+    return part_steps(d_keys, n, D, Q, BatchDev{}, L, small, hot, Q.parts, st);
+}
+
+cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const PartDev& part, const BatchDev& B,
+                              const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t part_lo,
+                              uint32_t part_hi, bool small, bool hot, cudaStream_t st) {
+    if (tiles == 0) return cudaSuccess;
+    PartDev Q = part;
+    Q.tile = small ? PART_TILE_SMALL : PART_TILE;
+    Q.tiles = tiles;
+    Q.part0 = part_lo;
+    k_part_plan<<<1, 1024, 0, st>>>(B, W, Q.tile, D.ctl);
+    if (hot) k_part_hot_batch<<<W.s_hi - W.s_lo, 256, 0, st>>>(d_keys, B, W.s_lo);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const uint64_t nq = ((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK;
-    return cudaLaunchKernel((const void*)k_part_link, dim3(L.num_sms), dim3(AP_THREADS), args, (size_t)nq * 4, st);
+    return part_steps(d_keys, 0, D, Q, B, L, small, hot, part_hi - part_lo, st);
 }
 
 }  // namespace qsb

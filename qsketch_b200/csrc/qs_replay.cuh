@@ -142,4 +142,42 @@ __device__ __forceinline__ uint32_t switch_rank(const MswsDev& D, const uint32_t
     return spre[q] + __reduce_add_sync(0xffffffffu, c);
 }
 
+// ---- batched streams ----------------------------------------------------------------------
+
+__device__ __forceinline__ bool in_window(const BatchDev& B, const BatchWindow& W, uint32_t s, uint64_t len) {
+    if (W.which == STREAMS_ALL) return true;
+    return batch_dense(len, B.desc[s].fm_low.d, B.desc[s].parts) == (W.which == STREAMS_DENSE);
+}
+
+// The stream whose bucket range holds global bucket g (bases strictly increase).
+__device__ __forceinline__ uint32_t stream_of_bucket(const BatchDev& B, uint32_t g) {
+    uint32_t lo = 0, hi = B.n_streams;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(&B.desc[mid].low_base) <= g)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// The stream of work item `it` (< item_off[n_streams]): the last s with item_off[s] <= it.
+// Called by a whole warp: each step probes 32 evenly spaced offsets, so 512 streams take two
+// dependent loads instead of nine.
+__device__ __forceinline__ uint32_t stream_of_item_warp(const BatchDev& B, uint32_t it) {
+    const int lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = B.n_streams;  // item_off[lo] <= it; the answer lies in [lo, hi)
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t idx = lo + lane * step;
+        const bool le = idx < hi && __ldcg(B.item_off + idx) <= it;
+        const uint32_t bal = __ballot_sync(0xffffffffu, le);  // lane 0 always holds
+        const uint32_t last = 31 - __clz(bal);
+        lo += last * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
 }  // namespace qsb
