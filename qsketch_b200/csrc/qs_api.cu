@@ -546,7 +546,7 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         CKB(sk->alloc(&D.seg_beg, cap), "alloc segments");
         CKB(sk->alloc(&D.totals, (uint64_t)D.long_cap * LOW_COUNTERS), "alloc totals");
         CKB(sk->alloc(&D.sw, links), "alloc link order");
-        CKB(sk->alloc(&D.sw_base, cap), "alloc link order");
+        CKB(sk->alloc(&D.sw_base, links), "alloc link order");
         CKB(sk->alloc(&D.sw_bits, (reach + 31) / 32), "alloc link order");
         CKB(sk->alloc(&D.sw_cnt, (reach + SW_BLOCK - 1) / SW_BLOCK), "alloc link order");
         CKB(cudaMemcpy(masks_d, sk->masks.data(), (size_t)H * 4, cudaMemcpyHostToDevice), "upload masks");
@@ -1821,11 +1821,15 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
                              small, hot, st),
            "partitioned batch insert");
         CK(sk->prof_end(0, st), "profile");
-        b->info.launches += hot ? 5 : 4;
+        b->info.launches += 4;
         return QS_OK;
     };
     for (int round = 0; round < 2; ++round) {
         const uint64_t r0 = round ? first : 0, r1 = round ? ~0ull : first;
+        if (round) {
+            CK(part_hot_batch(d_keys, B, first, st), "heavy keys");
+            ++b->info.launches;
+        }
         uint64_t slots = 0, keys = 0, runs = 0;
         uint32_t lo = 0;
         auto close = [&](uint32_t hi) -> qs_status {

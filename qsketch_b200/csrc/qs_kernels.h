@@ -52,7 +52,9 @@ cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cu
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
                         bool hot, cudaStream_t st);
 // The same for a window of a batch: `tiles` tiles (small or large) of the streams W names, whose
-// partitions are [part_lo, part_hi) of all streams'; hot: each stream's heavy keys are sampled.
+// partitions are [part_lo, part_hi) of all streams'; hot: the heavy keys that part_hot_batch left
+// for each stream (from its keys at `first` on) are counted in the split.
+cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, cudaStream_t st);
 cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const PartDev& part, const BatchDev& B,
                               const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t part_lo,
                               uint32_t part_hi, bool small, bool hot, cudaStream_t st);

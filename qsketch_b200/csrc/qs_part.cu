@@ -162,14 +162,15 @@ __global__ void __launch_bounds__(1024) k_part_plan(BatchDev B, BatchWindow W, u
 __device__ __forceinline__ uint32_t batch_hot_set(uint32_t key) { return (key * 0x9E3779B1u) >> 26; }
 static_assert(BATCH_HOT == 2 * 64, "batch_hot_set yields 6 bits, two keys per set");
 
-// A block per stream of the window: keys seen at least four times in 4096 samples of its slice
-// (short slices: none), the heaviest first, as k_part_hot.
-__global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restrict__ keys, BatchDev B, uint32_t s_lo) {
+// A block per dense stream: keys seen at least four times in 4096 samples of its keys from `first` on
+// (short streams: none), the heaviest first, as k_part_hot.
+__global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restrict__ keys, BatchDev B, uint64_t first) {
     constexpr uint32_t N = 4096, SLOTS = 4096;
     __shared__ uint32_t s_key[SLOTS], s_cnt[SLOTS], s_hot[BATCH_HOT];
-    const uint32_t tid = threadIdx.x, s = s_lo + blockIdx.x;
-    const uint64_t lo = __ldcg(B.lo + s), len = __ldcg(B.hi + s) - lo;
-    if (len == 0) return;
+    const uint32_t tid = threadIdx.x, s = blockIdx.x;
+    const uint64_t o0 = __ldcg(B.key_off + s), all = __ldcg(B.key_off + s + 1) - o0;
+    if (!batch_dense(all, B.desc[s].fm_low.d, B.desc[s].parts) || all <= first) return;
+    const uint64_t lo = o0 + first, len = all - first;
     for (uint32_t i = tid; i < BATCH_HOT; i += 256) s_hot[i] = HOT_EMPTY;
     if (len >= 8 * N) {
         for (uint32_t i = tid; i < SLOTS; i += 256) s_key[i] = HOT_EMPTY, s_cnt[i] = 0u;
@@ -367,6 +368,7 @@ struct ApShared {
     uint32_t* before;          // [AP_TILES + 1] entries of the staged runs before run r
     uint32_t* dlt;             // [AP_TILES] run r: its first entry minus before[r]
     uint16_t* map;             // [ap_unit] the run of each entry of the unit
+    uint32_t stream;           // batch: whose partition this is
 };
 
 __host__ __device__ inline size_t apply_smem(uint32_t shift, uint32_t n_masks) {
@@ -503,12 +505,13 @@ __device__ __forceinline__ void part_apply_batch(const MswsDev& D, const ApShare
 // A bucket that switched at array position pos, with n_after keys from there on: its increments
 // collect in an accumulator (or a row) until the link order is known.  Called by a whole warp,
 // lane c with counter c's high increment H.
-__device__ __forceinline__ void put_row(const MswsDev& D, uint32_t r, uint32_t bucket, uint32_t pos, uint32_t n_after,
-                                        uint32_t H) {
+__device__ __forceinline__ void put_row(const MswsDev& D, uint32_t r, uint32_t stream, uint32_t bucket, uint32_t pos,
+                                        uint32_t n_after, uint32_t H) {
     const int lane = threadIdx.x & 31;
     if (r < D.long_cap && lane < LOW_COUNTERS) __stcg(D.totals + (uint64_t)r * LOW_COUNTERS + lane, H);
     if (lane == 0) {
-        __stcg(D.flag_list + r, bucket);  // flag_cap covers every bucket a chunk can link
+        __stcg(D.flag_list + r, bucket);  // sized, as sw and sw_base, for every bucket a chunk can link
+        __stcg(D.sw_base + r, stream);    // (batch)
         __stcg(D.sw + r, make_uint2(pos, n_after));
         atomicOr(D.sw_bits + (pos >> 5), 1u << (pos & 31));
         atomicAdd(D.sw_cnt + pos / SW_BLOCK, 1u);
@@ -533,7 +536,7 @@ __device__ __forceinline__ void open_row(const MswsDev& D, const ApShared& S, ui
     uint32_t r = 0;
     if (lane == 0) r = atomicAdd(&D.ctl->n_switch, 1u);
     r = __shfl_sync(0xffffffffu, r, 0);
-    put_row(D, r, b0 + lb, pos, n_after, H);
+    put_row(D, r, S.stream, b0 + lb, pos, n_after, H);
     if (lane == 0) S.w7[lb] = r < D.long_cap ? (TEMP | r) : TEMP_NOROW;
 }
 
@@ -578,61 +581,155 @@ __device__ __forceinline__ void block_sort(unsigned long long* recs, uint32_t K)
         }
 }
 
-// Flagged bucket `s`, if it has at most 32 records among recs[0, K) (else false), replayed by one warp (buf: 32
-// words of its own; the run map's memory, which is done with by then): lane i takes
-// the i-th record in array order; counter c's occurrences are one ballot (kept by lane c), so a
-// record sees P + the bits before its lane in each counter it selects.
+// Flagged bucket `s` replayed by one warp from recs[0, K), which hold the unit's records in the order
+// of their entries: tile after tile, but in any order within a tile.  Counts over whole tiles do not
+// need the order, so the warp adds the bucket's records up, 32 at a time, to the record with which
+// some counter passes the threshold; the switching key is in that record's tile, and only that
+// tile's records (all of them, if there are at most 32) are put in order.  False, with nothing
+// changed, if there are more than 32.  buf: 32 words of the warp (the run map's memory, which is
+// done with by then); cnt: 32 counts of the warp.
 static_assert(ap_unit(11) * 2 >= AP_WARPS * 32 * 8, "the run map holds every warp's 32 records");
 template <bool WIDE>
-__device__ __forceinline__ bool replay_few(const MswsDev& D, const ApShared& S, unsigned long long* buf, uint32_t accs,
-                                           uint32_t* s_nacc, uint32_t s, uint32_t K, uint32_t b0, uint32_t* s_rb,
-                                           uint32_t* s_rk) {
-    const int lane = threadIdx.x & 31;
-    uint32_t n = 0;
-    for (uint32_t k0 = 0; k0 < K; k0 += 32) {
-        const unsigned long long r = k0 + lane < K ? S.recs[k0 + lane] : ~0ull;
-        const bool mine = (uint32_t)(r >> 46) == s;
-        const uint32_t bal = __ballot_sync(0xffffffffu, mine);
-        n += __popc(bal);
-        if (n > 32) return false;
-        if (mine) buf[n - __popc(bal) + __popc(bal & lanemask_lt())] = r;
-    }
-    __syncwarp();
-    unsigned long long r = lane < (int)n ? buf[lane] : ~0ull;
-    uint32_t rank = 0;
-    for (uint32_t k = 0; k < n; ++k) rank += buf[k] < r;
-    __syncwarp();
-    if (lane < (int)n) buf[rank] = r;  // positions are distinct
-    __syncwarp();
-    r = buf[lane];
-    const uint32_t m = lane < (int)n ? code_mask<WIDE>(S.mk[(uint32_t)r & ENT_MASK]) : 0u;
-    uint32_t occ = 0;  // lane c: the records that select counter c
+__device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, const ApShared& S,
+                                            unsigned long long* buf, uint32_t* cnt, uint32_t accs, uint32_t* s_nacc,
+                                            uint32_t s, uint32_t K, uint32_t b0, uint32_t* s_rb, uint32_t* s_rk) {
+    const uint32_t lane = threadIdx.x & 31, in_tile = Q.tile - 1u;
+    auto record = [&](uint32_t k, bool& mine) {
+        const unsigned long long r = k < K ? S.recs[k] : ~0ull;
+        mine = (uint32_t)(r >> 46) == s;
+        return r;
+    };
+    auto tile_of = [&](unsigned long long r) { return (uint32_t)(r >> ENT_MASK_BITS) & ~in_tile; };
+    // adds a record's counters to cnt; lane c then reads counter c
+    auto add = [&](unsigned long long r) {
+        const uint32_t q = S.mk[(uint32_t)r & ENT_MASK];
+        if (WIDE) {
+            for (uint32_t mm = q; mm; mm &= mm - 1) atomicAdd(cnt + (__ffs(mm) - 1), 1u);
+        } else {
+            atomicAdd(cnt + (q & 31u), 1u);
+            atomicAdd(cnt + ((q >> 5) & 31u), 1u);
+            atomicAdd(cnt + (q >> 10), 1u);
+        }
+    };
+    auto start = [&](uint32_t v) {
+        __syncwarp();
+        cnt[lane] = v;
+        __syncwarp();
+    };
+    auto counted = [&] {
+        __syncwarp();
+        return reinterpret_cast<volatile uint32_t*>(cnt)[lane];
+    };
+    // lane c: the records of a group (bit i: lane i's, mask mm) that select counter c
+    auto selecting = [&](uint32_t mm) {
+        uint32_t occ = 0;
 #pragma unroll
-    for (int c = 0; c < LOW_COUNTERS; ++c) {
-        const uint32_t bal = __ballot_sync(0xffffffffu, (m >> c) & 1u);
-        if (lane == c) occ = bal;
+        for (uint32_t c = 0; c < LOW_COUNTERS; ++c) {
+            const uint32_t bal = __ballot_sync(0xffffffffu, (mm >> c) & 1u);
+            if (lane == c) occ = bal;
+        }
+        return occ;
+    };
+    bool mine;
+    uint32_t n = 0;
+    ReplayOut o;
+    start(0u);
+    for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+        const unsigned long long r = record(k0 + lane, mine);
+        n += __popc(__ballot_sync(0xffffffffu, mine));
+        if (mine) add(r);
     }
+    o.T = counted();
     const uint32_t lb = S.tab[s * LOW_WORDS + 7];
     uint32_t* bw = S.tab + lb * LOW_WORDS;
-    ReplayOut o;
-    o.T = __popc(occ);
     o.P = part_pre(bw, o.T);
+    // the tile that crosses (n > 32), the counters and records before it
+    uint32_t cur = o.P, before = 0, x = NONE;
+    if (n > 32) {
+        start(o.P);
+        for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+            const unsigned long long r = record(k0 + lane, mine);
+            const uint32_t bal = __ballot_sync(0xffffffffu, mine);
+            if (!bal) continue;
+            if (mine) add(r);
+            const uint32_t now = counted();
+            if (!__any_sync(0xffffffffu, now != cur && now > LIMIT + 1)) {
+                cur = now;
+                before += __popc(bal);
+                continue;
+            }
+            // the record that takes a counter to LIMIT + 2, the first of all counters'
+            const uint32_t occ = selecting(mine ? code_mask<WIDE>(S.mk[(uint32_t)r & ENT_MASK]) : 0u);
+            const uint32_t need = LIMIT + 2 - cur;  // (cur <= LIMIT + 1 so far)
+            const uint32_t j = __reduce_min_sync(0xffffffffu, now > LIMIT + 1 && now != cur ? __fns(occ, 0, need) : 32u);
+            x = __shfl_sync(0xffffffffu, tile_of(r), j);
+            const uint32_t first = __shfl_sync(0xffffffffu, tile_of(r), __ffs(bal) - 1);
+            const uint32_t lt = __ballot_sync(0xffffffffu, mine && tile_of(r) < x);
+            cur += __popc(occ & lt);
+            before += __popc(lt);
+            if (x == first && k0) {  // it may have begun in earlier groups
+                start(0u);
+                for (uint32_t q = k0; q > 0;) {
+                    q -= 32;
+                    const unsigned long long e = record(q + lane, mine);
+                    const bool in = mine && tile_of(e) == x;
+                    if (in) add(e);
+                    before -= __popc(__ballot_sync(0xffffffffu, in));
+                    if (__any_sync(0xffffffffu, mine && !in)) break;  // records of an earlier tile
+                }
+                cur -= counted();
+            }
+            break;
+        }
+    }
+    uint32_t m = 0;
+    if (n <= 32 || x != NONE) {
+        uint32_t c = 0;
+        for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+            const unsigned long long r = record(k0 + lane, mine);
+            const bool in = mine && (x == NONE || tile_of(r) == x);
+            const uint32_t bal = __ballot_sync(0xffffffffu, in);
+            if (c + __popc(bal) > 32) return false;
+            if (in) buf[c + __popc(bal & lanemask_lt())] = r;
+            c += __popc(bal);
+        }
+        __syncwarp();
+        // in array order: by tile and index in it
+        unsigned long long r = ~0ull;
+        if (lane < c) {
+            r = buf[lane];
+            const uint32_t at = (uint32_t)(r >> ENT_MASK_BITS);
+            r = (unsigned long long)((at & ~in_tile) + __ldcg(Q.idx + at)) << ENT_MASK_BITS | (r & ENT_MASK);
+        }
+        __syncwarp();
+        buf[lane] = r;
+        __syncwarp();
+        uint32_t rank = 0;
+        for (uint32_t k = 0; k < c; ++k) rank += buf[k] < r;
+        __syncwarp();
+        if (lane < c) buf[rank] = r;  // positions are distinct
+        __syncwarp();
+        r = buf[lane];
+        m = lane < c ? code_mask<WIDE>(S.mk[(uint32_t)r & ENT_MASK]) : 0u;
+        o.L = (uint32_t)(r >> ENT_MASK_BITS);  // lane i: the i-th record's position
+    }
+    const uint32_t occ = selecting(m);
     bool trig = false;
     for (uint32_t mm = m; __any_sync(0xffffffffu, mm != 0); mm &= mm - 1) {
         const int c = mm ? __ffs(mm) - 1 : 0;
-        const uint32_t bal = __shfl_sync(0xffffffffu, occ, c), P = __shfl_sync(0xffffffffu, o.P, c);
+        const uint32_t bal = __shfl_sync(0xffffffffu, occ, c), P = __shfl_sync(0xffffffffu, cur, c);
         trig |= mm && P + __popc(bal & lanemask_lt()) > LIMIT;
     }
     const uint32_t tb = __ballot_sync(0xffffffffu, trig);
     if (tb) {
         const int j = __ffs(tb) - 1;
-        o.cur = o.P + __popc(occ & ((1u << j) - 1u));
+        o.cur = cur + __popc(occ & ((1u << j) - 1u));
         o.mL = __shfl_sync(0xffffffffu, m, j);
-        const uint32_t pos = __shfl_sync(0xffffffffu, (uint32_t)(r >> ENT_MASK_BITS), j);
+        const uint32_t pos = __shfl_sync(0xffffffffu, o.L, j);
         const uint32_t H = high_increments(D, o);
         __syncwarp();
         part_write_low(bw, o.cur);
-        open_row(D, S, accs, s_nacc, lb, b0, pos, n - j, H);
+        open_row(D, S, accs, s_nacc, lb, b0, pos, n - before - j, H);
     } else if (lane == 0) {
         S.w7[lb] = 0u;  // every key added low
     }
@@ -661,10 +758,13 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
     }
     const PartView V = part_view<BATCH>(D, Q, B, stream);
     if (V.tiles == 0) return;
-    const ApShared S = ap_carve(smem, V.shift, D.n_masks);
+    ApShared S = ap_carve(smem, V.shift, D.n_masks);
+    S.stream = stream;
     __shared__ uint32_t s_nflag, s_nrec, s_many, s_drop, s_rb, s_rk, s_nacc, s_new, s_row;
     __shared__ uint32_t s_cnt[LOW_COUNTERS + 2];  // bisection: counts per counter, keys, mask
     __shared__ uint32_t s_pre[LOW_COUNTERS];
+    __shared__ uint32_t s_wcnt[4096 / 32];  // records of each warp's 32 entries, then those before them
+    __shared__ uint32_t s_rcnt[AP_WARPS][32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (uint32_t i = tid; i < D.n_masks; i += AP_THREADS) S.mk[i] = mask_code<WIDE>(__ldg(D.masks + i));  // the host's
     const uint32_t accs = ap_accs(V.shift);
@@ -760,37 +860,73 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             __syncthreads();
             const uint32_t F = s_nflag;
             if (F == 0) continue;
-            // the records of the flagged buckets
-            auto record = [&](uint32_t x, uint32_t r, uint32_t at) {
-                const uint32_t w7 = S.w7[x >> ENT_MASK_BITS];
-                if (!(w7 & FLAG)) return;
-                const uint32_t k = atomicAdd(&s_nrec, 1u), pos = (tile_s + r) * tile + __ldcg(Q.idx + at);
-                if (k < cap)
-                    S.recs[k] = (unsigned long long)(w7 & ~FLAG) << 46 | (unsigned long long)pos << ENT_MASK_BITS |
-                                (x & ENT_MASK);
+            // the records of the flagged buckets (slot, entry, mask number), in the entries' order
+            auto put = [&](uint32_t k, uint32_t x, uint32_t at) {
+                S.recs[k] = (unsigned long long)(S.w7[x >> ENT_MASK_BITS] & ~FLAG) << 46 |
+                            (unsigned long long)at << ENT_MASK_BITS | (x & ENT_MASK);
             };
             if (!one_run) {
+                uint32_t hits = 0;  // bit u: entry u
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const uint32_t k = u * AP_THREADS + tid;
-                    if (k < sub) record(e[u], S.map[k], S.dlt[S.map[k]] + base + k);
+                    const bool hit = u * AP_THREADS + tid < sub && (S.w7[e[u] >> ENT_MASK_BITS] & FLAG);
+                    const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+                    hits |= hit ? 1u << u : 0u;
+                    if (lane == 0) s_wcnt[u * AP_WARPS + wid] = __popc(bal);
+                }
+                __syncthreads();
+                if (wid == 0) {
+                    uint32_t c[4], sum = 0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum += c[i] = s_wcnt[4 * lane + i];
+                    uint32_t v = sum;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, v, d);
+                        if (lane >= d) v += y;
+                    }
+                    if (lane == 31) s_nrec = v;
+                    v -= sum;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        s_wcnt[4 * lane + i] = v;
+                        v += c[i];
+                    }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t bal = __ballot_sync(0xffffffffu, (hits >> u) & 1u), k = u * AP_THREADS + tid;
+                    if ((hits >> u) & 1u)
+                        put(s_wcnt[u * AP_WARPS + wid] + __popc(bal & lanemask_lt()), e[u], S.dlt[S.map[k]] + base + k);
                 }
             } else {
-                for (uint32_t k = tid; k < sub; k += AP_THREADS)
-                    record(__ldcg(Q.ent + S.dlt[rb] + base + k), rb, S.dlt[rb] + base + k);
+                for (uint32_t k = tid; k < sub; k += AP_THREADS) {
+                    const uint32_t at = S.dlt[rb] + base + k, x = __ldcg(Q.ent + at);
+                    if (!(S.w7[x >> ENT_MASK_BITS] & FLAG)) continue;
+                    const uint32_t i = atomicAdd(&s_nrec, 1u);
+                    if (i < cap) put(i, x, at);
+                }
             }
             __syncthreads();
             const uint32_t K = s_nrec;
             if (K <= cap) {
-                // a warp replays a bucket of up to 32 records on its own
                 for (uint32_t s = wid; s < F; s += AP_WARPS)
-                    if (!replay_few<WIDE>(D, S, reinterpret_cast<unsigned long long*>(S.map) + wid * 32, accs, &s_nacc, s,
-                                          K, (uint32_t)b0, &s_rb, &s_rk) && lane == 0)
+                    if (!replay_warp<WIDE>(D, Q, S, reinterpret_cast<unsigned long long*>(S.map) + wid * 32, s_rcnt[wid], accs,
+                                           &s_nacc, s, K, (uint32_t)b0, &s_rb, &s_rk) && lane == 0)
                         s_many = 1;
                 __syncthreads();
             }
-            // longer ones: all records sorted (12 k cycles for 300 of them), then a warp each
+            // a bucket with more than 32 records of the tile that crosses: all records sorted by
+            // position (12 k cycles for 300 of them), then a warp each
             if (K <= cap && s_many) {
+                for (uint32_t k = tid; k < K; k += AP_THREADS) {
+                    const unsigned long long r = S.recs[k];
+                    const uint32_t at = (uint32_t)(r >> ENT_MASK_BITS);
+                    S.recs[k] = (r >> 46) << 46 |
+                                (unsigned long long)((at & ~(tile - 1u)) + __ldcg(Q.idx + at)) << ENT_MASK_BITS |
+                                (r & ENT_MASK);
+                }
                 block_sort(S.recs, K);
                 for (uint32_t s = wid; s < F; s += AP_WARPS) {
                     const uint32_t lb = S.tab[s * LOW_WORDS + 7];
@@ -931,7 +1067,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             uint32_t r = 0;
             if (lane == 0) r = atomicAdd(&s_row, 1u);
             r = __shfl_sync(0xffffffffu, r, 0);
-            put_row(D, r, (uint32_t)b0 + lb, id, S.acc[a * ACC_WORDS + LOW_COUNTERS], v);
+            put_row(D, r, S.stream, (uint32_t)b0 + lb, id, S.acc[a * ACC_WORDS + LOW_COUNTERS], v);
         } else {
             if (v) atomicAdd(D.high + (uint64_t)(id - START) * HIGH_WORDS + lane, v);
             if (lane == 0) S.w7[lb] = id;
@@ -978,8 +1114,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev 
         uint32_t id = base + switch_rank(D, spre, w.x), st = 0;
         bool ok = (uint64_t)(id - START) < D.n_high;
         if (BATCH) {  // ranked within the stream (its positions are contiguous) on its own allocator
-            if (lane == 0) st = stream_of_bucket(B, b);
-            st = __shfl_sync(0xffffffffu, st, 0);
+            st = __ldcg(D.sw_base + r);
             const uint32_t own = __ldcg(B.base_id + st) + (id - base) -
                                  switch_rank(D, spre, __ldcg(B.item_off + st) * Q.tile);
             const uint32_t nh = __ldg(&B.desc[st].n_high);
@@ -1116,6 +1251,11 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
     return part_steps(d_keys, n, D, Q, BatchDev{}, L, small, hot, Q.parts, st);
 }
 
+cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, cudaStream_t st) {
+    k_part_hot_batch<<<B.n_streams, 256, 0, st>>>(d_keys, B, first);
+    return cudaGetLastError();
+}
+
 cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const PartDev& part, const BatchDev& B,
                               const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t part_lo,
                               uint32_t part_hi, bool small, bool hot, cudaStream_t st) {
@@ -1125,7 +1265,6 @@ cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const Pa
     Q.tiles = tiles;
     Q.part0 = part_lo;
     k_part_plan<<<1, 1024, 0, st>>>(B, W, Q.tile, D.ctl);
-    if (hot) k_part_hot_batch<<<W.s_hi - W.s_lo, 256, 0, st>>>(d_keys, B, W.s_lo);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return part_steps(d_keys, 0, D, Q, B, L, small, hot, part_hi - part_lo, st);
