@@ -174,6 +174,7 @@ struct BatchDev {
     uint32_t* run_off;        // [n_streams + 1] prefix of the streams' run bounds in PartDev::off
     uint32_t* base_id;        // [n_streams] next_id when the window began
     uint32_t* hot;            // [n_streams][BATCH_HOT] heavy keys of each stream in this call
+    uint32_t* hot_mul;        // [n_streams] the multiplier of each stream's sets in `hot`
     uint32_t n_streams;       // 0: not a batch
     uint32_t pad;
 };

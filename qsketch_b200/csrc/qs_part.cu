@@ -159,13 +159,16 @@ __global__ void __launch_bounds__(1024) k_part_plan(BatchDev B, BatchWindow W, u
     }
 }
 
-__device__ __forceinline__ uint32_t batch_hot_set(uint32_t key) { return (key * 0x9E3779B1u) >> 26; }
+// The set of a key in a stream's table, under the multiplier its stream was given.
+__device__ __forceinline__ uint32_t batch_hot_set(uint32_t key, uint32_t mul) { return (key * mul) >> 26; }
 static_assert(BATCH_HOT == 2 * 64, "batch_hot_set yields 6 bits, two keys per set");
 
 // A block per dense stream: keys seen at least four times in 4096 samples of its keys from `first` on
-// (short streams: none), the heaviest first, as k_part_hot.
+// (short streams: none).  Sets are few, and a heavy key that finds its set full would go through
+// one block entry by entry (0.5 M of them, 0.9 ms), so each of the eight warps tries a multiplier
+// and the one that leaves the least weight out is kept with the stream.
 __global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restrict__ keys, BatchDev B, uint64_t first) {
-    constexpr uint32_t N = 4096, SLOTS = 4096;
+    constexpr uint32_t N = 4096, SLOTS = 4096, LIST = 512;
     __shared__ uint32_t s_key[SLOTS], s_cnt[SLOTS], s_hot[BATCH_HOT];
     const uint32_t tid = threadIdx.x, s = blockIdx.x;
     const uint64_t o0 = __ldcg(B.key_off + s), all = __ldcg(B.key_off + s + 1) - o0;
@@ -194,16 +197,46 @@ __global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restri
             }
         }
         __syncthreads();
+        // the candidates, the heaviest tier first
+        __shared__ uint32_t s_list[LIST], s_n, s_occ[8][BATCH_HOT / 2], s_lost[8];
+        if (tid == 0) s_n = 0;
+        for (uint32_t i = tid; i < 8 * BATCH_HOT / 2; i += 256) (&s_occ[0][0])[i] = 0u;
+        __syncthreads();
         uint32_t hi = 0xffffffffu;
         for (uint32_t least : {64u, 16u, 4u}) {
-            for (uint32_t i = tid; i < SLOTS; i += 256) {
-                if (s_cnt[i] < least || s_cnt[i] >= hi) continue;
-                const uint32_t h = 2 * batch_hot_set(s_key[i]);
-                if (atomicCAS(s_hot + h, HOT_EMPTY, s_key[i]) != HOT_EMPTY) atomicCAS(s_hot + h + 1, HOT_EMPTY, s_key[i]);
-            }
+            for (uint32_t i = tid; i < SLOTS; i += 256)
+                if (s_cnt[i] >= least && s_cnt[i] < hi) {
+                    const uint32_t at = atomicAdd(&s_n, 1u);
+                    if (at < LIST) s_list[at] = i;
+                }
             hi = least;
             __syncthreads();
         }
+        const uint32_t n = min(s_n, LIST), wid = tid >> 5, lane = tid & 31;
+        auto mul = [](uint32_t w) { return 0x9E3779B1u + w * 0x3C6EF372u; };  // odd
+        uint32_t lost = 0;
+        for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            if (i < n && atomicAdd(&s_occ[wid][batch_hot_set(s_key[s_list[i]], mul(wid))], 1u) >= 2u) lost += s_cnt[s_list[i]];
+            __syncwarp();
+        }
+        lost = __reduce_add_sync(0xffffffffu, lost);
+        if (lane == 0) s_lost[wid] = lost;
+        __syncthreads();
+        uint32_t best = 0;
+        for (uint32_t w = 1; w < 8; ++w) best = s_lost[w] < s_lost[best] ? w : best;
+        if (wid == 0) {
+            for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+                if (i0 + lane < n) {
+                    const uint32_t key = s_key[s_list[i0 + lane]], h = 2 * batch_hot_set(key, mul(best));
+                    if (atomicCAS(s_hot + h, HOT_EMPTY, key) != HOT_EMPTY) atomicCAS(s_hot + h + 1, HOT_EMPTY, key);
+                }
+                __syncwarp();
+            }
+            if (lane == 0) B.hot_mul[s] = mul(best);
+        }
+    } else if (tid == 0) {
+        B.hot_mul[s] = 1u;
     }
     __syncthreads();
     for (uint32_t i = tid; i < BATCH_HOT; i += 256) B.hot[(uint64_t)s * BATCH_HOT + i] = s_hot[i];
@@ -229,10 +262,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
         D.ctl->n_switch = 0;
         D.ctl->link_base = D.ctl->next_id;
     }
-    uint32_t stream = 0;
+    uint32_t stream = 0, hot_mul = 0;
     PartView V = part_view<false>(D, Q, B, 0);
     auto load_hot = [&] {  // the hot keys whose buckets are linked
         const uint32_t* hot = BATCH ? B.hot + (uint64_t)stream * BATCH_HOT : Q.hot;
+        if (BATCH) hot_mul = __ldcg(B.hot_mul + stream);
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
             uint32_t key = __ldcg(hot + i), id = 0;
             if (key != HOT_EMPTY) {
@@ -303,7 +337,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             bool live = i < cnt;
             if (!BATCH && D.skip && live) live = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
             if (HOT && live) {
-                const uint32_t s = 2 * (BATCH ? batch_hot_set(e[j]) : hot_set(e[j]));
+                const uint32_t s = 2 * (BATCH ? batch_hot_set(e[j], hot_mul) : hot_set(e[j]));
                 const uint2 hk = *reinterpret_cast<const uint2*>(s_hkey + s);
                 if (e[j] != HOT_EMPTY && (hk.x == e[j] || hk.y == e[j])) {
                     atomicAdd(s_hcnt + s + (hk.x != e[j]), 1u);
@@ -590,6 +624,17 @@ __device__ __forceinline__ void block_sort(unsigned long long* recs, uint32_t K)
 // done with by then); cnt: 32 counts of the warp.
 static_assert(ap_unit(11) * 2 >= AP_WARPS * 32 * 8, "the run map holds every warp's 32 records");
 template <bool WIDE>
+__device__ __forceinline__ void count_record(const ApShared& S, uint32_t* cnt, uint32_t x) {
+    const uint32_t q = S.mk[x & ENT_MASK];
+    if (WIDE) {
+        for (uint32_t mm = q; mm; mm &= mm - 1) atomicAdd(cnt + (__ffs(mm) - 1), 1u);
+    } else {
+        atomicAdd(cnt + (q & 31u), 1u);
+        atomicAdd(cnt + ((q >> 5) & 31u), 1u);
+        atomicAdd(cnt + (q >> 10), 1u);
+    }
+}
+template <bool WIDE>
 __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, const ApShared& S,
                                             unsigned long long* buf, uint32_t* cnt, uint32_t accs, uint32_t* s_nacc,
                                             uint32_t s, uint32_t K, uint32_t b0, uint32_t* s_rb, uint32_t* s_rk) {
@@ -601,16 +646,7 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
     };
     auto tile_of = [&](unsigned long long r) { return (uint32_t)(r >> ENT_MASK_BITS) & ~in_tile; };
     // adds a record's counters to cnt; lane c then reads counter c
-    auto add = [&](unsigned long long r) {
-        const uint32_t q = S.mk[(uint32_t)r & ENT_MASK];
-        if (WIDE) {
-            for (uint32_t mm = q; mm; mm &= mm - 1) atomicAdd(cnt + (__ffs(mm) - 1), 1u);
-        } else {
-            atomicAdd(cnt + (q & 31u), 1u);
-            atomicAdd(cnt + ((q >> 5) & 31u), 1u);
-            atomicAdd(cnt + (q >> 10), 1u);
-        }
-    };
+    auto add = [&](unsigned long long r) { count_record<WIDE>(S, cnt, (uint32_t)r); };
     auto start = [&](uint32_t v) {
         __syncwarp();
         cnt[lane] = v;
@@ -633,18 +669,23 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
     bool mine;
     uint32_t n = 0;
     ReplayOut o;
-    start(0u);
-    for (uint32_t k0 = 0; k0 < K; k0 += 32) {
-        const unsigned long long r = record(k0 + lane, mine);
-        n += __popc(__ballot_sync(0xffffffffu, mine));
-        if (mine) add(r);
+    if (s < AP_WARPS) {  // counted as the records were gathered (cnt is this slot's row)
+        n = __shfl_sync(0xffffffffu, cnt[lane], LOW_COUNTERS);
+    } else {
+        start(0u);
+        for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+            const unsigned long long r = record(k0 + lane, mine);
+            n += __popc(__ballot_sync(0xffffffffu, mine));
+            if (mine) add(r);
+        }
+        __syncwarp();
     }
-    o.T = counted();
+    o.T = lane < LOW_COUNTERS ? cnt[lane] : 0u;
     const uint32_t lb = S.tab[s * LOW_WORDS + 7];
     uint32_t* bw = S.tab + lb * LOW_WORDS;
     o.P = part_pre(bw, o.T);
     // the tile that crosses (n > 32), the counters and records before it
-    uint32_t cur = o.P, before = 0, x = NONE;
+    uint32_t cur = o.P, before = 0, x = NONE, from = 0;  // from: the first group with records of tile x
     if (n > 32) {
         start(o.P);
         for (uint32_t k0 = 0; k0 < K; k0 += 32) {
@@ -667,10 +708,11 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
             const uint32_t lt = __ballot_sync(0xffffffffu, mine && tile_of(r) < x);
             cur += __popc(occ & lt);
             before += __popc(lt);
+            from = k0;
             if (x == first && k0) {  // it may have begun in earlier groups
                 start(0u);
                 for (uint32_t q = k0; q > 0;) {
-                    q -= 32;
+                    from = q -= 32;
                     const unsigned long long e = record(q + lane, mine);
                     const bool in = mine && tile_of(e) == x;
                     if (in) add(e);
@@ -685,10 +727,11 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
     uint32_t m = 0;
     if (n <= 32 || x != NONE) {
         uint32_t c = 0;
-        for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+        for (uint32_t k0 = from; k0 < K; k0 += 32) {
             const unsigned long long r = record(k0 + lane, mine);
             const bool in = mine && (x == NONE || tile_of(r) == x);
             const uint32_t bal = __ballot_sync(0xffffffffu, in);
+            if (x != NONE && __any_sync(0xffffffffu, mine && tile_of(r) > x) && !bal) break;
             if (c + __popc(bal) > 32) return false;
             if (in) buf[c + __popc(bal & lanemask_lt())] = r;
             c += __popc(bal);
@@ -835,9 +878,12 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             const bool one_run = sub > cap;  // then r1 == rb + 1: no map needed
             uint32_t e[U];
             if (!one_run) {
-                for (uint32_t r = rb + wid * 4 + (lane >> 3); r < r1; r += AP_WARPS * 4) {  // eight lanes per run
+                // the run of each entry: eight lanes per run, a warp or the whole block where a unit
+                // has few long ones (eight lanes alone take 10 k cycles for 3,000 entries)
+                const uint32_t nruns = r1 - rb, G = nruns > 4 * AP_WARPS ? 8u : nruns > 2 ? 32u : (uint32_t)AP_THREADS;
+                for (uint32_t r = rb + tid / G; r < r1; r += AP_THREADS / G) {
                     const uint32_t k1 = S.before[r + 1] - base;
-                    for (uint32_t k = S.before[r] - base + (lane & 7); k < k1; k += 8) S.map[k] = (uint16_t)r;
+                    for (uint32_t k = S.before[r] - base + (tid & (G - 1u)); k < k1; k += G) S.map[k] = (uint16_t)r;
                 }
                 __syncthreads();
 #pragma unroll
@@ -862,9 +908,14 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             if (F == 0) continue;
             // the records of the flagged buckets (slot, entry, mask number), in the entries' order
             auto put = [&](uint32_t k, uint32_t x, uint32_t at) {
-                S.recs[k] = (unsigned long long)(S.w7[x >> ENT_MASK_BITS] & ~FLAG) << 46 |
-                            (unsigned long long)at << ENT_MASK_BITS | (x & ENT_MASK);
+                const uint32_t slot = S.w7[x >> ENT_MASK_BITS] & ~FLAG;
+                S.recs[k] = (unsigned long long)slot << 46 | (unsigned long long)at << ENT_MASK_BITS | (x & ENT_MASK);
+                if (slot < AP_WARPS) {  // the totals of the first slots, one per warp
+                    count_record<WIDE>(S, s_rcnt[slot], x);
+                    atomicAdd(&s_rcnt[slot][LOW_COUNTERS], 1u);
+                }
             };
+            s_rcnt[wid][lane] = 0u;
             if (!one_run) {
                 uint32_t hits = 0;  // bit u: entry u
 #pragma unroll
@@ -901,6 +952,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
                         put(s_wcnt[u * AP_WARPS + wid] + __popc(bal & lanemask_lt()), e[u], S.dlt[S.map[k]] + base + k);
                 }
             } else {
+                __syncthreads();
                 for (uint32_t k = tid; k < sub; k += AP_THREADS) {
                     const uint32_t at = S.dlt[rb] + base + k, x = __ldcg(Q.ent + at);
                     if (!(S.w7[x >> ENT_MASK_BITS] & FLAG)) continue;

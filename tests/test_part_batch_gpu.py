@@ -47,7 +47,7 @@ def draw(lengths, seed, s=1.1, ranks=1 << 14):
 
 
 # lengths at the edges of the first round, the tiles and the rule; sketches at the edges of the partitions
-LENGTHS = [32767, 32768, 32769, 0, 1, 49152, 49153, 100001, 262144, 600011]
+LENGTHS = [32767, 32768, 32769, 0, 1, 131072, 131073, 100001, 262144, 600011]
 LOWS = [63, 64, 1021, 1024, 1025, 16381, 32749, 131071, 131073, 5003]
 
 
