@@ -261,10 +261,15 @@ qs_status insert_device(qs_sketch* sk, const uint32_t* d_keys, size_t n, cudaStr
     if (sk->kind == QS_KIND_MSWS) {
         bool hot = false;  // the call's heavy keys are sampled
         for (size_t off = 0; off < n;) {
-            if (sk->P.parts && !table && n >= sk->part_min) {
+            if (sk->P.parts && n >= sk->part_min) {
                 const uint64_t c = part_chunk(sk, n - off);
                 MswsDev D = sk->D;
                 D.skip = skip ? skip + off / 32 : nullptr;
+                if (table) {
+                    D.tbl_keys = table->keys;
+                    D.tbl_counts = table->counts;
+                    D.tbl_slots = table->slots;
+                }
                 CK(sk->prof_begin(0, st), "profile");
                 if (!hot && sk->fresh && n - off >= PART_HOT_MIN) {
                     CK(part_hot(d_keys + off, n - off, sk->P, st), "heavy keys");
@@ -536,8 +541,9 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         P.ent = rb;
         P.idx = reinterpret_cast<uint16_t*>(rb + sk->part_cap);
         if (P.parts) {
-            // tiles of a chunk: whole ones, or the small ones of a chunk below PART_SMALL_MAX keys
-            P.stride = (uint32_t)std::max(sk->part_cap / PART_TILE,
+            // tiles of a chunk: PART_TILE_TABLE keys at least, or the small ones of a chunk below
+            // PART_SMALL_MAX keys
+            P.stride = (uint32_t)std::max(sk->part_cap / PART_TILE_TABLE,
                                           std::min(sk->part_cap, PART_SMALL_MAX) / PART_TILE_SMALL);
             CKB(sk->alloc(&P.hot, PART_HOT), "alloc heavy keys");
             CKB(sk->alloc(&P.off, (uint64_t)(P.parts + 1) * P.stride), "alloc run bounds");
@@ -1800,9 +1806,11 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
     qs_sketch* sk = b->sk;
     BatchDev B = b->B;
     B.key_off = d_offsets;
-    const uint64_t first = 1ull << 17;  // (2^14: 11.8 ms a pass over 512 streams, 2^16 11.2, 2^17 11.0)
+    // (2^14: 11.8 ms a pass over 512 streams, 2^16 11.2, 2^17 11.0)
+    const uint64_t first = std::min<uint64_t>(1ull << 17, sk->part_cap / 4);
     // one window: the streams [s_lo, s_hi), each stream's keys [r0, r1)
-    auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1, bool small) -> qs_status {
+    auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1, bool small,
+                   bool hot) -> qs_status {
         const uint64_t tile = small ? PART_TILE_SMALL : PART_TILE;
         uint64_t tiles = 0;
         for (uint32_t i = s_lo; i < s_hi; ++i) {
@@ -1815,7 +1823,6 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
         W.rel_lo = r0;
         W.rel_hi = r1;
         W.which = STREAMS_DENSE;
-        const bool hot = r0 > 0;
         CK(sk->prof_begin(0, st), "profile");
         CK(part_insert_batch(d_keys, sk->D, b->P, B, sk->PL, W, (uint32_t)tiles, b->part_off[s_lo], b->part_off[s_hi],
                              small, hot, st),
@@ -1836,7 +1843,7 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
             qs_status s = QS_OK;
             // tiles of 2048 keys in the first round (a heavy key's run of a tile stays within a
             // unit), and while larger ones would leave SMs idle
-            if (keys) s = run(lo, hi, r0, r1, !round);
+            if (keys) s = run(lo, hi, r0, r1, !round, round != 0);
             slots = keys = runs = 0;
             lo = hi;
             return s;
@@ -1848,8 +1855,8 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
             if (part > sk->part_cap) {  // one stream's slice alone exceeds a window: split it
                 qs_status s = close(i);
                 if (s != QS_OK) return s;
-                for (uint64_t a = r0; a < len; a += sk->part_cap) {
-                    s = run(i, i + 1, a, std::min(len, a + sk->part_cap), false);
+                for (uint64_t a = r0; a < std::min(len, r1); a += sk->part_cap) {
+                    s = run(i, i + 1, a, std::min(std::min(len, r1), a + sk->part_cap), false, round != 0);
                     if (s != QS_OK) return s;
                 }
                 lo = i + 1;

@@ -57,7 +57,7 @@ __host__ __device__ constexpr uint32_t ap_accs(uint32_t shift) { return shift > 
 constexpr uint32_t HOT_SETS = PART_HOT / 2;  // two keys per set
 constexpr uint32_t HOT_BLOCKS = 16, HOT_THREADS = 512;
 constexpr uint32_t HOT_SAMPLES = 16384, HOT_SLOTS = 2048, HOT_MIN = 3;
-constexpr uint32_t HOT_EMPTY = 0xffffffffu;
+constexpr uint32_t HOT_EMPTY = 0xffffffffu, IN_TABLE = 0x80000000u;
 
 __device__ __forceinline__ uint32_t hot_set(uint32_t key) { return (key * 0x9E3779B1u) >> 22; }
 static_assert(HOT_SETS == 1024, "hot_set yields 10 bits");
@@ -246,7 +246,10 @@ __global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restri
 
 // HOT: keys of the call's hot table whose bucket is linked when the chunk begins are counted in
 // shared memory (high-level additions commute) and never become entries.
-template <int PT_THREADS, int KPT, bool HOT, bool BATCH>
+// TABLE (learned split): keys of the exact table count there (D.tbl_keys, D.tbl_counts) and never
+// become entries; four lookups of a thread are in flight at a time, and the table's heavy keys are
+// counted in shared memory with the others.
+template <int PT_THREADS, int KPT, bool HOT, bool BATCH, bool TABLE>
 __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(const uint32_t* __restrict__ keys, uint64_t n, MswsDev D,
                                                               PartDev Q, BatchDev B) {
     constexpr uint32_t R = PT_THREADS * KPT, HOTS = BATCH ? BATCH_HOT : PART_HOT;
@@ -269,7 +272,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
         if (BATCH) hot_mul = __ldcg(B.hot_mul + stream);
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
             uint32_t key = __ldcg(hot + i), id = 0;
-            if (key != HOT_EMPTY) {
+            const int ts = TABLE && key != HOT_EMPTY ? table_find(D.tbl_keys, D.tbl_slots, key) : -1;
+            if (ts >= 0) {
+                id = IN_TABLE | (uint32_t)ts;
+            } else if (key != HOT_EMPTY) {
                 id = __ldcg(D.low + (uint64_t)(V.low_base + fast_mod(V.fm, key * V.seed)) * LOW_WORDS + 7);
                 if (!is_linked(D, id)) key = HOT_EMPTY;
             }
@@ -282,6 +288,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
             const uint32_t c = s_hcnt[i];
             if (!c) continue;
+            if (TABLE && (s_hid[i] & IN_TABLE)) {
+                atomicAdd(D.tbl_counts + (s_hid[i] & ~IN_TABLE), c);
+                continue;
+            }
             uint32_t* hb = D.high + (uint64_t)(s_hid[i] - START) * HIGH_WORDS;
             for (uint32_t m = __ldg(D.masks + fast_mod(D.fm_mask, s_hkey[i] * V.seed)); m; m &= m - 1)
                 atomicAdd(hb + (__ffs(m) - 1), c);
@@ -331,23 +341,60 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             }
         }
         __syncthreads();
+        uint32_t live = 0;  // bit j: key j goes to the sketch
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
             const uint32_t i = (j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3);
-            bool live = i < cnt;
-            if (!BATCH && D.skip && live) live = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
-            if (HOT && live) {
+            bool on = i < cnt;
+            if (!BATCH && !TABLE && D.skip && on) on = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
+            if (HOT && on) {
                 const uint32_t s = 2 * (BATCH ? batch_hot_set(e[j], hot_mul) : hot_set(e[j]));
                 const uint2 hk = *reinterpret_cast<const uint2*>(s_hkey + s);
                 if (e[j] != HOT_EMPTY && (hk.x == e[j] || hk.y == e[j])) {
                     atomicAdd(s_hcnt + s + (hk.x != e[j]), 1u);
-                    live = false;
+                    on = false;
                 }
             }
+            live |= on ? 1u << j : 0u;
+        }
+        if (TABLE) {
+#pragma unroll
+            for (int j0 = 0; j0 < KPT; j0 += 4) {
+                uint4 a[4], c[4];  // the keys' first sectors
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t sec = mix32(e[j0 + j]) & (D.tbl_slots / TBL_SECTOR - 1u);
+                    const uint4* q = reinterpret_cast<const uint4*>(D.tbl_keys + (uint64_t)sec * TBL_SECTOR);
+                    a[j] = (live >> (j0 + j)) & 1u ? __ldg(q) : make_uint4(HOT_EMPTY, 0, 0, 0);
+                    c[j] = (live >> (j0 + j)) & 1u ? __ldg(q + 1) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t key = e[j0 + j];
+                    if (!((live >> (j0 + j)) & 1u) || key == HOT_EMPTY) continue;
+                    const uint32_t k8[8] = {a[j].x, a[j].y, a[j].z, a[j].w, c[j].x, c[j].y, c[j].z, c[j].w};
+                    int at = -1;
+                    bool room = false;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        if (k8[q] == key) at = q;
+                        room |= k8[q] == HOT_EMPTY;
+                    }
+                    int ts = at < 0 ? -1 : (int)((mix32(key) & (D.tbl_slots / TBL_SECTOR - 1u)) * TBL_SECTOR + at);
+                    if (at < 0 && !room) ts = table_find(D.tbl_keys, D.tbl_slots, key);  // a full first sector
+                    if (ts >= 0) {
+                        atomicAdd(D.tbl_counts + ts, 1u);
+                        live &= ~(1u << (j0 + j));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
             const uint32_t hv = e[j] * V.seed;
             const uint32_t b = fast_mod(V.fm, hv), p = b >> V.shift;
             e[j] = ((b & ((1u << V.shift) - 1u)) << ENT_MASK_BITS) | fast_mod(D.fm_mask, hv);
-            pr[j] = live ? (p << 16) | atomicAdd(s_hist + p, 1u) : NONE;
+            pr[j] = (live >> j) & 1u ? (p << 16) | atomicAdd(s_hist + p, 1u) : NONE;
         }
         __syncthreads();
         {  // first position of each partition; its row of the run bounds
@@ -1227,14 +1274,20 @@ static size_t split_smem(uint32_t tile, uint32_t parts, uint32_t hot) {
     return (size_t)tile * 6 + parts * 4 + hot * 12;
 }
 
-static const void* split_fn(bool small, bool hot, bool batch) {
+// Kernel and threads of a split by tile size.
+static const void* split_fn(uint32_t tile, bool hot, bool batch) {
+    if (tile == PART_TILE_TABLE)
+        return hot ? (const void*)k_part_split<1024, 8, true, false, true> : (const void*)k_part_split<1024, 8, false, false, true>;
+    const bool small = tile == PART_TILE_SMALL;
     if (batch)
-        return small ? (hot ? (const void*)k_part_split<512, 4, true, true> : (const void*)k_part_split<512, 4, false, true>)
-                     : (hot ? (const void*)k_part_split<1024, 16, true, true>
-                            : (const void*)k_part_split<1024, 16, false, true>);
-    return small ? (hot ? (const void*)k_part_split<512, 4, true, false> : (const void*)k_part_split<512, 4, false, false>)
-                 : (hot ? (const void*)k_part_split<1024, 16, true, false>
-                        : (const void*)k_part_split<1024, 16, false, false>);
+        return small ? (hot ? (const void*)k_part_split<512, 4, true, true, false>
+                            : (const void*)k_part_split<512, 4, false, true, false>)
+                     : (hot ? (const void*)k_part_split<1024, 16, true, true, false>
+                            : (const void*)k_part_split<1024, 16, false, true, false>);
+    return small ? (hot ? (const void*)k_part_split<512, 4, true, false, false>
+                        : (const void*)k_part_split<512, 4, false, false, false>)
+                 : (hot ? (const void*)k_part_split<1024, 16, true, false, false>
+                        : (const void*)k_part_split<1024, 16, false, false, false>);
 }
 
 static const void* apply_fn(bool wide, bool batch) {
@@ -1255,7 +1308,8 @@ cudaError_t part_configure(int num_sms, PartLaunch* L) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
     for (int batch = 0; batch < 2; ++batch) {
-        for (int i = 0; i < 4; ++i) cap(split_fn(i & 1, i & 2, batch != 0), split_max);
+        for (uint32_t tile : {PART_TILE, PART_TILE_SMALL, PART_TILE_TABLE})
+            for (int hot = 0; hot < 2; ++hot) cap(split_fn(tile, hot != 0, batch != 0), split_max);
         for (int wide = 0; wide < 2; ++wide) cap(apply_fn(wide != 0, batch != 0), apply_max);
     }
     cap((const void*)k_part_link<false>, link_max);
@@ -1272,15 +1326,16 @@ cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cu
 
 // Split, apply and link of a chunk (or a batch's window) whose tiles Q names.
 static cudaError_t part_steps(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& Q, const BatchDev& B,
-                              const PartLaunch& L, bool small, bool hot, uint32_t blocks, cudaStream_t st) {
+                              const PartLaunch& L, bool hot, uint32_t blocks, cudaStream_t st) {
     MswsDev Dc = D;
     PartDev Qc = Q;
     BatchDev Bc = B;
     const bool batch = B.n_streams != 0;
     {
         void* args[] = {(void*)&d_keys, (void*)&n, (void*)&Dc, (void*)&Qc, (void*)&Bc};
+        const bool small = Q.tile == PART_TILE_SMALL;
         const int grid = (int)std::min<uint64_t>(Q.tiles, (uint64_t)(small ? 2 * L.num_sms : L.num_sms));
-        const cudaError_t e = cudaLaunchKernel(split_fn(small, hot, batch), dim3(grid), dim3(small ? 512 : 1024), args,
+        const cudaError_t e = cudaLaunchKernel(split_fn(Q.tile, hot, batch), dim3(grid), dim3(small ? 512 : 1024), args,
                                                split_smem(Q.tile, Q.parts, hot ? (batch ? BATCH_HOT : PART_HOT) : 0), st);
         if (e != cudaSuccess) return e;
     }
@@ -1297,10 +1352,9 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
     if (n == 0) return cudaSuccess;
     PartDev Q = part;
     // tiles of 2048 keys while larger ones would leave SMs idle
-    const bool small = n < PART_SMALL_MAX;
-    Q.tile = small ? PART_TILE_SMALL : PART_TILE;
+    Q.tile = D.tbl_keys ? PART_TILE_TABLE : n < PART_SMALL_MAX ? PART_TILE_SMALL : PART_TILE;
     Q.tiles = (uint32_t)((n + Q.tile - 1) / Q.tile);
-    return part_steps(d_keys, n, D, Q, BatchDev{}, L, small, hot, Q.parts, st);
+    return part_steps(d_keys, n, D, Q, BatchDev{}, L, hot, Q.parts, st);
 }
 
 cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, cudaStream_t st) {
@@ -1319,7 +1373,7 @@ cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const Pa
     k_part_plan<<<1, 1024, 0, st>>>(B, W, Q.tile, D.ctl);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return part_steps(d_keys, 0, D, Q, B, L, small, hot, part_hi - part_lo, st);
+    return part_steps(d_keys, 0, D, Q, B, L, hot, part_hi - part_lo, st);
 }
 
 }  // namespace qsb
