@@ -108,6 +108,7 @@ struct qs_sketch {
     MswsLaunch L{};
     PartDev P{};              // partitioned insert: its scratch (P.parts == 0: not used)
     PartLaunch PL{};
+    bool own_knobs = false;   // the caller fixed a pass-1 knob: its calls go through pass 1
     uint64_t part_cap = 0;    // keys a partitioned chunk takes
     uint64_t part_min = 0;    // and the fewest it pays for
     CmDev C{};
@@ -259,6 +260,13 @@ qs_status insert_device(qs_sketch* sk, const uint32_t* d_keys, size_t n, cudaStr
                         const uint32_t* skip = nullptr, const TableDev* table = nullptr, uint32_t* skipbuf = nullptr) {
     sk->seen = std::min(sk->seen + n, SEEN_UNKNOWN);
     if (sk->kind == QS_KIND_MSWS) {
+        if (n <= SMALL_STREAM && !sk->own_knobs && !skip && !table) {
+            CK(sk->prof_begin(0, st), "profile");
+            CK(small_insert(d_keys, n, sk->D, st), "small insert");
+            CK(sk->prof_end(0, st), "profile");
+            sk->fresh += n;
+            return QS_OK;
+        }
         bool hot = false;  // the call's heavy keys are sampled
         for (size_t off = 0; off < n;) {
             if (sk->P.parts && n >= sk->part_min) {
@@ -502,6 +510,7 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         // knobs are left to the library
         const bool own_knobs = p.lanes_per_key || p.aggregate || p.route || p.ctas_per_sm || p.keys_per_tile ||
                                (p.flags & QS_FLAG_NO_CHUNK_RAMP);
+        sk->own_knobs = own_knobs;
         PartDev& P = sk->P;
         P.shift = PART_MIN_SHIFT;
         while (P.shift < PART_MAX_SHIFT && (n_low >> P.shift) >= 640) ++P.shift;
@@ -1769,6 +1778,13 @@ BatchWindow flat_window(uint64_t c0, uint64_t c1) {
     return W;
 }
 
+// The window of an insert graph: its short slices a block each, unless the caller fixed pass-1 knobs.
+BatchWindow graph_window(const qs_batch* b, uint64_t max_total) {
+    BatchWindow W = flat_window(0, max_total);
+    if (!b->sk->own_knobs) W.which = STREAMS_LONG;
+    return W;
+}
+
 // Consecutive size classes with the same lanes per key share one pass-1 launch.
 void batch_rebuild_runs(qs_batch* b) {
     b->runs.clear();
@@ -1788,6 +1804,10 @@ qs_status batch_insert_seq(qs_batch* b, const uint32_t* d_keys, const uint64_t* 
     B.key_off = d_offsets;
     CK(batch_plan(B, sk->D.ctl, W, strict, st), "batch plan");
     if (timed) CK(sk->prof_begin(0, st), "profile");
+    if (W.which == STREAMS_LONG) {
+        CK(small_insert_batch(d_keys, sk->D, B, st), "small batch insert");
+        ++b->info.launches;
+    }
     for (size_t r = 0; r < b->runs.size(); ++r)
         CK(batch_insert_pass(d_keys, sk->D, B, sk->L, sk->agg, b->runs[r].lpk, b->runs[r].k_lo, b->runs[r].k_hi,
                              (uint32_t)r, st),
@@ -2233,10 +2253,10 @@ qs_status qs_batch_insert_graph(qs_batch* b, const uint32_t* d_keys, const uint6
     bool ran = false;
     s = batch_graph(b, 0, d_keys, d_offsets, nullptr, max_total, st,
                     [&](cudaStream_t cs) {
-                        return batch_insert_seq(b, d_keys, d_offsets, flat_window(0, max_total), true, cs, false);
+                        return batch_insert_seq(b, d_keys, d_offsets, graph_window(b, max_total), true, cs, false);
                     },
                     &ran);
-    if (s == QS_OK && !ran) s = batch_insert_seq(b, d_keys, d_offsets, flat_window(0, max_total), true, st);
+    if (s == QS_OK && !ran) s = batch_insert_seq(b, d_keys, d_offsets, graph_window(b, max_total), true, st);
     if (s == QS_OK) ++b->info.inserts;
     return s;
 }

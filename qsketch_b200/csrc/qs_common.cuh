@@ -189,9 +189,12 @@ struct BatchWindow {
     uint64_t rel_lo, rel_hi;
     uint32_t s_lo, s_hi;
     uint32_t flat;
-    uint32_t which;  // all streams, or only the dense or the sparse ones (batch_dense)
+    uint32_t which;  // all streams, or only the dense or the sparse ones (batch_dense), or (flat)
+                     // work items only for the slices of more than SMALL_STREAM keys
 };
-enum { STREAMS_ALL = 0, STREAMS_DENSE = 1, STREAMS_SPARSE = 2 };
+enum { STREAMS_ALL = 0, STREAMS_DENSE = 1, STREAMS_SPARSE = 2, STREAMS_LONG = 3 };
+// Keys of a stream in one call that one block takes by itself (k_msws_small).
+constexpr uint64_t SMALL_STREAM = 4096;
 // Streams whose keys go through the partitioned insert: at least a key to a bucket and 2^15 keys in
 // the call.  The partitioned insert streams a sketch's table twice (about 46 ps a bucket) and takes
 // 20-30 ps a key; pass 1 and the replay take 66 ps a key.

@@ -40,6 +40,11 @@ cudaError_t msws_repair(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
 cudaError_t msws_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, const MswsDev& D, const MswsLaunch& L,
                        cudaStream_t st);
 
+// Few keys (qs_small.cu): one block, start to end; a batch's slices of at most SMALL_STREAM keys (their
+// bounds from batch_plan), a block each.
+cudaError_t small_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, cudaStream_t st);
+cudaError_t small_insert_batch(const uint32_t* d_keys, const MswsDev& D, const BatchDev& B, cudaStream_t st);
+
 // Partitioned insert (qs_part.cu) of one chunk: split, apply, link.
 struct PartLaunch {
     int num_sms = 0;

@@ -1778,6 +1778,8 @@ __global__ void __launch_bounds__(1024) k_batch_plan(BatchDev B, BatchWindow W, 
         }
         B.lo[s] = lo;
         B.hi[s] = hi;
+        // a slice that one block takes by itself keeps its bounds but no work items
+        if (W.which == STREAMS_LONG && hi - lo <= SMALL_STREAM) lo = hi;
         B.item_off[s] = (uint32_t)((hi - lo + INS_TILE - 1) / INS_TILE);
         B.wpre[s] = (uint32_t)(hi - lo);
     }
