@@ -216,14 +216,24 @@ qs_status check_status_word(qs_sketch* sk) {
     return QS_OK;
 }
 
+Ctl ctl_init() {
+    Ctl c;
+    std::memset(&c, 0, sizeof c);
+    c.next_id = FIRST_ID;
+    return c;
+}
+
 qs_status ctl_reset(qs_sketch* sk, cudaStream_t st) {
-    static const Ctl init = [] {
-        Ctl c;
-        std::memset(&c, 0, sizeof c);
-        c.next_id = FIRST_ID;
-        return c;
-    }();
+    static const Ctl init = ctl_init();
     CK(cudaMemcpyAsync(sk->D.ctl, &init, sizeof init, cudaMemcpyHostToDevice, st), "reset control block");
+    return QS_OK;
+}
+
+// Clears an MSWS sketch (or a batch's arena and its per-stream state).
+qs_status clear_msws(qs_sketch* sk, const BatchDev& B, cudaStream_t st) {
+    sk->seen = sk->arena ? SEEN_UNKNOWN : 0;
+    sk->fresh = 0;
+    CK(msws_clear(sk->D, ctl_init(), B, sk->L.num_sms, st), "clear");
     return QS_OK;
 }
 
@@ -765,13 +775,8 @@ qs_status qs_clear(qs_sketch* sk, void* stream) {
     if (!sk) return fail(QS_ERR_INVALID_ARG, "null sketch");
     DeviceGuard guard(sk->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    sk->seen = sk->arena ? SEEN_UNKNOWN : 0;
-    if (sk->kind == QS_KIND_MSWS) {
-        CK(cudaMemsetAsync(sk->D.low, 0, sk->D.n_low * LOW_WORDS * 4, st), "clear low");
-        CK(cudaMemsetAsync(sk->D.high, 0, sk->D.n_high * HIGH_WORDS * 4, st), "clear high");
-        sk->fresh = 0;
-        return ctl_reset(sk, st);
-    }
+    if (sk->kind == QS_KIND_MSWS) return clear_msws(sk, BatchDev{}, st);
+    sk->seen = 0;
     CK(cudaMemsetAsync(sk->C.table, 0, sk->C.n * sk->C.rows * 4, st), "clear table");
     return QS_OK;
 }
@@ -2393,17 +2398,8 @@ qs_status qs_batch_autotune(qs_batch* b, const uint32_t* d_keys, const uint64_t*
 
 qs_status qs_batch_clear(qs_batch* b, void* stream) {
     if (!b) return fail(QS_ERR_INVALID_ARG, "null batch");
-    qs_status s = qs_clear(b->sk, stream);
-    if (s != QS_OK) return s;
     DeviceGuard guard(b->sk->device);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    std::vector<uint32_t> first(b->S, FIRST_ID);
-    CK(cudaMemcpyAsync(b->B.next_id, first.data(), (size_t)b->S * 4, cudaMemcpyHostToDevice, st), "reset allocators");
-    CK(cudaMemsetAsync(b->B.status, 0, (size_t)b->S * 4, st), "reset stream status");
-    // the clear restarts the control block's link generation, which tags these
-    CK(cudaMemsetAsync(b->B.first, 0, (size_t)b->S * 8, st), "reset link ranks");
-    CK(cudaStreamSynchronize(st), "clear sync");  // the host vector above must outlive the copy
-    return QS_OK;
+    return clear_msws(b->sk, b->B, static_cast<cudaStream_t>(stream));
 }
 
 qs_status qs_batch_sync(qs_batch* b, void* stream) {

@@ -252,6 +252,32 @@ __global__ void __launch_bounds__(SM_THREADS) k_msws_small(const uint32_t* __res
     }
 }
 
+// A cleared sketch in one launch (two memsets and a copy before, three more copies and memsets and a
+// host wait for a batch): tables to zero with 16-byte stores, the control block and the batch's
+// per-stream state to their initial values.
+__global__ void __launch_bounds__(512) k_msws_clear(MswsDev D, Ctl init, BatchDev B) {
+    const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, all = (uint64_t)gridDim.x * blockDim.x;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4* low = reinterpret_cast<uint4*>(D.low);
+    uint4* high = reinterpret_cast<uint4*>(D.high);
+    const uint64_t nl = D.n_low * (LOW_WORDS / 4), nh = D.n_high * (HIGH_WORDS / 4);
+    for (uint64_t i = gtid; i < nl; i += all) low[i] = zero;
+    for (uint64_t i = gtid; i < nh; i += all) high[i] = zero;
+    if (gtid == 0) *D.ctl = init;
+    for (uint64_t s = gtid; s < B.n_streams; s += all) {
+        B.next_id[s] = FIRST_ID;
+        B.status[s] = 0u;
+        B.first[s] = 0ull;  // the control block's link generation, which tags these, restarts
+    }
+}
+
+cudaError_t msws_clear(const MswsDev& D, const Ctl& init, const BatchDev& B, int num_sms, cudaStream_t st) {
+    const uint64_t words = std::max<uint64_t>(D.n_low * (LOW_WORDS / 4), D.n_high * (HIGH_WORDS / 4));
+    const int grid = (int)std::min<uint64_t>((uint64_t)num_sms * 4, (words + 511) / 512);
+    k_msws_clear<<<grid, 512, 0, st>>>(D, init, B);
+    return cudaGetLastError();
+}
+
 cudaError_t small_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     MswsDev Dc = D;
