@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
     uint32_t* s_hcnt = s_hkey + HOTS;
     uint32_t* s_hid = s_hcnt + HOTS;
     uint32_t* s_hist = HOT ? s_hid + HOTS : s_hkey;                // [parts] counts, then first positions
+    __shared__ uint32_t s_dead[TABLE ? R / 32 : 1], s_more;  // TABLE: keys found after their first sector
     const int tid = threadIdx.x;
     if (!BATCH && blockIdx.x == 0 && tid == 0) {
         D.ctl->n_switch = 0;
@@ -347,46 +348,83 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             const uint32_t i = (j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3);
             bool on = i < cnt;
             if (!BATCH && !TABLE && D.skip && on) on = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
-            if (HOT && on) {
-                const uint32_t s = 2 * (BATCH ? batch_hot_set(e[j], hot_mul) : hot_set(e[j]));
-                const uint2 hk = *reinterpret_cast<const uint2*>(s_hkey + s);
-                if (e[j] != HOT_EMPTY && (hk.x == e[j] || hk.y == e[j])) {
-                    atomicAdd(s_hcnt + s + (hk.x != e[j]), 1u);
-                    on = false;
-                }
-            }
             live |= on ? 1u << j : 0u;
         }
-        if (TABLE) {
+        if (HOT) {  // four sets' loads in flight: a thread otherwise waits one shared-memory round per key
 #pragma unroll
             for (int j0 = 0; j0 < KPT; j0 += 4) {
-                uint4 a[4], c[4];  // the keys' first sectors
+                uint32_t set[4];
+                uint2 hk[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    set[j] = 2 * (BATCH ? batch_hot_set(e[j0 + j], hot_mul) : hot_set(e[j0 + j]));
+                    hk[j] = *reinterpret_cast<const uint2*>(s_hkey + set[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t key = e[j0 + j], bit = 1u << (j0 + j);
+                    const bool x = hk[j].x == key, y = hk[j].y == key;
+                    if ((x || y) && key != HOT_EMPTY && (live & bit)) {
+                        atomicAdd(s_hcnt + set[j] + (x ? 0u : 1u), 1u);
+                        live &= ~bit;
+                    }
+                }
+            }
+        }
+        if (TABLE) {
+            // Each key's first sector; the few whose sector is full without the key (one in
+            // five at the table's highest fill) are listed and probed on by whole warps.
+            uint32_t* l_key = s_ent;   // free until the scatter
+            uint16_t* l_idx = s_idx;
+            if (tid == 0) s_more = 0;
+            for (uint32_t i = tid; i < R / 32; i += PT_THREADS) s_dead[i] = 0u;
+            __syncthreads();
+#pragma unroll
+            for (int j0 = 0; j0 < KPT; j0 += 4) {
+                uint4 a[4], c[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t sec = mix32(e[j0 + j]) & (D.tbl_slots / TBL_SECTOR - 1u);
                     const uint4* q = reinterpret_cast<const uint4*>(D.tbl_keys + (uint64_t)sec * TBL_SECTOR);
-                    a[j] = (live >> (j0 + j)) & 1u ? __ldg(q) : make_uint4(HOT_EMPTY, 0, 0, 0);
-                    c[j] = (live >> (j0 + j)) & 1u ? __ldg(q + 1) : make_uint4(0, 0, 0, 0);
+                    const bool on = (live >> (j0 + j)) & 1u;
+                    a[j] = on ? __ldg(q) : make_uint4(HOT_EMPTY, 0, 0, 0);
+                    c[j] = on ? __ldg(q + 1) : make_uint4(0, 0, 0, 0);
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const uint32_t key = e[j0 + j];
-                    if (!((live >> (j0 + j)) & 1u) || key == HOT_EMPTY) continue;
+                    const uint32_t key = e[j0 + j], bit = 1u << (j0 + j);
                     const uint32_t k8[8] = {a[j].x, a[j].y, a[j].z, a[j].w, c[j].x, c[j].y, c[j].z, c[j].w};
-                    int at = -1;
+                    uint32_t at = 8;
                     bool room = false;
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        if (k8[q] == key) at = q;
+                        at = k8[q] == key ? (uint32_t)q : at;
                         room |= k8[q] == HOT_EMPTY;
                     }
-                    int ts = at < 0 ? -1 : (int)((mix32(key) & (D.tbl_slots / TBL_SECTOR - 1u)) * TBL_SECTOR + at);
-                    if (at < 0 && !room) ts = table_find(D.tbl_keys, D.tbl_slots, key);  // a full first sector
-                    if (ts >= 0) {
-                        atomicAdd(D.tbl_counts + ts, 1u);
-                        live &= ~(1u << (j0 + j));
+                    const bool on = (live & bit) && key != HOT_EMPTY;
+                    if (on && at < 8u) {
+                        atomicAdd(D.tbl_counts + (mix32(key) & (D.tbl_slots / TBL_SECTOR - 1u)) * TBL_SECTOR + at, 1u);
+                        live &= ~bit;
+                    } else if (on && !room) {
+                        const uint32_t l = atomicAdd(&s_more, 1u);
+                        l_key[l] = key;
+                        l_idx[l] = (uint16_t)((j0 / 4) * 4 * PT_THREADS + 4 * tid + j);
                     }
                 }
+            }
+            __syncthreads();
+            for (uint32_t l = tid; l < s_more; l += PT_THREADS) {
+                const int ts = table_find(D.tbl_keys, D.tbl_slots, l_key[l]);
+                if (ts >= 0) {
+                    atomicAdd(D.tbl_counts + ts, 1u);
+                    atomicOr(s_dead + (l_idx[l] >> 5), 1u << (l_idx[l] & 31));
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int v = 0; v < KPT / 4; ++v) {
+                const uint32_t i = v * 4 * PT_THREADS + 4 * tid;
+                live &= ~(((s_dead[i >> 5] >> (i & 31)) & 0xfu) << (4 * v));
             }
         }
 #pragma unroll
@@ -419,11 +457,17 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             if (tid == 0) V.off[(uint64_t)parts * V.stride + lt] = (uint16_t)total;
             __syncthreads();
 #pragma unroll
-            for (int j = 0; j < KPT; ++j) {
-                if (pr[j] == NONE) continue;
-                const uint32_t pos = s_hist[pr[j] >> 16] + (pr[j] & 0xffffu);
-                s_ent[pos] = e[j];
-                s_idx[pos] = (uint16_t)((j / 4) * 4 * PT_THREADS + 4 * tid + (j & 3));
+            for (int j0 = 0; j0 < KPT; j0 += 4) {
+                uint32_t pos[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    pos[j] = pr[j0 + j] == NONE ? NONE : s_hist[pr[j0 + j] >> 16] + (pr[j0 + j] & 0xffffu);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (pos[j] == NONE) continue;
+                    s_ent[pos[j]] = e[j0 + j];
+                    s_idx[pos[j]] = (uint16_t)((j0 / 4) * 4 * PT_THREADS + 4 * tid + j);
+                }
             }
             __syncthreads();
             uint4* ge = reinterpret_cast<uint4*>(Q.ent + p0);
