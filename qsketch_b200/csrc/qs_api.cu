@@ -560,9 +560,8 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         P.ent = rb;
         P.idx = reinterpret_cast<uint16_t*>(rb + sk->part_cap);
         if (P.parts) {
-            // tiles of a chunk: PART_TILE_TABLE keys at least, or the small ones of a chunk below
-            // PART_SMALL_MAX keys
-            P.stride = (uint32_t)std::max(sk->part_cap / PART_TILE_TABLE,
+            // tiles of a chunk: whole ones, or the small ones of a chunk below PART_SMALL_MAX keys
+            P.stride = (uint32_t)std::max(sk->part_cap / PART_TILE,
                                           std::min(sk->part_cap, PART_SMALL_MAX) / PART_TILE_SMALL);
             CKB(sk->alloc(&P.hot, PART_HOT), "alloc heavy keys");
             CKB(sk->alloc(&P.off, (uint64_t)(P.parts + 1) * P.stride), "alloc run bounds");

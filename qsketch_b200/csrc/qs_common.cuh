@@ -131,7 +131,6 @@ struct PartDev {
     uint32_t part0;   // batch: the window's first partition among all streams'
 };
 constexpr uint32_t PART_TILE = 16384, PART_TILE_SMALL = 2048;
-constexpr uint32_t PART_TILE_TABLE = 8192;        // with the learned split's table lookups
 constexpr uint64_t PART_SMALL_MAX = 148ull * PART_TILE;  // chunks below this many keys take small tiles
 constexpr uint32_t PART_MAX_PARTS = 2048, PART_MIN_SHIFT = 6, PART_MAX_SHIFT = 11;
 constexpr uint32_t PART_MAX_MASKS = 2048;         // mask tables the apply step keeps in shared memory

@@ -268,7 +268,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
     }
     uint32_t stream = 0, hot_mul = 0;
     PartView V = part_view<false>(D, Q, B, 0);
+    bool any_hot = false;
     auto load_hot = [&] {  // the hot keys whose buckets are linked
+        bool mine = false;
         const uint32_t* hot = BATCH ? B.hot + (uint64_t)stream * BATCH_HOT : Q.hot;
         if (BATCH) hot_mul = __ldcg(B.hot_mul + stream);
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
@@ -283,7 +285,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             s_hkey[i] = key;
             s_hcnt[i] = 0u;
             s_hid[i] = id;
+            mine |= key != HOT_EMPTY;
         }
+        any_hot = __syncthreads_or(mine);
     };
     auto flush_hot = [&] {  // their counts: one add per counter
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             if (!BATCH && !TABLE && D.skip && on) on = !((__ldg(D.skip + ((k0 + i) >> 5)) >> ((k0 + i) & 31)) & 1u);
             live |= on ? 1u << j : 0u;
         }
-        if (HOT) {  // four sets' loads in flight: a thread otherwise waits one shared-memory round per key
+        if (HOT && any_hot) {  // four sets' loads in flight: a thread otherwise waits one shared-memory round per key
 #pragma unroll
             for (int j0 = 0; j0 < KPT; j0 += 4) {
                 uint32_t set[4];
@@ -1319,9 +1323,9 @@ static size_t split_smem(uint32_t tile, uint32_t parts, uint32_t hot) {
 }
 
 // Kernel and threads of a split by tile size.
-static const void* split_fn(uint32_t tile, bool hot, bool batch) {
-    if (tile == PART_TILE_TABLE)
-        return hot ? (const void*)k_part_split<1024, 8, true, false, true> : (const void*)k_part_split<1024, 8, false, false, true>;
+static const void* split_fn(uint32_t tile, bool hot, bool batch, bool table) {
+    if (table)
+        return hot ? (const void*)k_part_split<1024, 16, true, false, true> : (const void*)k_part_split<1024, 16, false, false, true>;
     const bool small = tile == PART_TILE_SMALL;
     if (batch)
         return small ? (hot ? (const void*)k_part_split<512, 4, true, true, false>
@@ -1352,8 +1356,7 @@ cudaError_t part_configure(int num_sms, PartLaunch* L) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
     for (int batch = 0; batch < 2; ++batch) {
-        for (uint32_t tile : {PART_TILE, PART_TILE_SMALL, PART_TILE_TABLE})
-            for (int hot = 0; hot < 2; ++hot) cap(split_fn(tile, hot != 0, batch != 0), split_max);
+        for (int i = 0; i < 8; ++i) cap(split_fn(i & 1 ? PART_TILE : PART_TILE_SMALL, i & 2, batch != 0, i & 4), split_max);
         for (int wide = 0; wide < 2; ++wide) cap(apply_fn(wide != 0, batch != 0), apply_max);
     }
     cap((const void*)k_part_link<false>, link_max);
@@ -1379,7 +1382,7 @@ static cudaError_t part_steps(const uint32_t* d_keys, uint64_t n, const MswsDev&
         void* args[] = {(void*)&d_keys, (void*)&n, (void*)&Dc, (void*)&Qc, (void*)&Bc};
         const bool small = Q.tile == PART_TILE_SMALL;
         const int grid = (int)std::min<uint64_t>(Q.tiles, (uint64_t)(small ? 2 * L.num_sms : L.num_sms));
-        const cudaError_t e = cudaLaunchKernel(split_fn(Q.tile, hot, batch), dim3(grid), dim3(small ? 512 : 1024), args,
+        const cudaError_t e = cudaLaunchKernel(split_fn(Q.tile, hot, batch, D.tbl_keys != nullptr), dim3(grid), dim3(small ? 512 : 1024), args,
                                                split_smem(Q.tile, Q.parts, hot ? (batch ? BATCH_HOT : PART_HOT) : 0), st);
         if (e != cudaSuccess) return e;
     }
@@ -1396,7 +1399,7 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
     if (n == 0) return cudaSuccess;
     PartDev Q = part;
     // tiles of 2048 keys while larger ones would leave SMs idle
-    Q.tile = D.tbl_keys ? PART_TILE_TABLE : n < PART_SMALL_MAX ? PART_TILE_SMALL : PART_TILE;
+    Q.tile = !D.tbl_keys && n < PART_SMALL_MAX ? PART_TILE_SMALL : PART_TILE;
     Q.tiles = (uint32_t)((n + Q.tile - 1) / Q.tile);
     return part_steps(d_keys, n, D, Q, BatchDev{}, L, hot, Q.parts, st);
 }
