@@ -131,12 +131,16 @@ struct PartDev {
     uint32_t part0;   // batch: the window's first partition among all streams'
 };
 constexpr uint32_t PART_TILE = 16384, PART_TILE_SMALL = 2048;
-constexpr uint64_t PART_SMALL_MAX = 148ull * PART_TILE;  // chunks below this many keys take small tiles
+// Chunks below this many keys (half a large tile per SM) take small tiles.  Uniform calls of 2^20 keys
+// 34 us with small tiles, 36 with large ones; 1.3M 42 / 36; 2.4M 83 / 65.
+constexpr uint64_t PART_SMALL_MAX = 74ull * PART_TILE;
 constexpr uint32_t PART_MAX_PARTS = 2048, PART_MIN_SHIFT = 6, PART_MAX_SHIFT = 11;
 constexpr uint32_t PART_MAX_MASKS = 2048;         // mask tables the apply step keeps in shared memory
 constexpr uint64_t PART_MAX_CHUNK = 1ull << 26;
 constexpr uint32_t PART_HOT = 2048;               // heavy keys of a call
-constexpr uint64_t PART_HOT_MIN = 1ull << 21;      // calls of at least this many keys are sampled for them
+// Calls of at least this many keys are sampled for them (9-12 us a call with the lookups): 1.6M Zipf 1.1
+// keys 140 -> 59 us, Zipf 0.8 67 -> 65, uniform 36 -> 47; at 2^20 95 -> 61, 54 -> 63, 34 -> 43.
+constexpr uint64_t PART_HOT_MIN = 3ull << 19;
 
 // Batched streams: many per-stream MSWS sketches share one low-table arena and one high
 // pool arena.  A stream's sketch is the bucket range [low_base, low_base + fm_low.d) of the

@@ -55,16 +55,17 @@ __host__ __device__ constexpr uint32_t ap_accs(uint32_t shift) { return shift > 
 // ---- 0: the heavy keys of a call ---------------------------------------------------------
 
 constexpr uint32_t HOT_SETS = PART_HOT / 2;  // two keys per set
-constexpr uint32_t HOT_BLOCKS = 16, HOT_THREADS = 512;
-constexpr uint32_t HOT_SAMPLES = 16384, HOT_SLOTS = 2048, HOT_MIN = 3;
+constexpr uint32_t HOT_BLOCKS = 64, HOT_THREADS = 1024;
+constexpr uint32_t HOT_SAMPLES = 16384, HOT_SLOTS = 1024, HOT_MIN = 3;
 constexpr uint32_t HOT_EMPTY = 0xffffffffu, IN_TABLE = 0x80000000u;
 
 __device__ __forceinline__ uint32_t hot_set(uint32_t key) { return (key * 0x9E3779B1u) >> 22; }
 static_assert(HOT_SETS == 1024, "hot_set yields 10 bits");
 
 // Keys seen at least HOT_MIN times among HOT_SAMPLES evenly spaced ones (a share of about 2e-4).
-// Every block reads the whole sample and counts the keys of its own sets: one block's atomics on
-// one SM take 28 us, sixteen blocks' a quarter of it.  Which keys the table keeps when a set
+// Every block reads the whole sample and counts the keys of its own sets.  What bounds it is the
+// latency of one block's steps: 16 blocks of 512 threads with a sector per key 19 us, with a sector
+// per four keys 13 us, 64 blocks of 1024 threads 7 us.  Which keys the table keeps when a set
 // overflows (the heaviest go first) does not change any result.
 __global__ void __launch_bounds__(HOT_THREADS) k_part_hot(const uint32_t* __restrict__ keys, uint64_t n, uint32_t* hot) {
     __shared__ uint32_t s_key[HOT_SLOTS], s_cnt[HOT_SLOTS];
@@ -73,11 +74,16 @@ __global__ void __launch_bounds__(HOT_THREADS) k_part_hot(const uint32_t* __rest
     const uint32_t tid = threadIdx.x, set0 = blockIdx.x * SETS;
     for (uint32_t i = tid; i < HOT_SLOTS; i += HOT_THREADS) s_key[i] = HOT_EMPTY, s_cnt[i] = 0u;
     for (uint32_t i = tid; i < 2 * SETS; i += HOT_THREADS) s_hot[i] = HOT_EMPTY;
-    const uint64_t step = n / HOT_SAMPLES;
+    // four neighbouring keys per place: the scattered sectors bound the reads (an SM takes one in
+    // about two cycles), not the keys
+    const uint32_t* base = reinterpret_cast<const uint32_t*>((reinterpret_cast<uintptr_t>(keys) + 15) & ~(uintptr_t)15);
+    const uint64_t step = (n - 3) / HOT_SAMPLES;  // in units of four keys, times four places
     uint32_t k[HOT_SAMPLES / HOT_THREADS];
 #pragma unroll
-    for (uint32_t j = 0; j < HOT_SAMPLES / HOT_THREADS; ++j)
-        k[j] = __ldg(keys + step * (uint64_t)(j * HOT_THREADS + tid));
+    for (uint32_t j = 0; j < HOT_SAMPLES / HOT_THREADS / 4; ++j) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(base) + step * (uint64_t)(j * HOT_THREADS + tid));
+        k[4 * j] = q.x, k[4 * j + 1] = q.y, k[4 * j + 2] = q.z, k[4 * j + 3] = q.w;
+    }
     __syncthreads();
 #pragma unroll
     for (uint32_t j = 0; j < HOT_SAMPLES / HOT_THREADS; ++j) {
@@ -268,7 +274,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
     }
     uint32_t stream = 0, hot_mul = 0;
     PartView V = part_view<false>(D, Q, B, 0);
-    bool any_hot = false;
+    // Learned chunks skip the lookups while no hot key is linked or in the table (0.45 -> 0.44 ms a pass);
+    // for plain ones the branch costs Zipf streams more (1 %) than it gives uniform ones.
+    bool any_hot = !TABLE;
     auto load_hot = [&] {  // the hot keys whose buckets are linked
         bool mine = false;
         const uint32_t* hot = BATCH ? B.hot + (uint64_t)stream * BATCH_HOT : Q.hot;
@@ -287,7 +295,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             s_hid[i] = id;
             mine |= key != HOT_EMPTY;
         }
-        any_hot = __syncthreads_or(mine);
+        if (TABLE) any_hot = __syncthreads_or(mine);
     };
     auto flush_hot = [&] {  // their counts: one add per counter
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
@@ -1324,9 +1332,12 @@ static size_t split_smem(uint32_t tile, uint32_t parts, uint32_t hot) {
 
 // Kernel and threads of a split by tile size.
 static const void* split_fn(uint32_t tile, bool hot, bool batch, bool table) {
-    if (table)
-        return hot ? (const void*)k_part_split<1024, 16, true, false, true> : (const void*)k_part_split<1024, 16, false, false, true>;
     const bool small = tile == PART_TILE_SMALL;
+    if (table)
+        return small ? (hot ? (const void*)k_part_split<512, 4, true, false, true>
+                            : (const void*)k_part_split<512, 4, false, false, true>)
+                     : (hot ? (const void*)k_part_split<1024, 16, true, false, true>
+                            : (const void*)k_part_split<1024, 16, false, false, true>);
     if (batch)
         return small ? (hot ? (const void*)k_part_split<512, 4, true, true, false>
                             : (const void*)k_part_split<512, 4, false, true, false>)
@@ -1398,8 +1409,8 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
                         bool hot, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     PartDev Q = part;
-    // tiles of 2048 keys while larger ones would leave SMs idle
-    Q.tile = !D.tbl_keys && n < PART_SMALL_MAX ? PART_TILE_SMALL : PART_TILE;
+    // small tiles while large ones would leave more than half of the SMs idle
+    Q.tile = n < PART_SMALL_MAX ? PART_TILE_SMALL : PART_TILE;
     Q.tiles = (uint32_t)((n + Q.tile - 1) / Q.tile);
     return part_steps(d_keys, n, D, Q, BatchDev{}, L, hot, Q.parts, st);
 }

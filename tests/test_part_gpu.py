@@ -44,6 +44,14 @@ def test_sizes_at_tile_edges_and_alignments(gpu, n, off):
     compare(sk, orc, [keys], data.rank_keys(7, 0, 1 << 15))
 
 
+@pytest.mark.parametrize("n", [74 * 16384 - 1, 74 * 16384, (3 << 19) - 1, 3 << 19])
+@pytest.mark.parametrize("off", [0, 1, 3])
+def test_second_call_at_the_edges_of_tile_size_and_heavy_key_sample(gpu, n, off):
+    sk, orc = pair(16381, 4096)
+    first, keys = data.zipf_keys(5000, 1 << 15, 1.1, seed=n, perm_seed=7), data.zipf_keys(n + off, 1 << 15, 1.1, seed=n, perm_seed=7)
+    compare(sk, orc, [first, keys[off:]], data.rank_keys(7, 0, 1 << 15))
+
+
 @pytest.mark.parametrize("n_low", [449, 512, 513, 2039, 40961, 655359, 655361, 1310719, 1310721])
 def test_table_sizes_at_partition_edges(gpu, n_low):
     sk, orc = pair(n_low, 8192)
