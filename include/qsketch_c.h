@@ -101,12 +101,12 @@ typedef struct qs_params {
                                     a multiple of 32, at most 2^26; 0 = 1<<22 */
     int32_t device;              /* CUDA device ordinal; -1 = current */
     /* Insert-kernel knobs; none changes any result.  They shape pass 1, which takes the calls
-     * that are small against the table; with all of them (and QS_FLAG_NO_CHUNK_RAMP) left at 0,
+     * that are small against the table.  With all of them (and QS_FLAG_NO_CHUNK_RAMP) left at 0,
      * calls of at least max(2^18, 1.5 n_low) keys are partitioned by bucket range and applied in
-     * shared memory instead, in chunks of up to 4 * max_batch keys.  When lanes_per_key, aggregate, route
-     * and ctas_per_sm are all 0, qs_create takes them (and max_batch, if 0) from the
-     * autotuner's entry for the sketch's size class (qs_autotune), else the defaults
-     * 4 / 3 / 1 / 0. */
+     * shared memory instead, in chunks of up to 4 * max_batch keys, and calls of at most 4096
+     * keys run in one kernel of one block.  When lanes_per_key, aggregate, route and ctas_per_sm
+     * are all 0, qs_create takes them (and max_batch, if 0) from the autotuner's entry for the
+     * sketch's size class (qs_autotune), else the defaults 4 / 3 / 1 / 0. */
     uint32_t lanes_per_key;      /* lanes serving one key in pass 1: 1, 2, 4, 8 (one lane
                                     per bucket word, the reference's sub-warp), 16 or 32 */
     uint32_t aggregate;          /* 1 = off, 2 = warp, 3 = warp + block pre-aggregation
@@ -214,7 +214,7 @@ qs_status qs_get_stats(qs_sketch *sk, qs_stats *out);
  * profiling was on, measured with CUDA events recorded around each launch on the stream
  * it ran on, and are reset by each qs_get_profile call. */
 typedef struct qs_profile {
-    double insert_ms;          /* pass-1 insert kernels (MSWS) / insert kernels (CM) */
+    double insert_ms;          /* insert kernels: pass 1, partitioned or small (MSWS), CM */
     double repair_ms;          /* ordered-repair kernels (MSWS) */
     double query_ms;           /* query kernels */
     uint64_t insert_timed, repair_timed, query_timed;
@@ -418,8 +418,10 @@ void qs_autotune_reset(void);
  * table arena.  A call takes the keys of every stream at once as one flat device array and
  * device offsets: stream s is d_keys[d_offsets[s] .. d_offsets[s+1]), offsets non-decreasing
  * from d_offsets[0] = 0 (else QS_ERR_INVALID_ARG at the next sync), empty streams allowed.
- * One persistent launch inserts all streams (tiles of one stream each, taken from a device
- * work queue), followed by the ordered replay; each stream's result is that of inserting its
+ * Long streams are partitioned by bucket range and applied in shared memory; the others go
+ * through one persistent launch (tiles of one stream each, taken from a device work queue),
+ * followed by the ordered replay, or (graph batches' slices of at most 4096 keys) one block
+ * each; each stream's result is that of inserting its
  * keys alone, in order, into a qs_create'd sketch with the same n_low, n_high, seed and
  * masks.  Long batches run in windows of max_batch keys.  The _graph variants record the
  * whole launch sequence once per (d_keys, d_offsets, d_counts, max_total) in a CUDA graph and
@@ -442,7 +444,10 @@ typedef struct qs_batch_params {
     uint64_t first_chunk;         /* per-stream chunk ramp of qs_batch_insert: rounds over every
                                      stream's keys [0, f), [f, 2f), [2f, 4f), ... (windows of at
                                      most max_batch keys); 0 = 2^14; QS_FLAG_NO_CHUNK_RAMP in
-                                     flags: flat windows of max_batch keys */
+                                     flags: flat windows of max_batch keys.  With it and the
+                                     insert knobs left at 0, the streams of at least 2^15 and
+                                     n_low keys go through the partitioned insert in rounds of
+                                     their own, from 2^17 keys per stream */
     int32_t device;
     const uint32_t *class_lanes_per_key; /* optional host [64]: lanes per key of pass 1 for the
                                      streams of size class c = floor(log2 n_low); 0 entries take
