@@ -1753,16 +1753,12 @@ cudaError_t learned_query(const uint32_t* d_keys, uint64_t n, const TableDev& T,
 // non-decreasing from 0 latch ST_BAD_OFFSETS and empty the window; strict (flat) mode
 // latches ST_CAPACITY if the keys run past c1.
 __global__ void __launch_bounds__(1024) k_batch_plan(BatchDev B, BatchWindow W, uint32_t strict, Ctl* ctl) {
-    const uint32_t S = B.n_streams;
+    const uint32_t S = B.n_streams, tid = threadIdx.x;
+    const uint64_t first = __ldcg(B.key_off), total = __ldcg(B.key_off + S);
     bool bad = false;
-    for (uint32_t s = threadIdx.x; s < S; s += blockDim.x)
-        bad |= __ldcg(B.key_off + s + 1) < __ldcg(B.key_off + s);
-    bad = __syncthreads_or(bad) || __ldcg(B.key_off) != 0;
-    const uint64_t total = __ldcg(B.key_off + S);
-    const uint64_t e = bad ? W.c0 : umin64(W.c1, total);
-    const uint64_t b0 = umin64(W.c0, e);
-    for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
-        const uint64_t o0 = __ldcg(B.key_off + s), o1 = __ldcg(B.key_off + s + 1);
+    uint64_t e = 0, b0 = 0;
+    // stream s at [o0, o1): its slice to B.lo and B.hi; the keys of its work items
+    auto slice = [&](uint32_t s, uint64_t o0, uint64_t o1) {
         uint64_t lo, hi;
         if (bad) {
             lo = hi = 0;
@@ -1779,20 +1775,54 @@ __global__ void __launch_bounds__(1024) k_batch_plan(BatchDev B, BatchWindow W, 
         B.lo[s] = lo;
         B.hi[s] = hi;
         // a slice that one block takes by itself keeps its bounds but no work items
-        if (W.which == STREAMS_LONG && hi - lo <= SMALL_STREAM) lo = hi;
-        B.item_off[s] = (uint32_t)((hi - lo + INS_TILE - 1) / INS_TILE);
-        B.wpre[s] = (uint32_t)(hi - lo);
+        return W.which == STREAMS_LONG && hi - lo <= SMALL_STREAM ? 0u : (uint32_t)(hi - lo);
+    };
+    auto checked = [&](bool order) {
+        bad = __syncthreads_or(order) || first != 0;
+        e = bad ? W.c0 : umin64(W.c1, total);
+        b0 = umin64(W.c0, e);
+    };
+    uint32_t items, keys;
+    if (S <= 1024) {
+        // a thread per stream, everything in registers and shared memory: what bounds this one
+        // block is dependent trips to L2 (7.2 us with the arrays below at 512 streams, 5.0 so)
+        __shared__ uint32_t s_items[1024];
+        const bool on = tid < S;
+        const uint64_t o0 = on ? __ldcg(B.key_off + tid) : 0, o1 = on ? __ldcg(B.key_off + tid + 1) : 0;
+        const uint32_t grp = on ? __ldg(B.cls_streams + tid) : 0;
+        checked(o1 < o0);
+        const uint32_t len = on ? slice(tid, o0, o1) : 0u, it = (len + INS_TILE - 1) / INS_TILE;
+        s_items[tid] = it;
+        __syncthreads();
+        const uint32_t g = on ? s_items[grp] : 0u;  // in the grouped (size-class) order of the pass-1 launches
+        uint32_t unused;
+        const uint32_t i0 = block_exclusive_scan(it, &items), k0 = block_exclusive_scan(len, &keys),
+                       g0 = block_exclusive_scan(g, &unused);
+        if (on) {
+            B.item_off[tid] = i0;
+            B.wpre[tid] = k0;
+            B.cls_item_off[tid] = g0;
+        }
+    } else {
+        bool order = false;
+        for (uint32_t s = tid; s < S; s += blockDim.x) order |= __ldcg(B.key_off + s + 1) < __ldcg(B.key_off + s);
+        checked(order);
+        for (uint32_t s = tid; s < S; s += blockDim.x) {
+            const uint32_t len = slice(s, __ldcg(B.key_off + s), __ldcg(B.key_off + s + 1));
+            B.item_off[s] = (len + INS_TILE - 1) / INS_TILE;
+            B.wpre[s] = len;
+        }
+        __syncthreads();
+        // the same work items in the grouped (size-class) order of the pass-1 launches
+        for (uint32_t k = tid; k < S; k += blockDim.x) {
+            const uint32_t s = __ldg(B.cls_streams + k);
+            B.cls_item_off[k] = B.item_off[s];
+        }
+        __syncthreads();
+        items = block_scan_array(B.item_off, S);
+        keys = block_scan_array(B.wpre, S);
+        block_scan_array(B.cls_item_off, S);
     }
-    __syncthreads();
-    // the same work items in the grouped (size-class) order of the pass-1 launches
-    for (uint32_t k = threadIdx.x; k < S; k += blockDim.x) {
-        const uint32_t s = __ldg(B.cls_streams + k);
-        B.cls_item_off[k] = B.item_off[s];
-    }
-    __syncthreads();
-    const uint32_t items = block_scan_array(B.item_off, S);
-    const uint32_t keys = block_scan_array(B.wpre, S);
-    block_scan_array(B.cls_item_off, S);
     for (uint32_t c = threadIdx.x; c < MAX_SIZE_CLASSES; c += blockDim.x) B.work[c] = 0;
     if (threadIdx.x == 0) {
         B.item_off[S] = items;

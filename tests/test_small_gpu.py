@@ -57,3 +57,26 @@ def test_graph_batches_with_short_and_long_slices(gpu, lengths, pool):
         assert np.array_equal(low, orcs[s].low) and np.array_equal(high, orcs[s].high), s
     assert full == (_lib.QS_ERR_POOL_FULL if any(o.pool_full for o in orcs) else _lib.QS_OK)
     assert [bool(v & 1) for v in b.stream_status()] == [bool(o.pool_full) for o in orcs]
+
+
+@pytest.mark.parametrize("streams", [1023, 1024, 1025])
+def test_batches_at_the_edge_of_the_one_thread_per_stream_plan(gpu, streams):
+    rng = np.random.default_rng(streams)
+    lengths = rng.integers(0, 120, streams)
+    lengths[[5, streams - 1]] = [9000, 5000]
+    n_low = rng.integers(3, 600, streams).tolist()
+    b = BatchedSketches(n_low, [n + 2 for n in n_low], seed_rng=3)
+    masks = qs.generate_hashmask(1021, 32, 3, 4, 1)
+    off = np.zeros(streams + 1, np.int64)
+    off[1:] = np.cumsum(lengths)
+    h = data.zipf_keys(int(off[-1]), 200, 1.1, seed=4, perm_seed=1).cpu().numpy()
+    keys, offs = torch.from_numpy(h.view(np.int32)).cuda(), torch.from_numpy(off).cuda()
+    b.insert_graph(keys, offs)
+    b.insert(keys, offs)
+    got = b.search(keys, offs).cpu().numpy().view(np.uint32)
+    assert b.status() == _lib.QS_OK
+    for s, seed in enumerate(b.seeds()):
+        o = oracle.Msws(n_low[s], n_low[s] + 2, int(seed), masks)
+        mine = h[off[s]:off[s + 1]]
+        o.insert(np.concatenate([mine, mine]))
+        assert np.array_equal(got[off[s]:off[s + 1]], o.query(mine)), s
