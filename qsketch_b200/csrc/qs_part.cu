@@ -17,11 +17,11 @@
 //      insertion hands them out; rows move to their high buckets.
 // Nothing waits across blocks: the order between the steps is the order of the launches.
 //
-// What bounds it (2^24-key chunks): the split, instruction issue (84 warp instructions and 11
-// shared-memory passes per 32 keys; 82 us); the apply step, the latency of a unit's dependent
+// What bounds it (2^24-key chunks): the split, instruction issue and the shared-memory pipe, each
+// half busy between its barriers (88-96 warp instructions per 32 keys; 86-93 us); the apply step, the latency of a unit's dependent
 // shared-memory steps with 32 warps an SM (95 us for uniform keys, 155 us for Zipf 1.1 with the
 // heavy keys counted in the split).  Against pass 1 and the replay: 2^24 uniform keys into 8 MB
-// 0.55 -> 0.22 ms, 2^27 Zipf 1.1 keys into 64 MB 6.4 -> 2.2 ms (both with default knobs).
+// 0.55 -> 0.21 ms, 2^27 Zipf 1.1 keys into 64 MB 6.4 -> 2.2 ms (both with default knobs).
 #include "qs_kernels.h"
 #include "qs_replay.cuh"
 
@@ -255,6 +255,8 @@ __global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restri
 // TABLE (learned split): keys of the exact table count there (D.tbl_keys, D.tbl_counts) and never
 // become entries; four lookups of a thread are in flight at a time, and the table's heavy keys are
 // counted in shared memory with the others.
+// Bound by the random 32-byte sectors of the table in L2 (1 MB table, 2^24 keys: 263 us against 92
+// without); 8,192-key tiles and whole-warp probing of every key took 302 us.
 template <int PT_THREADS, int KPT, bool HOT, bool BATCH, bool TABLE>
 __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(const uint32_t* __restrict__ keys, uint64_t n, MswsDev D,
                                                               PartDev Q, BatchDev B) {

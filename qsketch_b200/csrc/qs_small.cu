@@ -7,6 +7,11 @@
 // order, so the record that takes a counter past the threshold is the switching key, and the
 // order of the switching keys gives the high ids.  Longer key runs go chunk after chunk.  A batch
 // runs one block per short stream.  Nothing waits across blocks.
+//
+// What bounds it: a chunk's three dependent trips to L2 (index words, counter atomics, link), then
+// the replay where a bucket crossed.  1,000 keys, clear + insert + query 46 -> 25 us; 512 slices of
+// 1,000 keys, pass 1 + replay 118 us -> 37 us.  256 threads a block measured the same as 512.  The
+// limit of SMALL_STREAM keys: two chunks; beyond it pass 1 spreads the keys over more SMs.
 #include "qs_kernels.h"
 #include "qs_replay.cuh"
 
