@@ -407,9 +407,9 @@ qs_status qs_draw_seeds(uint32_t rng_seed, size_t count, uint32_t* out) {
     return QS_OK;
 }
 
-// arena_chunk (batch arenas only, else 0): keys of the batch's partitioned windows; the arena's own
-// bucket ranges are not partitioned.
-static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_t arena_chunk) {
+// part_arena: a batch's arena, whose streams' bucket ranges are partitioned, each by itself, and its
+// own are not.
+static qs_status create_sketch(const qs_params* params, qs_sketch** out, bool part_arena) {
     if (!params || !out) return fail(QS_ERR_INVALID_ARG, "qs_create: null argument");
     *out = nullptr;
     const qs_params& p = *params;
@@ -528,15 +528,19 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         if (!own_knobs && B >= PART_TILE && parts >= 8 && parts <= PART_MAX_PARTS && H <= PART_MAX_MASKS &&
             p.n_high < (1ull << 28))
             P.parts = (uint32_t)parts;
+        // scratch words per chunk: the replay's records and their positions (24 B a key of B), or a
+        // partitioned chunk's entries and key indices (6 B a key); every partitioned chunk or
+        // window of this sketch, or of the batch whose arena it is, goes by part_cap
         sk->part_cap = std::min<uint64_t>(B * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE;
+        const uint64_t record_words = std::max(B * 6, (sk->part_cap * 6 + 3) / 4);
         // A partitioned chunk streams the whole table through shared memory (64 MB: 45 us), pass 1
         // touches the buckets of its keys only.  Per call, measured: 2^18 Zipf 1.1 keys into a 4 MB
         // table 48 us against 80 (uniform 22 against 19), 2^20 117 against 137 (38 / 45), 2^22 136
         // against 269 (85 / 139); 2^22 keys into 64 MB 168 against 273 (124 / 145), but 2^20 174
         // against 141 (73 / 49).
         sk->part_min = std::max<uint64_t>(1ull << 18, n_low + n_low / 2);
-        if (arena_chunk) P.parts = 0;
-        const uint64_t reach = std::max(B, P.parts ? sk->part_cap : arena_chunk);  // keys of the largest chunk
+        if (part_arena) P.parts = 0;
+        const uint64_t reach = P.parts || part_arena ? std::max(B, sk->part_cap) : B;  // keys of the largest chunk
         const uint64_t cap = std::min<uint64_t>(n_low, B), links = std::min<uint64_t>(n_low, reach);
         D.flag_cap = (uint32_t)cap;
         D.max_tiles = (uint32_t)((B + REPAIR_TILE - 1) / REPAIR_TILE);
@@ -549,10 +553,8 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         CKB(sk->alloc(&D.ctl, 1), "alloc control");
         CKB(sk->alloc(&D.flag_list, links), "alloc flag list");
         CKB(sk->alloc(&D.tile_counts, D.max_tiles), "alloc tile counts");
-        // one block: the replay's records and their positions (24 B per key of max_batch), or a
-        // partitioned chunk's entries and key indices (6 B per key of up to 4 max_batch)
         uint32_t* rb = nullptr;
-        CKB(sk->alloc(&rb, B * 6), "alloc records");
+        CKB(sk->alloc(&rb, record_words), "alloc records");
         D.rec[0] = reinterpret_cast<uint2*>(rb);
         D.rec[1] = reinterpret_cast<uint2*>(rb + 2 * B);
         D.rpos[0] = rb + 4 * B;
@@ -579,7 +581,7 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
         CKB(cudaStreamSynchronize(0), "create sync");
         e = msws_configure(dev, H, &sk->L);
         if (e != cudaSuccess) return bail(cuda_fail(e, "configure kernels"));
-        if (P.parts || arena_chunk) {
+        if (P.parts || part_arena) {
             e = part_configure(sk->L.num_sms, &sk->PL);
             if (e != cudaSuccess) return bail(cuda_fail(e, "configure partitioned insert"));
             sk->PL.apply_smem = part_apply_smem(P.shift, H);
@@ -663,7 +665,7 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, uint64_
     return QS_OK;
 }
 
-qs_status qs_create(const qs_params* params, qs_sketch** out) { return create_sketch(params, out, 0); }
+qs_status qs_create(const qs_params* params, qs_sketch** out) { return create_sketch(params, out, false); }
 
 qs_status qs_destroy(qs_sketch* sk) {
     if (!sk) return QS_OK;
@@ -2005,10 +2007,8 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
     qs_batch* b = new qs_batch();
     const bool own_knobs = p->lanes_per_key || p->aggregate || p->route || p->ctas_per_sm || p->class_lanes_per_key ||
                            p->first_chunk || (p->flags & QS_FLAG_NO_CHUNK_RAMP);
-    const uint64_t mb = p->max_batch ? p->max_batch : (1ull << 22);
-    const bool part = !own_knobs && mb >= PART_TILE && th < (1ull << 28) && p->hash_mask_table_sz <= PART_MAX_MASKS;
-    const uint64_t part_cap = part ? std::min<uint64_t>(mb * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE : 0;
-    qs_status s = create_sketch(&ap, &b->sk, part_cap);
+    bool part = !own_knobs && th < (1ull << 28) && p->hash_mask_table_sz <= PART_MAX_MASKS;
+    qs_status s = create_sketch(&ap, &b->sk, part);
     if (s != QS_OK) {
         delete b;
         return s;
@@ -2019,6 +2019,8 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
         return st;
     };
     qs_sketch* sk = b->sk;
+    // max_batch 0 takes the tuner's, so only the arena knows the windows its scratch was sized for
+    part = part && sk->max_batch >= PART_TILE;
     sk->arena = true;
     sk->seen = SEEN_UNKNOWN;  // the batch's inserts do not go through the arena sketch's
     DeviceGuard guard(sk->device);
@@ -2056,10 +2058,9 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
             if (desc[i].parts) smem = std::max(smem, part_apply_smem(sh, p->hash_mask_table_sz));
         }
         sk->PL.apply_smem = smem;
-        sk->part_cap = part_cap;
         b->P = sk->P;
         for (uint32_t i = 0; i < S; ++i) b->P.parts = std::max(b->P.parts, desc[i].parts);  // sizes the split's counts
-        b->run_cap = part_cap / PART_TILE_SMALL * 520;
+        b->run_cap = sk->part_cap / PART_TILE_SMALL * 520;
         CKB(sk->alloc(&b->P.off, b->run_cap), "alloc run bounds");
     }
     BatchDev& B = b->B;
