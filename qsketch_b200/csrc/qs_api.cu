@@ -2393,7 +2393,11 @@ qs_status qs_batch_autotune(qs_batch* b, const uint32_t* d_keys, const uint64_t*
     batch_rebuild_runs(b);
     if (h_class_lpk)
         for (uint32_t c = 0; c < MAX_SIZE_CLASSES; ++c) h_class_lpk[c] = pick[c] ? best_set[c] : 0u;
-    return qs_batch_clear(b, nullptr);
+    st = qs_batch_clear(b, nullptr);
+    if (st != QS_OK) return st;
+    // the call takes no stream: the sketches are clear for whatever stream comes next
+    CK(cudaStreamSynchronize(nullptr), "autotune sync");
+    return QS_OK;
 }
 
 qs_status qs_batch_clear(qs_batch* b, void* stream) {
