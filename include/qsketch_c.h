@@ -192,8 +192,12 @@ qs_status qs_query(qs_sketch *sk, const uint32_t *d_keys, size_t n, uint32_t *d_
  * one, floored at 0.  A removal of a key that was never inserted lowers the estimates of the
  * keys sharing its counters (as in any count-min with deletions); and for MSWS, one whose
  * earlier occurrences were counted in the low level before its bucket linked lowers the high
- * counters instead.  Contended counters are updated by compare-and-swap loops bounded to
- * 2^22 tries (QS_ERR_TIMEOUT if one gives up). */
+ * counters instead.  u32 counters lose their removals in one atomic subtraction each (what it
+ * takes too much goes back) while no counter can hold 2^31: fewer than 2^29 keys inserted since
+ * create or clear.  Beyond that, in a sketch loaded from a snapshot or one whose inserts or clears
+ * were ever captured into a CUDA graph (their replays are not counted), in a captured qs_remove,
+ * and for the 8-bit counters they are updated by compare-and-swap loops bounded to 2^22 tries
+ * (QS_ERR_TIMEOUT if one gives up). */
 qs_status qs_remove(qs_sketch *sk, const uint32_t *d_keys, size_t n, void *stream);
 
 /* Host-buffer variants: keys / counts in host memory (pinned or pageable).  The copies

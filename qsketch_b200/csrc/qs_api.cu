@@ -97,6 +97,8 @@ struct qs_sketch {
     uint64_t max_batch = 0;
     uint64_t seen = 0;        // keys inserted since create / clear, or SEEN_UNKNOWN: bounds every
                               // u32 counter (a key adds at most 4 to one, see high_increments)
+    bool recorded = false;    // an insert or a clear was captured into a graph: its replays are not
+                              // counted in `seen`, which stays SEEN_UNKNOWN from then on
     bool arena = false;       // the tables of a batch
     uint64_t fresh = 0;       // keys inserted since create / clear (drives the chunk-size ramp)
     uint64_t ramp_first = 0;  // first chunk of the ramp, 0 = no ramp
@@ -229,9 +231,25 @@ qs_status ctl_reset(qs_sketch* sk, cudaStream_t st) {
     return QS_OK;
 }
 
+// Whether work issued to `st` goes into a graph that the caller is recording (unknown: as if it did).
+bool is_captured(cudaStream_t st) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return c != cudaStreamCaptureStatusNone;
+}
+
+// n more keys, or none left (cleared), in every counter of the sketch.
+void count_seen(qs_sketch* sk, uint64_t n, bool cleared, cudaStream_t st) {
+    sk->recorded |= is_captured(st);
+    sk->seen = sk->recorded || sk->arena ? SEEN_UNKNOWN : cleared ? 0 : std::min(sk->seen + n, SEEN_UNKNOWN);
+}
+
 // Clears an MSWS sketch (or a batch's arena and its per-stream state).
 qs_status clear_msws(qs_sketch* sk, const BatchDev& B, cudaStream_t st) {
-    sk->seen = sk->arena ? SEEN_UNKNOWN : 0;
+    count_seen(sk, 0, true, st);
     sk->fresh = 0;
     CK(msws_clear(sk->D, ctl_init(), B, sk->L.num_sms, st), "clear");
     return QS_OK;
@@ -268,7 +286,7 @@ uint64_t part_chunk(const qs_sketch* sk, uint64_t rest) {
 // replay.
 qs_status insert_device(qs_sketch* sk, const uint32_t* d_keys, size_t n, cudaStream_t st,
                         const uint32_t* skip = nullptr, const TableDev* table = nullptr, uint32_t* skipbuf = nullptr) {
-    sk->seen = std::min(sk->seen + n, SEEN_UNKNOWN);
+    count_seen(sk, n, false, st);
     if (sk->kind == QS_KIND_MSWS) {
         if (n <= SMALL_STREAM && !sk->own_knobs && !skip && !table) {
             CK(sk->prof_begin(0, st), "profile");
@@ -705,7 +723,8 @@ qs_status qs_remove(qs_sketch* sk, const uint32_t* d_keys, size_t n, void* strea
     if ((reinterpret_cast<uintptr_t>(d_keys) & 3u) != 0) return fail(QS_ERR_INVALID_ARG, "keys not 4-byte aligned");
     DeviceGuard guard(sk->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool low = sk->seen < (1ull << 29) && n < (1ull << 31);
+    // (a captured call may be replayed when the sketch holds any number of keys)
+    const bool low = sk->seen < (1ull << 29) && n < (1ull << 31) && !is_captured(st);
     if (sk->kind == QS_KIND_MSWS)
         CK(msws_remove(d_keys, n, sk->D, sk->L, low, st), "msws remove");
     else
@@ -777,7 +796,7 @@ qs_status qs_clear(qs_sketch* sk, void* stream) {
     DeviceGuard guard(sk->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (sk->kind == QS_KIND_MSWS) return clear_msws(sk, BatchDev{}, st);
-    sk->seen = 0;
+    count_seen(sk, 0, true, st);
     CK(cudaMemsetAsync(sk->C.table, 0, sk->C.n * sk->C.rows * 4, st), "clear table");
     return QS_OK;
 }
