@@ -201,8 +201,9 @@ qs_status qs_query(qs_sketch *sk, const uint32_t *d_keys, size_t n, uint32_t *d_
 qs_status qs_remove(qs_sketch *sk, const uint32_t *d_keys, size_t n, void *stream);
 
 /* Host-buffer variants: keys / counts in host memory (pinned or pageable).  The copies
- * run chunked and overlapped with the kernels on internal streams; the call returns
- * when the results are in h_counts (query) or the keys are consumed (insert). */
+ * run chunked and overlapped with the kernels on internal streams, which wait for the sketch's
+ * device calls issued before; the call returns when the results are in h_counts (query) or
+ * the keys are consumed (insert). */
 qs_status qs_insert_host(qs_sketch *sk, const uint32_t *h_keys, size_t n);
 qs_status qs_query_host(qs_sketch *sk, const uint32_t *h_keys, size_t n, uint32_t *h_counts);
 

@@ -117,7 +117,8 @@ struct qs_sketch {
     int cm_grid = 0;
     // host-buffer pipeline
     cudaStream_t io[2] = {nullptr, nullptr};
-    cudaEvent_t done = nullptr;
+    cudaEvent_t done = nullptr;    // the last slice inserted
+    cudaEvent_t issued = nullptr;  // the last device call
     uint32_t* stage_keys[2] = {nullptr, nullptr};
     uint32_t* stage_out[2] = {nullptr, nullptr};
     uint64_t stage_n = 0;
@@ -255,6 +256,13 @@ qs_status clear_msws(qs_sketch* sk, const BatchDev& B, cudaStream_t st) {
     return QS_OK;
 }
 
+// A device call was issued to `st`: the host-buffer calls, whose streams are their own, wait for it.
+// (Captured work runs when its graph is launched; ordering that is the caller's.)
+qs_status mark_issued(qs_sketch* sk, cudaStream_t st) {
+    if (sk->issued && !is_captured(st)) CK(cudaEventRecord(sk->issued, st), "record call");
+    return QS_OK;
+}
+
 qs_status setup_io(qs_sketch* sk) {
     if (sk->io[0]) return QS_OK;
     sk->stage_n = std::min<uint64_t>(sk->max_batch, 1ull << 22);
@@ -264,6 +272,8 @@ qs_status setup_io(qs_sketch* sk) {
         CK(sk->alloc(&sk->stage_out[i], sk->stage_n), "staging counts");
     }
     CK(cudaEventCreateWithFlags(&sk->done, cudaEventDisableTiming), "io event");
+    CK(cudaEventCreateWithFlags(&sk->issued, cudaEventDisableTiming), "io event");
+    CK(cudaDeviceSynchronize(), "io setup");  // earlier calls recorded no event
     return QS_OK;
 }
 
@@ -695,6 +705,7 @@ qs_status qs_destroy(qs_sketch* sk) {
                 cudaStreamDestroy(sk->io[i]);
             }
         if (sk->done) cudaEventDestroy(sk->done);
+        if (sk->issued) cudaEventDestroy(sk->issued);
         for (auto& v : sk->ev)
             for (auto& pr : v) {
                 cudaEventDestroy(pr.first);
@@ -713,7 +724,8 @@ qs_status qs_insert(qs_sketch* sk, const uint32_t* d_keys, size_t n, void* strea
     if (!d_keys) return fail(QS_ERR_INVALID_ARG, "null keys");
     if ((reinterpret_cast<uintptr_t>(d_keys) & 3u) != 0) return fail(QS_ERR_INVALID_ARG, "keys not 4-byte aligned");
     DeviceGuard guard(sk->device);
-    return insert_device(sk, d_keys, n, static_cast<cudaStream_t>(stream));
+    const qs_status s = insert_device(sk, d_keys, n, static_cast<cudaStream_t>(stream));
+    return s != QS_OK ? s : mark_issued(sk, static_cast<cudaStream_t>(stream));
 }
 
 qs_status qs_remove(qs_sketch* sk, const uint32_t* d_keys, size_t n, void* stream) {
@@ -729,7 +741,7 @@ qs_status qs_remove(qs_sketch* sk, const uint32_t* d_keys, size_t n, void* strea
         CK(msws_remove(d_keys, n, sk->D, sk->L, low, st), "msws remove");
     else
         CK(cm_remove(d_keys, n, sk->C, sk->cm_grid, low, sk->D.ctl ? &sk->D.ctl->status : nullptr, st), "cm remove");
-    return QS_OK;
+    return mark_issued(sk, st);
 }
 
 qs_status qs_query(qs_sketch* sk, const uint32_t* d_keys, size_t n, uint32_t* d_counts, void* stream) {
@@ -739,7 +751,8 @@ qs_status qs_query(qs_sketch* sk, const uint32_t* d_keys, size_t n, uint32_t* d_
     if (((reinterpret_cast<uintptr_t>(d_keys) | reinterpret_cast<uintptr_t>(d_counts)) & 3u) != 0)
         return fail(QS_ERR_INVALID_ARG, "keys/counts not 4-byte aligned");
     DeviceGuard guard(sk->device);
-    return query_device(sk, d_keys, n, d_counts, static_cast<cudaStream_t>(stream));
+    const qs_status s = query_device(sk, d_keys, n, d_counts, static_cast<cudaStream_t>(stream));
+    return s != QS_OK ? s : mark_issued(sk, static_cast<cudaStream_t>(stream));
 }
 
 qs_status qs_insert_host(qs_sketch* sk, const uint32_t* h_keys, size_t n) {
@@ -758,7 +771,7 @@ qs_status qs_insert_host(qs_sketch* sk, const uint32_t* h_keys, size_t n) {
         const int b = (int)(c & 1);
         const uint64_t len = std::min<uint64_t>(sk->stage_n, n - off);
         CK(cudaMemcpyAsync(sk->stage_keys[b], h_keys + off, len * 4, cudaMemcpyHostToDevice, sk->io[b]), "H2D keys");
-        if (!first) CK(cudaStreamWaitEvent(sk->io[b], sk->done, 0), "order inserts");
+        CK(cudaStreamWaitEvent(sk->io[b], first ? sk->issued : sk->done, 0), "order inserts");
         s = insert_device(sk, sk->stage_keys[b], len, sk->io[b]);
         if (s != QS_OK) return s;
         CK(cudaEventRecord(sk->done, sk->io[b]), "record insert");
@@ -782,6 +795,7 @@ qs_status qs_query_host(qs_sketch* sk, const uint32_t* h_keys, size_t n, uint32_
         const int b = (int)(c & 1);
         const uint64_t len = std::min<uint64_t>(sk->stage_n, n - off);
         CK(cudaMemcpyAsync(sk->stage_keys[b], h_keys + off, len * 4, cudaMemcpyHostToDevice, sk->io[b]), "H2D keys");
+        if (c < 2) CK(cudaStreamWaitEvent(sk->io[b], sk->issued, 0), "order queries");
         s = query_device(sk, sk->stage_keys[b], len, sk->stage_out[b], sk->io[b]);
         if (s != QS_OK) return s;
         CK(cudaMemcpyAsync(h_counts + off, sk->stage_out[b], len * 4, cudaMemcpyDeviceToHost, sk->io[b]), "D2H counts");
@@ -795,10 +809,13 @@ qs_status qs_clear(qs_sketch* sk, void* stream) {
     if (!sk) return fail(QS_ERR_INVALID_ARG, "null sketch");
     DeviceGuard guard(sk->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (sk->kind == QS_KIND_MSWS) return clear_msws(sk, BatchDev{}, st);
+    if (sk->kind == QS_KIND_MSWS) {
+        const qs_status s = clear_msws(sk, BatchDev{}, st);
+        return s != QS_OK ? s : mark_issued(sk, st);
+    }
     count_seen(sk, 0, true, st);
     CK(cudaMemsetAsync(sk->C.table, 0, sk->C.n * sk->C.rows * 4, st), "clear table");
-    return QS_OK;
+    return mark_issued(sk, st);
 }
 
 qs_status qs_sync(qs_sketch* sk, void* stream) {
