@@ -110,7 +110,8 @@ struct qs_sketch {
     MswsLaunch L{};
     PartDev P{};              // partitioned insert: its scratch (P.parts == 0: not used)
     PartLaunch PL{};
-    bool own_knobs = false;   // the caller fixed a pass-1 knob: its calls go through pass 1
+    bool own_knobs = false;   // the caller fixed a pass-1 knob: its calls go through pass 1 (a batch's
+                              // arena: see the batch's own)
     uint64_t part_cap = 0;    // keys a partitioned chunk takes
     uint64_t part_min = 0;    // and the fewest it pays for
     CmDev C{};
@@ -547,7 +548,7 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, bool pa
         // the partitioned insert (qs_part.cu) takes the large chunks of a sketch whose pass-1
         // knobs are left to the library
         const bool own_knobs = p.lanes_per_key || p.aggregate || p.route || p.ctas_per_sm || p.keys_per_tile ||
-                               (p.flags & QS_FLAG_NO_CHUNK_RAMP);
+                               p.first_chunk || (p.flags & QS_FLAG_NO_CHUNK_RAMP);
         sk->own_knobs = own_knobs;
         PartDev& P = sk->P;
         P.shift = PART_MIN_SHIFT;
@@ -1797,6 +1798,7 @@ struct qs_batch {
     // grouped by size class floor(log2 n_low) (the grouped order lives in B.cls_streams).
     std::vector<uint32_t> grp_class;   // size class of each grouped position
     // partitioned insert of the streams with enough keys (batch_dense)
+    bool own_knobs = false;            // the caller fixed a pass-1 knob: every stream goes through pass 1
     std::vector<uint32_t> part_off;    // [S + 1] prefix of the streams' partitions (empty: not used)
     std::vector<uint32_t> n_low;       // [S]
     PartDev P{};
@@ -1823,7 +1825,7 @@ BatchWindow flat_window(uint64_t c0, uint64_t c1) {
 // The window of an insert graph: its short slices a block each, unless the caller fixed pass-1 knobs.
 BatchWindow graph_window(const qs_batch* b, uint64_t max_total) {
     BatchWindow W = flat_window(0, max_total);
-    if (!b->sk->own_knobs) W.which = STREAMS_LONG;
+    if (!b->own_knobs) W.which = STREAMS_LONG;
     return W;
 }
 
@@ -2041,9 +2043,9 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
     ap.lanes_per_key = p->lanes_per_key;
     ap.ctas_per_sm = p->ctas_per_sm;
     qs_batch* b = new qs_batch();
-    const bool own_knobs = p->lanes_per_key || p->aggregate || p->route || p->ctas_per_sm || p->class_lanes_per_key ||
-                           p->first_chunk || (p->flags & QS_FLAG_NO_CHUNK_RAMP);
-    bool part = !own_knobs && th < (1ull << 28) && p->hash_mask_table_sz <= PART_MAX_MASKS;
+    b->own_knobs = p->lanes_per_key || p->aggregate || p->route || p->ctas_per_sm || p->class_lanes_per_key ||
+                   p->first_chunk || (p->flags & QS_FLAG_NO_CHUNK_RAMP);
+    bool part = !b->own_knobs && th < (1ull << 28) && p->hash_mask_table_sz <= PART_MAX_MASKS;
     qs_status s = create_sketch(&ap, &b->sk, part);
     if (s != QS_OK) {
         delete b;
