@@ -401,7 +401,9 @@ qs_status qs_mlp_train(qs_learned *lk, const uint32_t *d_keys, const uint8_t *d_
  * chunk size is then not searched, and the sample is inserted in chunks of that size.  The
  * fastest setting is returned in *best, recorded in a process-wide
  * table for the size class floor(log2(n_low)) of `base`, and used by later qs_create calls
- * of that class whose knobs are all 0.  h_all (may be null) receives up to max_all of the
+ * of that class whose knobs are all 0: in their calls that go through pass 1.  The partitioned
+ * and one-block inserts have no knobs and are not timed; a tuned max_batch below 2^22 leaves
+ * their chunks at the default's, one above widens them.  h_all (may be null) receives up to max_all of the
  * timed settings, *n_all how many were timed. */
 typedef struct qs_tune_config {
     uint32_t lanes_per_key, aggregate, route, ctas_per_sm;

@@ -5,7 +5,8 @@ device_sketch_v3.h:587).  Pass-1 knobs — lanes per key (1, 2, 4, 8, 16, 32 ove
 bucket), duplicate-key aggregation, level routing, CTAs per SM and the chunk size — never
 change results, only speed; qs_autotune times them on a sample and records the fastest for
 the sketch's size class floor(log2(n_low)), which later sketches of that class use when
-their knobs are left at 0.
+their knobs are left at 0, for the calls that go through pass 1 (large calls are partitioned and
+the smallest run in one block; neither has knobs).
 """
 import ctypes
 

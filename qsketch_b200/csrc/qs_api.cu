@@ -554,13 +554,16 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, bool pa
         P.shift = PART_MIN_SHIFT;
         while (P.shift < PART_MAX_SHIFT && (n_low >> P.shift) >= 640) ++P.shift;
         const uint64_t parts = (n_low + (1ull << P.shift) - 1) >> P.shift;
-        if (!own_knobs && B >= PART_TILE && parts >= 8 && parts <= PART_MAX_PARTS && H <= PART_MAX_MASKS &&
+        // The tuner times pass 1 alone: a chunk size that it picked below the default's must not cut
+        // the partitioned chunks, each of which streams the whole table (one above widens them).
+        const uint64_t PB = p.max_batch ? B : std::max<uint64_t>(B, 1ull << 22);
+        if (!own_knobs && PB >= PART_TILE && parts >= 8 && parts <= PART_MAX_PARTS && H <= PART_MAX_MASKS &&
             p.n_high < (1ull << 28))
             P.parts = (uint32_t)parts;
         // scratch words per chunk: the replay's records and their positions (24 B a key of B), or a
         // partitioned chunk's entries and key indices (6 B a key); every partitioned chunk or
         // window of this sketch, or of the batch whose arena it is, goes by part_cap
-        sk->part_cap = std::min<uint64_t>(B * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE;
+        sk->part_cap = PB >= PART_TILE ? std::min<uint64_t>(PB * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE : 0;
         const uint64_t record_words = std::max(B * 6, (sk->part_cap * 6 + 3) / 4);
         // A partitioned chunk streams the whole table through shared memory (64 MB: 45 us), pass 1
         // touches the buckets of its keys only.  Per call, measured: 2^18 Zipf 1.1 keys into a 4 MB
@@ -2057,8 +2060,8 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
         return st;
     };
     qs_sketch* sk = b->sk;
-    // max_batch 0 takes the tuner's, so only the arena knows the windows its scratch was sized for
-    part = part && sk->max_batch >= PART_TILE;
+    // max_batch 0 takes the tuner's: only the arena knows the windows that its scratch was sized for
+    part = part && sk->part_cap;
     sk->arena = true;
     sk->seen = SEEN_UNKNOWN;  // the batch's inserts do not go through the arena sketch's
     DeviceGuard guard(sk->device);

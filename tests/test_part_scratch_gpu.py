@@ -51,3 +51,26 @@ def test_batch_windows_fit_the_scratch_of_a_tuned_chunk_size(gpu, tuned):
         low, high = b.stream_tables(s)
         assert np.array_equal(low, orc.low) and np.array_equal(high, orc.high)
     b.close()
+
+
+@pytest.mark.parametrize("max_batch", [4096, 1 << 20, 1 << 21])
+def test_a_tuned_chunk_size_does_not_cut_the_partitioned_chunks(gpu, tuned, max_batch):
+    def sketch():
+        return qs.Sketch_GPU_Sub_Warp_Level(65521, 8, 8192, 32, hash_seed=2654435769)
+    keys = [data.zipf_keys(n, 1 << 16, 1.1, seed=n, perm_seed=3) for n in (9000011, 1 << 22, 70001)]
+    plain = sketch()
+    tuned(65521, max_batch)
+    other = sketch()
+    for i, k in enumerate(keys):
+        for sk in (plain, other):
+            sk.insert(k)
+            if i < 2:
+                assert sk.profile()["repair_launches"] == 0
+    for i in range(2):
+        assert np.array_equal(plain.tables()[i], other.tables()[i])
+    plain.clear()
+    other.clear()
+    launches = [sk.profile()["insert_launches"] for sk in (plain, other)]
+    for sk in (plain, other):
+        sk.insert(keys[0])
+    assert plain.profile()["insert_launches"] - launches[0] == other.profile()["insert_launches"] - launches[1]
