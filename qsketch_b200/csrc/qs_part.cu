@@ -45,10 +45,9 @@ constexpr uint32_t ENT_MASK = (1u << ENT_MASK_BITS) - 1u;
 // ACC: the path takes pools of less than 2^28 buckets):
 //   ACC | a        linked; its high increments collect in row a of the block's accumulators
 //   ACC | NEW | a  the same for a bucket linked in this chunk, whose id is not known yet
-//   TEMP | row     linked in this chunk with no accumulator left: a row in global memory
-//                  (TEMP_NOROW: no row left either, counted again when the id is known)
+//   TEMP | row     linked in this chunk with no accumulator left: a row in global memory (from
+//                  long_cap on there is none: counted again when the id is known)
 constexpr uint32_t ACC = 0x20000000u, NEW = 0x10000000u, TEMP = 0x40000000u;
-constexpr uint32_t TEMP_NOROW = 0x7fffffffu;
 constexpr uint32_t ACC_WORDS = LOW_COUNTERS + 1;  // 28 counters and the keys of a NEW bucket
 // Accumulator rows of a block: the linked buckets of a partition, a few per cent of its buckets.
 __host__ __device__ constexpr uint32_t ap_accs(uint32_t shift) { return shift > 10 ? 80u : 192u; }
@@ -598,8 +597,8 @@ __device__ __forceinline__ void part_apply_entry(const MswsDev& D, const ApShare
     }
     uint32_t* hb;
     if (w7 & TEMP) {
-        if (w7 == TEMP_NOROW) return;
         const uint32_t r = w7 & ~TEMP;
+        if (r >= D.long_cap) return;
         hb = D.totals + (uint64_t)r * LOW_COUNTERS;
         atomicAdd(&D.sw[r].y, c);
     } else if (is_linked(D, w7)) {
@@ -676,7 +675,7 @@ __device__ __forceinline__ void open_row(const MswsDev& D, const ApShared& S, ui
     if (lane == 0) r = atomicAdd(&D.ctl->n_switch, 1u);
     r = __shfl_sync(0xffffffffu, r, 0);
     put_row(D, r, S.stream, b0 + lb, pos, n_after, H);
-    if (lane == 0) S.w7[lb] = r < D.long_cap ? (TEMP | r) : TEMP_NOROW;
+    if (lane == 0) S.w7[lb] = TEMP | r;
 }
 
 // Pre-chunk counter of lane i: the bucket's words minus the packed increments T (counter c in
@@ -889,12 +888,12 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
     return true;
 }
 
-template <bool WIDE, bool BATCH>
-__global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev Q, BatchDev B) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint32_t p = blockIdx.x, stream = 0;
-    if (BATCH) {  // block: partition `part0 + blockIdx.x` of all streams'
-        p += Q.part0;
+// The partition `p` (batch: of all streams') that a block works on.
+template <bool BATCH>
+__device__ __forceinline__ PartView part_of_block(const MswsDev& D, const PartDev& Q, const BatchDev& B, uint32_t& p,
+                                                  uint32_t& stream) {
+    stream = 0;
+    if (BATCH) {
         uint32_t lo = 0, hi = B.n_streams;  // part_off[lo] <= p < part_off[hi]
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -904,7 +903,14 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
         stream = lo;
         p -= __ldg(B.part_off + lo);
     }
-    const PartView V = part_view<BATCH>(D, Q, B, stream);
+    return part_view<BATCH>(D, Q, B, stream);
+}
+
+template <bool WIDE, bool BATCH>
+__global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev Q, BatchDev B) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint32_t p = BATCH ? Q.part0 + blockIdx.x : blockIdx.x, stream;
+    const PartView V = part_of_block<BATCH>(D, Q, B, p, stream);
     if (V.tiles == 0) return;
     ApShared S = ap_carve(smem, V.shift, D.n_masks);
     S.stream = stream;
@@ -1225,6 +1231,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
             if (lane == 0) r = atomicAdd(&s_row, 1u);
             r = __shfl_sync(0xffffffffu, r, 0);
             put_row(D, r, S.stream, (uint32_t)b0 + lb, id, S.acc[a * ACC_WORDS + LOW_COUNTERS], v);
+            if (lane == 0 && r >= D.long_cap) S.w7[lb] = TEMP | r;
         } else {
             if (v) atomicAdd(D.high + (uint64_t)(id - START) * HIGH_WORDS + lane, v);
             if (lane == 0) S.w7[lb] = id;
@@ -1250,8 +1257,101 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
 
 // ---- 3: high ids in the array order of the switching keys -----------------------------------
 
+// The id of a bucket that switched at position pos, ranked by spre and the switch bits (a batch:
+// within the stream, whose positions are contiguous, on its own allocator); ok: inside the pool.
+// Called by a whole warp.
 template <bool BATCH>
-__global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev Q, BatchDev B) {
+__device__ __forceinline__ uint32_t part_link_id(const MswsDev& D, const PartDev& Q, const BatchDev& B, const uint32_t* spre,
+                                                 uint32_t base, uint32_t stream, uint32_t pos, bool& ok) {
+    const uint32_t id = base + switch_rank(D, spre, pos);
+    if (!BATCH) {
+        ok = (uint64_t)(id - START) < D.n_high;
+        return id;
+    }
+    const uint32_t own = __ldcg(B.base_id + stream) + (id - base) - switch_rank(D, spre, __ldcg(B.item_off + stream) * Q.tile);
+    const uint32_t nh = __ldg(&B.desc[stream].n_high);
+    ok = (uint64_t)(own - START) < nh;
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(B.next_id + stream, (uint32_t)min((unsigned long long)own + 1ull, (unsigned long long)START + nh));
+        if (!ok) atomicOr(B.status + stream, ST_POOL_FULL);
+    }
+    return own + __ldg(&B.desc[stream].high_base);
+}
+
+// More buckets linked in the chunk than there are rows of counts: the others' index words still hold
+// their rows' numbers.  A block takes a partition, links its buckets of that kind and counts their
+// entries from the switches on again, all in one pass over the partition's entries.  (Bucket by
+// bucket, each by a warp over the partition's entries, 2^24 keys that link most of 2^19 uniform
+// buckets took 9.4 ms and 0.6 M buckets of equal keys 184 ms; so 0.93 and 5.1, the ranks of the ids.)
+template <bool BATCH>
+__device__ __forceinline__ void part_link_rest(const MswsDev& D, const PartDev& Q, const BatchDev& B, const uint32_t* spre,
+                                               uint32_t base, uint32_t parts) {
+    __shared__ uint32_t s_pos[1u << PART_MAX_SHIFT], s_id[1u << PART_MAX_SHIFT];  // by bucket; id 0: dropped
+    __shared__ uint16_t s_list[1u << PART_MAX_SHIFT];
+    __shared__ uint32_t s_n, s_first;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    bool full = false;  // a bucket found the pool exhausted
+    for (uint32_t q = blockIdx.x; q < parts; q += gridDim.x) {
+        uint32_t p = BATCH ? Q.part0 + q : q, stream;
+        const PartView V = part_of_block<BATCH>(D, Q, B, p, stream);
+        if (V.tiles == 0) continue;
+        const uint64_t b0 = V.low_base + ((uint64_t)p << V.shift);
+        const uint32_t nb = (uint32_t)umin64((uint64_t)1 << V.shift, V.fm.d - ((uint64_t)p << V.shift));
+        __syncthreads();
+        if (tid == 0) s_n = 0, s_first = NONE;
+        __syncthreads();
+        for (uint32_t i = tid; i < nb; i += AP_THREADS) {
+            const uint32_t w7 = __ldcg(D.low + (b0 + i) * LOW_WORDS + 7), r = w7 & ~TEMP;
+            uint32_t pos = NONE;
+            if (w7 < FLAG && (w7 & TEMP) && r >= D.long_cap) {
+                pos = __ldcg(&D.sw[r].x);
+                atomicMin(&s_first, pos);
+                s_list[atomicAdd(&s_n, 1u)] = (uint16_t)i;
+            }
+            s_pos[i] = pos;
+        }
+        __syncthreads();
+        const uint32_t n = s_n;
+        if (n == 0) continue;
+        for (uint32_t l = wid; l < n; l += AP_WARPS) {
+            const uint32_t i = s_list[l];
+            bool ok;
+            const uint32_t id = part_link_id<BATCH>(D, Q, B, spre, base, stream, s_pos[i], ok);
+            if (ok) {
+                link_bucket(D, (uint32_t)(b0 + i), id, true, 0u, 0u);
+            } else if (lane == 0) {
+                __stcg(D.low + (b0 + i) * LOW_WORDS + 7, SATURATED);
+                full = true;
+            }
+            if (lane == 0) s_id[i] = ok ? id : 0u;
+        }
+        __syncthreads();
+        const uint16_t* o0 = V.off + (uint64_t)p * V.stride - V.tile0;
+        constexpr uint32_t G = 8;  // lanes per run
+        uint32_t dropped = 0;
+        for (uint32_t t = s_first / Q.tile + tid / G; t < V.tile0 + V.tiles; t += AP_THREADS / G) {
+            const uint32_t e1 = t * Q.tile + __ldcg(o0 + V.stride + t);
+            for (uint32_t i = t * Q.tile + __ldcg(o0 + t) + (tid & (G - 1u)); i < e1; i += G) {
+                const uint32_t e = __ldcg(Q.ent + i), first = s_pos[e >> ENT_MASK_BITS];
+                if (first == NONE) continue;
+                const uint32_t pos = t * Q.tile + __ldcg(Q.idx + i), id = s_id[e >> ENT_MASK_BITS];
+                if (pos < first) continue;
+                if (id == 0u) {
+                    ++dropped;
+                    continue;
+                }
+                uint32_t* hb = D.high + (uint64_t)(id - START) * HIGH_WORDS;
+                const uint32_t wrap = D.compat_v3 && pos == first ? 7u : 31u;  // the switching key lands on bit % 8
+                for (uint32_t m = __ldg(D.masks + (e & ENT_MASK)); m; m &= m - 1) atomicAdd(hb + ((__ffs(m) - 1) & wrap), 1u);
+            }
+        }
+        if (dropped) atomicAdd(&D.ctl->dropped, (unsigned long long)dropped);
+    }
+    if (full) atomicOr(&D.ctl->status, ST_POOL_FULL);
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev Q, BatchDev B, uint32_t parts) {
     extern __shared__ __align__(16) uint32_t spre[];  // switches per SW_BLOCK positions, then their prefix
     Ctl* ctl = D.ctl;
     const uint32_t ns = __ldcg(&ctl->n_switch);
@@ -1265,65 +1365,16 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_link(MswsDev D, PartDev 
     for (uint32_t i = tid; i < nq; i += AP_THREADS) spre[i] = __ldcg(D.sw_cnt + i);
     __syncthreads();
     block_scan_smem(spre, nq);
-    for (uint32_t r = blockIdx.x * AP_WARPS + wid; r < ns; r += gridDim.x * AP_WARPS) {
-        const uint32_t b = __ldcg(D.flag_list + r);
+    const uint32_t rows = min(ns, D.long_cap);
+    for (uint32_t r = blockIdx.x * AP_WARPS + wid; r < rows; r += gridDim.x * AP_WARPS) {
         const uint2 w = __ldcg(D.sw + r);
-        uint32_t id = base + switch_rank(D, spre, w.x), st = 0;
-        bool ok = (uint64_t)(id - START) < D.n_high;
-        if (BATCH) {  // ranked within the stream (its positions are contiguous) on its own allocator
-            st = __ldcg(D.sw_base + r);
-            const uint32_t own = __ldcg(B.base_id + st) + (id - base) -
-                                 switch_rank(D, spre, __ldcg(B.item_off + st) * Q.tile);
-            const uint32_t nh = __ldg(&B.desc[st].n_high);
-            ok = (uint64_t)(own - START) < nh;
-            id = own + __ldg(&B.desc[st].high_base);
-            if (lane == 0) {
-                atomicMax(B.next_id + st, (uint32_t)min((unsigned long long)own + 1ull, (unsigned long long)START + nh));
-                if (!ok) atomicOr(B.status + st, ST_POOL_FULL);
-            }
-        }
-        uint32_t H = 0, n_after = w.y;
-        if (r < D.long_cap) {
-            if (lane < LOW_COUNTERS) H = __ldcg(D.totals + (uint64_t)r * LOW_COUNTERS + lane);
-        } else {
-            // no row was left: count the bucket's entries from the switch on again
-            const PartView V = part_view<BATCH>(D, Q, B, st);
-            const uint32_t part = (b - V.low_base) >> V.shift, lb = (b - V.low_base) & ((1u << V.shift) - 1u);
-            const uint16_t* o0 = V.off + (uint64_t)part * V.stride - V.tile0;
-            uint32_t keys = 0;
-            for (uint32_t t = w.x / Q.tile; t < V.tile0 + V.tiles; ++t) {
-                const uint32_t e1 = t * Q.tile + __ldcg(o0 + V.stride + t);
-                for (uint32_t i0 = t * Q.tile + __ldcg(o0 + t); i0 < e1; i0 += 32) {
-                    const uint32_t i = i0 + lane;
-                    uint32_t m = 0;
-                    bool first = false;
-                    if (i < e1) {
-                        const uint32_t e = __ldcg(Q.ent + i);
-                        if ((e >> ENT_MASK_BITS) == lb) {
-                            const uint32_t pos = t * Q.tile + __ldcg(Q.idx + i);
-                            if (pos >= w.x) m = __ldg(D.masks + (e & ENT_MASK));
-                            first = pos == w.x;
-                        }
-                    }
-                    keys += __popc(__ballot_sync(0xffffffffu, m != 0));
-                    if (!__any_sync(0xffffffffu, m != 0)) continue;
-                    H += group_counts(m);
-                    if (D.compat_v3) {  // the switching key lands on bit % 8
-                        const uint32_t fb = __ballot_sync(0xffffffffu, first);
-                        if (fb) {
-                            ReplayOut o;
-                            o.T = H;
-                            o.cur = o.P = 0;
-                            o.mL = __shfl_sync(0xffffffffu, m, __ffs(fb) - 1);
-                            H = high_increments(D, o);
-                        }
-                    }
-                }
-            }
-            n_after = keys;
-        }
-        link_bucket(D, b, id, ok, H, n_after);
+        const uint32_t stream = BATCH ? __ldcg(D.sw_base + r) : 0u, b = __ldcg(D.flag_list + r);
+        bool ok;
+        const uint32_t id = part_link_id<BATCH>(D, Q, B, spre, base, stream, w.x, ok);
+        const uint32_t H = lane < LOW_COUNTERS ? __ldcg(D.totals + (uint64_t)r * LOW_COUNTERS + lane) : 0u;
+        link_bucket(D, b, id, ok, H, w.y);
     }
+    if (ns > rows) part_link_rest<BATCH>(D, Q, B, spre, base, parts);
 }
 
 // ---- launchers ------------------------------------------------------------------------------
@@ -1403,8 +1454,9 @@ static cudaError_t part_steps(const uint32_t* d_keys, uint64_t n, const MswsDev&
     const cudaError_t e = cudaLaunchKernel(apply_fn(D.wide != 0, batch), dim3(blocks), dim3(AP_THREADS), args, L.apply_smem, st);
     if (e != cudaSuccess) return e;
     const uint64_t nq = ((uint64_t)Q.tiles * Q.tile + SW_BLOCK - 1) / SW_BLOCK;
+    void* largs[] = {(void*)&Dc, (void*)&Qc, (void*)&Bc, (void*)&blocks};
     return cudaLaunchKernel(batch ? (const void*)k_part_link<true> : (const void*)k_part_link<false>, dim3(L.num_sms),
-                            dim3(AP_THREADS), args, (size_t)nq * 4, st);
+                            dim3(AP_THREADS), largs, (size_t)nq * 4, st);
 }
 
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
