@@ -22,7 +22,8 @@
 // told from large: the caller knows how many keys were inserted (SIGNED); otherwise the
 // compare-and-swap loop stays.
 // What bounds it now: the two round trips to L2 per pair of distinct keys of a tile.  3 M keys of
-// a power law 130 ms -> 0.23 ms, 2 M uniform keys 0.139 -> 0.108, 30,000 keys 0.335 -> 0.057.
+// a power law (exponent 1) 130 ms -> 0.23 ms; 2^20 uniform keys out of 64 MB 74 us -> 53, out of 0.5 MB
+// 84 -> 88 (the compare-and-swaps of words that keys share); 1,000 keys 13 -> 10 us.
 #include "qs_device.cuh"
 #include "qs_kernels.h"
 
@@ -92,67 +93,98 @@ __device__ __forceinline__ bool sub_mask(uint32_t* base, uint32_t m, uint32_t c)
     return ok;
 }
 
-constexpr uint32_t RM_TILE = 2048, RM_SLOTS = 4096, RM_PROBES = 16;
+constexpr uint32_t RM_TILE = 2048, RM_BITS = 12, RM_SLOTS = 1u << RM_BITS, RM_PROBES = 16;
 constexpr uint32_t RM_EMPTY = 0xffffffffu;
+
+constexpr uint32_t RM_KPT = RM_TILE / RM_THREADS;
 
 struct RmTable {
     uint32_t key[RM_SLOTS], cnt[RM_SLOTS];
     uint32_t top;  // occurrences of the key that equals RM_EMPTY
 };
 
-// Tile by tile: equal keys merge in the table, then fn(keys, counts, how many) over the distinct
-// keys, RM_KEYS at a time, so that a thread waits one round trip for their loads (a key
-// that finds no slot within RM_PROBES goes to fn at once).
-template <class F>
-__device__ __forceinline__ void merged_tiles(const uint32_t* __restrict__ keys, uint64_t n, uint32_t tile, RmTable& T,
-                                             F fn) {
-    const uint32_t tid = threadIdx.x;
-    for (uint32_t i = tid; i < RM_SLOTS; i += RM_THREADS) T.key[i] = RM_EMPTY, T.cnt[i] = 0u;
+// Tile by tile: equal keys merge in the table, then fn(keys, counts) over the distinct keys, RM_KEYS
+// of a thread at a time, so that it waits one round trip for their loads (a key that finds no
+// slot within RM_PROBES is taken by itself).  The table has 2^bits slots, at least two per key of the
+// tile: small tiles clear and walk no more than they fill (walking all 4096 slots for 1,000 uniform
+// keys 18 us, so 10).  Who takes a distinct key:
+//   OWN   the thread that brought it first, from its registers: 2^18 uniform keys 23 -> 21 us
+//   else  the threads walk the slots, which spreads the distinct keys of skewed tiles evenly:
+//         full tiles, 2^21 keys of a power law 0.6 172 us against 203, uniform 98 against 113; and
+//         tables of a few buckets, 2^18 keys into 509 91 us against 98
+template <bool OWN, class F>
+__device__ __forceinline__ void merged_tiles(const uint32_t* __restrict__ keys, uint64_t n, uint32_t tile, uint32_t bits,
+                                             RmTable& T, F fn) {
+    const uint32_t tid = threadIdx.x, slots = 1u << bits;
+    for (uint32_t i = tid; i < slots; i += RM_THREADS) T.key[i] = RM_EMPTY, T.cnt[i] = 0u;
     if (tid == 0) T.top = 0u;
     for (uint64_t t0 = (uint64_t)blockIdx.x * tile; t0 < n; t0 += (uint64_t)gridDim.x * tile) {
         const uint64_t t1 = umin64(n, t0 + tile);
-        uint32_t k[RM_TILE / RM_THREADS];
+        uint32_t k[RM_KPT], slot[RM_KPT];  // slot: NONE another thread's, LONE without one
+        constexpr uint32_t NONE = 0xffffffffu, LONE = 0xfffffffeu;
 #pragma unroll
-        for (uint32_t j = 0; j < RM_TILE / RM_THREADS; ++j) {
+        for (uint32_t j = 0; j < RM_KPT; ++j) {
             const uint64_t i = t0 + j * RM_THREADS + tid;
             k[j] = i < t1 ? __ldcs(keys + i) : 0u;
+            slot[j] = NONE;
         }
         __syncthreads();
 #pragma unroll
-        for (uint32_t j = 0; j < RM_TILE / RM_THREADS; ++j) {
+        for (uint32_t j = 0; j < RM_KPT; ++j) {
             if (t0 + j * RM_THREADS + tid >= t1) break;
             if (k[j] == RM_EMPTY) {
                 atomicAdd(&T.top, 1u);
                 continue;
             }
-            const uint32_t h = k[j] * 0x9E3779B1u >> 20;
-            uint32_t q = 0;
-            for (; q < RM_PROBES; ++q) {
-                const uint32_t s = (h + q) & (RM_SLOTS - 1);
+            const uint32_t h = k[j] * 0x9E3779B1u >> (32u - bits);
+            slot[j] = LONE;
+            for (uint32_t q = 0; q < RM_PROBES; ++q) {
+                const uint32_t s = (h + q) & (slots - 1u);
                 uint32_t seen = reinterpret_cast<volatile uint32_t*>(T.key)[s];
                 if (seen == RM_EMPTY) seen = atomicCAS(T.key + s, RM_EMPTY, k[j]);
                 if (seen == RM_EMPTY || seen == k[j]) {
                     atomicAdd(T.cnt + s, 1u);
+                    slot[j] = OWN && seen == RM_EMPTY ? s : NONE;
                     break;
                 }
             }
-            if (q == RM_PROBES) {
+            if (!OWN && slot[j] == LONE) {
                 const uint32_t one[RM_KEYS] = {k[j]}, c[RM_KEYS] = {1u};
                 fn(one, c);
             }
         }
         __syncthreads();
-        for (uint32_t i0 = tid; i0 < RM_SLOTS; i0 += RM_KEYS * RM_THREADS) {
-            uint32_t key[RM_KEYS], c[RM_KEYS];
+        if (OWN) {
 #pragma unroll
-            for (int u = 0; u < RM_KEYS; ++u) {
-                const uint32_t i = i0 + u * RM_THREADS;
-                key[u] = T.key[i];
-                c[u] = key[u] == RM_EMPTY ? 0u : T.cnt[i];
-                T.key[i] = RM_EMPTY;
-                T.cnt[i] = 0u;
+            for (uint32_t j0 = 0; j0 < RM_KPT; j0 += RM_KEYS) {
+                if (t0 + j0 * RM_THREADS >= t1) break;  // uniform over the block
+                uint32_t key[RM_KEYS], c[RM_KEYS];
+#pragma unroll
+                for (int u = 0; u < RM_KEYS; ++u) {
+                    const uint32_t s = slot[j0 + u];
+                    key[u] = k[j0 + u];
+                    c[u] = s == NONE ? 0u : 1u;
+                    if (s < slots) {
+                        c[u] = T.cnt[s];
+                        T.key[s] = RM_EMPTY;
+                        T.cnt[s] = 0u;
+                    }
+                }
+                fn(key, c);
             }
-            fn(key, c);
+        } else {
+            for (uint32_t i0 = tid; i0 < slots; i0 += RM_KEYS * RM_THREADS) {
+                uint32_t key[RM_KEYS], c[RM_KEYS];
+#pragma unroll
+                for (int u = 0; u < RM_KEYS; ++u) {
+                    const uint32_t i = i0 + u * RM_THREADS;
+                    key[u] = T.key[i];
+                    c[u] = key[u] == RM_EMPTY ? 0u : T.cnt[i];
+                    T.key[i] = RM_EMPTY;
+                    T.cnt[i] = 0u;
+                }
+                fn(key, c);
+            }
         }
         if (tid == 0 && T.top) {
             const uint32_t one[RM_KEYS] = {RM_EMPTY}, c[RM_KEYS] = {T.top};
@@ -161,16 +193,21 @@ __device__ __forceinline__ void merged_tiles(const uint32_t* __restrict__ keys, 
         }
     }
 }
-static_assert(RM_SLOTS == 1u << 12, "12 hash bits");
-static_assert(RM_SLOTS % (RM_KEYS * RM_THREADS) == 0 && RM_TILE % RM_THREADS == 0, "whole rounds");
+static_assert(RM_SLOTS == 1u << RM_BITS && RM_SLOTS == 2 * RM_TILE, "two slots per key of a full tile");
+constexpr uint32_t RM_MIN_BITS = 9;
+static_assert((1u << RM_MIN_BITS) % (RM_KEYS * RM_THREADS) == 0 && RM_TILE % RM_THREADS == 0 && RM_KPT % RM_KEYS == 0, "whole rounds");
 
-template <bool SIGNED>
+// SERIAL: the words of an unlinked bucket one after the other, each loaded just before its
+// compare-and-swap, for tables whose words many keys in flight share (all words at once, with the
+// values the bucket was read with, mostly retry: 2^21 uniform keys, 16,381 buckets 234 us against
+// 174, 65,521 150 against 139; 131,071 125 against 134).
+template <bool SIGNED, bool OWN, bool SERIAL>
 __global__ void __launch_bounds__(RM_THREADS, 4) k_msws_remove(const uint32_t* __restrict__ keys, uint64_t n, uint32_t tile,
-                                                               MswsDev D) {
+                                                               uint32_t bits, MswsDev D) {
     __shared__ RmTable T;
     bool ok = true;
     uint32_t dropped = 0;
-    merged_tiles(keys, n, tile, T, [&](const uint32_t (&key)[RM_KEYS], const uint32_t (&c)[RM_KEYS]) {
+    merged_tiles<OWN>(keys, n, tile, bits, T, [&](const uint32_t (&key)[RM_KEYS], const uint32_t (&c)[RM_KEYS]) {
         uint32_t m[RM_KEYS];
         uint32_t* wp[RM_KEYS];
         uint4 lo[RM_KEYS], hi[RM_KEYS];
@@ -181,6 +218,45 @@ __global__ void __launch_bounds__(RM_THREADS, 4) k_msws_remove(const uint32_t* _
             m[u] = c[u] ? __ldg(D.masks + fast_mod(D.fm_mask, hv)) : 0u;
             lo[u] = c[u] ? __ldcg(reinterpret_cast<const uint4*>(wp[u])) : make_uint4(0, 0, 0, 0);
             hi[u] = c[u] ? __ldcg(reinterpret_cast<const uint4*>(wp[u]) + 1) : make_uint4(0, 0, 0, 0);
+        }
+        if (SERIAL) {
+            uint32_t left[RM_KEYS];  // the next selected word of each key at a time
+#pragma unroll
+            for (int u = 0; u < RM_KEYS; ++u) {
+                const uint32_t ptr = hi[u].w;
+                left[u] = ptr == SATURATED || (ptr > START && (uint64_t)(ptr - START) < D.n_high) ? 0u : m[u];
+            }
+            for (;;) {
+                uint32_t any = 0;
+#pragma unroll
+                for (int u = 0; u < RM_KEYS; ++u) any |= left[u];
+                if (!any) break;
+                uint32_t old[RM_KEYS], dec[RM_KEYS];
+                uint32_t* p[RM_KEYS];
+#pragma unroll
+                for (int u = 0; u < RM_KEYS; ++u) {
+                    dec[u] = 0;
+                    if (!left[u]) continue;
+                    const uint32_t i = (uint32_t)(__ffs(left[u]) - 1) >> 2, nib = (left[u] >> (4 * i)) & 0xfu;
+                    left[u] &= ~(0xfu << (4 * i));
+                    p[u] = wp[u] + i;
+                    dec[u] = expand_nibble(nib) * min(c[u], 255u);
+                    old[u] = __ldcg(p[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < RM_KEYS; ++u)
+                    if (dec[u]) ok &= sat_sub_bytes(p[u], old[u], dec[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < RM_KEYS; ++u) {
+                if (!c[u]) continue;
+                const uint32_t ptr = hi[u].w;
+                if (ptr == SATURATED)
+                    dropped += c[u];
+                else if (ptr > START && (uint64_t)(ptr - START) < D.n_high)
+                    ok &= sub_mask<SIGNED>(D.high + (uint64_t)(ptr - START) * HIGH_WORDS, m[u], c[u]);
+            }
+            return;
         }
         uint32_t prev[RM_KEYS][7];  // low level: the words' compare-and-swaps, all in flight
 #pragma unroll
@@ -219,11 +295,11 @@ __global__ void __launch_bounds__(RM_THREADS, 4) k_msws_remove(const uint32_t* _
 }
 
 template <bool SIGNED>
-__global__ void __launch_bounds__(RM_THREADS, 4) k_cm_remove(const uint32_t* __restrict__ keys, uint64_t n, uint32_t tile, CmDev D,
-                                                          uint32_t* __restrict__ status) {
+__global__ void __launch_bounds__(RM_THREADS, 4) k_cm_remove(const uint32_t* __restrict__ keys, uint64_t n, uint32_t tile,
+                                                          uint32_t bits, CmDev D, uint32_t* __restrict__ status) {
     __shared__ RmTable T;
     bool ok = true;
-    merged_tiles(keys, n, tile, T, [&](const uint32_t (&key)[RM_KEYS], const uint32_t (&c)[RM_KEYS]) {
+    merged_tiles<true>(keys, n, tile, bits, T, [&](const uint32_t (&key)[RM_KEYS], const uint32_t (&c)[RM_KEYS]) {
 #pragma unroll
         for (int u = 0; u < RM_KEYS; ++u) {
             if (!c[u]) continue;
@@ -253,16 +329,30 @@ static uint32_t rm_tile(uint64_t n, int blocks) {
     return (uint32_t)std::min<uint64_t>(RM_TILE, std::max<uint64_t>(RM_THREADS, even));
 }
 
+static uint32_t rm_bits(uint32_t tile) {
+    uint32_t bits = RM_MIN_BITS;
+    while ((1u << bits) < 2 * tile) ++bits;
+    return bits;
+}
+
 cudaError_t msws_remove(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const MswsLaunch& L, bool below_2_31,
                         cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const uint32_t tile = rm_tile(n, L.num_sms * 4);
+    uint32_t tile = rm_tile(n, L.num_sms * 4), bits = rm_bits(tile);
     const int grid = (int)std::min<uint64_t>((uint64_t)L.num_sms * 4, (n + tile - 1) / tile);
-    if (below_2_31)
-        k_msws_remove<true><<<grid, RM_THREADS, 0, st>>>(d_keys, n, tile, D);
-    else
-        k_msws_remove<false><<<grid, RM_THREADS, 0, st>>>(d_keys, n, tile, D);
-    return cudaGetLastError();
+    // below 4,096 buckets nearly all are linked by the time words are shared; walked slots beside
+    // SERIAL took 358 us where the 2^21 keys into 16,381 buckets take 174
+    const bool few = D.n_low < (1u << 12), serial = !few && D.n_low < 3u << 15;
+    const bool own = serial || (!few && tile <= RM_TILE / 2);
+    const void* fn = below_2_31 ? (serial ? (const void*)k_msws_remove<true, true, true>
+                                   : own  ? (const void*)k_msws_remove<true, true, false>
+                                          : (const void*)k_msws_remove<true, false, false>)
+                                : (serial ? (const void*)k_msws_remove<false, true, true>
+                                   : own  ? (const void*)k_msws_remove<false, true, false>
+                                          : (const void*)k_msws_remove<false, false, false>);
+    MswsDev Dc = D;
+    void* args[] = {(void*)&d_keys, (void*)&n, (void*)&tile, (void*)&bits, (void*)&Dc};
+    return cudaLaunchKernel(fn, dim3(grid), dim3(RM_THREADS), args, 0, st);
 }
 
 cudaError_t cm_remove(const uint32_t* d_keys, uint64_t n, const CmDev& D, int grid, bool below_2_31, uint32_t* d_status,
@@ -271,9 +361,9 @@ cudaError_t cm_remove(const uint32_t* d_keys, uint64_t n, const CmDev& D, int gr
     const uint32_t tile = rm_tile(n, grid / 2);  // grid: eight blocks an SM
     const int g = (int)std::min<uint64_t>((uint64_t)grid / 2, (n + tile - 1) / tile);
     if (below_2_31)
-        k_cm_remove<true><<<g, RM_THREADS, 0, st>>>(d_keys, n, tile, D, d_status);
+        k_cm_remove<true><<<g, RM_THREADS, 0, st>>>(d_keys, n, tile, rm_bits(tile), D, d_status);
     else
-        k_cm_remove<false><<<g, RM_THREADS, 0, st>>>(d_keys, n, tile, D, d_status);
+        k_cm_remove<false><<<g, RM_THREADS, 0, st>>>(d_keys, n, tile, rm_bits(tile), D, d_status);
     return cudaGetLastError();
 }
 
