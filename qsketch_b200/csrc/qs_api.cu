@@ -608,6 +608,17 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, bool pa
         CKB(sk->alloc(&D.sw_bits, (reach + 31) / 32), "alloc link order");
         CKB(sk->alloc(&D.sw_cnt, (reach + SW_BLOCK - 1) / SW_BLOCK), "alloc link order");
         CKB(cudaMemcpy(masks_d, sk->masks.data(), (size_t)H * 4, cudaMemcpyHostToDevice), "upload masks");
+        if (!D.wide) {
+            std::vector<uint32_t> codes(H);
+            for (uint32_t i = 0; i < H; ++i) {
+                const uint32_t m = sk->masks[i], m1 = m & (m - 1), m2 = m1 & (m1 - 1);
+                codes[i] = (uint32_t)(__builtin_ctz(m) | __builtin_ctz(m1) << 5 | __builtin_ctz(m2) << 10);
+            }
+            uint32_t* codes_d = nullptr;
+            CKB(sk->alloc(&codes_d, H), "alloc mask codes");
+            D.codes = codes_d;
+            CKB(cudaMemcpy(codes_d, codes.data(), (size_t)H * 4, cudaMemcpyHostToDevice), "upload mask codes");
+        }
         qs_status s = ctl_reset(sk, 0);
         if (s != QS_OK) return bail(s);
         CKB(cudaStreamSynchronize(0), "create sync");

@@ -74,6 +74,7 @@ struct MswsDev {
     uint32_t* low;           // n_low * 8 words
     uint32_t* high;          // n_high * 32 words
     const uint32_t* masks;   // n_masks mask words (bit i selects counter i)
+    const uint32_t* codes;   // masks of three counters: the counters' numbers, 5 bits each (!wide)
     Ctl* ctl;
     uint64_t n_low;
     uint64_t n_high;

@@ -1648,7 +1648,7 @@ __device__ __forceinline__ void high_counters(const MswsDev& D, uint32_t ptr, ui
 
 template <bool WIDE>
 __device__ __forceinline__ void stage_codes(const MswsDev& D, uint32_t* s_codes) {
-    for (uint32_t i = threadIdx.x; i < D.n_masks; i += blockDim.x) s_codes[i] = mask_code<WIDE>(__ldg(D.masks + i));
+    for (uint32_t i = threadIdx.x; i < D.n_masks; i += blockDim.x) s_codes[i] = __ldg(mask_codes<WIDE>(D) + i);
 }
 
 // K keys of a thread, all of one sketch: the low buckets of all of them first, then the high
@@ -2138,7 +2138,13 @@ cudaError_t msws_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, cons
     const int grid = (int)umin64((uint64_t)L.query_grid, std::max<uint64_t>(1ull, want));
     MswsDev Dc = D;
     void* args[] = {(void*)&d_keys, (void*)&n, (void*)&d_out, (void*)&Dc};
-    const void* fn = D.wide ? (const void*)k_msws_query<true> : (const void*)k_msws_query<false>;
+    // The mask form takes any mask.  It keeps twice the registers (72 against 36: all of a thread's
+    // loads in flight, on half the warps), which long queries of tables beyond the L2 gain from: 2^24
+    // uniform keys on 256 MB 271 us against 292, on 1 GB 374 / 420 (Zipf 1.1 189 / 203, 221 / 217);
+    // on 96 MB 167 / 180 and 188 / 184, on 64 MB 156 / 141 and 185 / 178; 2^22 keys on 256 MB 79 / 82
+    // and 61 / 52.
+    const bool masks = D.wide || (D.n_low >= (1u << 22) && n >= (1u << 23));
+    const void* fn = masks ? (const void*)k_msws_query<true> : (const void*)k_msws_query<false>;
     return launch_pdl(fn, dim3(grid), dim3(QRY_THREADS), (size_t)D.n_masks * 4, st, args, false);
 }
 

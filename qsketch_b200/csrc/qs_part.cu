@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
 struct ApShared {
     uint32_t* tab;             // [2^shift][8] the partition's buckets (word 7: flagged buckets by slot)
     uint32_t* w7;              // [2^shift] their index words
-    uint32_t* mk;              // [n_masks] mask_code
+    uint32_t* mk;              // [n_masks] mask_codes
     uint32_t* acc;             // [ap_accs][ACC_WORDS]
     uint32_t* accid;           // [ap_accs] a row's high id, or (NEW) its switch position
     uint16_t* accb;            // [ap_accs] and its bucket
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev
     __shared__ uint32_t s_wcnt[4096 / 32];  // records of each warp's 32 entries, then those before them
     __shared__ uint32_t s_rcnt[AP_WARPS][32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (uint32_t i = tid; i < D.n_masks; i += AP_THREADS) S.mk[i] = mask_code<WIDE>(__ldg(D.masks + i));  // the host's
+    for (uint32_t i = tid; i < D.n_masks; i += AP_THREADS) S.mk[i] = __ldg(mask_codes<WIDE>(D) + i);
     const uint32_t accs = ap_accs(V.shift);
     for (uint32_t i = tid; i < accs * ACC_WORDS; i += AP_THREADS) S.acc[i] = 0u;
     if (tid == 0) s_nflag = s_nrec = s_many = s_drop = s_rb = s_rk = s_nacc = s_new = 0;

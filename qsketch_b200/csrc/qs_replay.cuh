@@ -14,12 +14,11 @@ __device__ __forceinline__ bool is_linked(const MswsDev& D, uint32_t w7) {
 }
 
 // A mask table of three counters per mask (the default) is kept as the counters' numbers, 5 bits
-// each; any other (WIDE) as the masks.
+// each; any other (WIDE) as the masks.  Computed once, at create: recoding the table in every block of
+// a query cost 0.2 us of the 3.5 that 10,007 keys take.
 template <bool WIDE>
-__device__ __forceinline__ uint32_t mask_code(uint32_t m) {
-    if (WIDE) return m;
-    const uint32_t a = __ffs(m) - 1, m1 = m & (m - 1), b = __ffs(m1) - 1, c = __ffs(m1 & (m1 - 1)) - 1;
-    return a | b << 5 | c << 10;
+__device__ __forceinline__ const uint32_t* mask_codes(const MswsDev& D) {
+    return WIDE ? D.masks : D.codes;
 }
 template <bool WIDE>
 __device__ __forceinline__ uint32_t code_mask(uint32_t q) {
