@@ -11,7 +11,10 @@
 // What bounds it: a chunk's three dependent trips to L2 (index words, counter atomics, link), then
 // the replay where a bucket crossed.  1,000 keys, clear + insert + query 46 -> 25 us; 512 slices of
 // 1,000 keys, pass 1 + replay 118 us -> 37 us.  256 threads a block measured the same as 512.  The
-// limit of SMALL_STREAM keys: two chunks; beyond it pass 1 spreads the keys over more SMs.
+// limit of SMALL_STREAM keys: two chunks; beyond it pass 1 spreads the keys over more SMs.  Against pass 1
+// and the replay, cleared / warm, at 4,096 keys: Zipf 1.4 120 -> 51 / 34 -> 21 us, Zipf 1.1 69 -> 35 /
+// 34 -> 28, exponent 0.7 17 -> 21 / 34 -> 29, uniform 15 -> 21 / 15 -> 21 (3,000 keys: 15 -> 17).  One
+// chunk of 1,024 threads instead of two: uniform 18, but Zipf 1.4 64.
 #include "qs_kernels.h"
 #include "qs_replay.cuh"
 
