@@ -323,7 +323,7 @@ qs_status insert_device(qs_sketch* sk, const uint32_t* d_keys, size_t n, cudaStr
                     ++sk->launches[0];
                     hot = true;
                 }
-                CK(part_insert(d_keys + off, c, D, sk->P, sk->PL, hot, st), "partitioned insert");
+                CK(part_insert(d_keys + off, c, D, sk->P, sk->PL, hot ? 1 : sk->fresh ? 2 : 0, st), "partitioned insert");
                 CK(sk->prof_end(0, st), "profile");
                 sk->launches[0] += 2;  // three kernels, one timed interval
                 off += c;

@@ -139,8 +139,10 @@ constexpr uint32_t PART_MAX_PARTS = 2048, PART_MIN_SHIFT = 6, PART_MAX_SHIFT = 1
 constexpr uint32_t PART_MAX_MASKS = 2048;         // mask tables the apply step keeps in shared memory
 constexpr uint64_t PART_MAX_CHUNK = 1ull << 26;
 constexpr uint32_t PART_HOT = 2048;               // heavy keys of a call
-// Calls of at least this many keys are sampled for them (9-12 us a call with the lookups): 1.6M Zipf 1.1
-// keys 140 -> 59 us, Zipf 0.8 67 -> 65, uniform 36 -> 47; at 2^20 95 -> 61, 54 -> 63, 34 -> 43.
+// Calls of at least this many keys into a warm sketch are sampled for them by a kernel of its own
+// (9-12 us a call with the lookups): 1.6M Zipf 1.1 keys 140 -> 59 us, Zipf 0.8 67 -> 65, uniform 36 -> 47.
+// Shorter ones by each block of the split for itself: at 2^20 Zipf 1.1 the call's sample gave 95 -> 61
+// us and uniform 34 -> 43, the blocks' 107 -> 44 and 30 -> 32.
 constexpr uint64_t PART_HOT_MIN = 3ull << 19;
 
 // Batched streams: many per-stream MSWS sketches share one low-table arena and one high

@@ -54,10 +54,11 @@ struct PartLaunch {
 };
 cudaError_t part_configure(int num_sms, PartLaunch* L);
 size_t part_apply_smem(uint32_t shift, uint32_t n_masks);
-// The call's heavy keys (a sample of its n keys) into part.hot, for part_insert's `hot`.
+// The call's heavy keys (a sample of its n keys) into part.hot, for part_insert's `hot` = 1 (0: none are
+// counted in the split, 2: the blocks of the split sample their keys).
 cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cudaStream_t st);
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
-                        bool hot, cudaStream_t st);
+                        int hot, cudaStream_t st);
 // The same for a window of a batch: `tiles` tiles (small or large) of the streams W names, whose
 // partitions are [part_lo, part_hi) of all streams'; hot: the heavy keys that part_hot_batch left
 // for each stream (from its keys at `first` on) are counted in the split.

@@ -249,14 +249,57 @@ __global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restri
 
 // ---- 1: tiles ordered by partition ---------------------------------------------------------
 
-// HOT: keys of the call's hot table whose bucket is linked when the chunk begins are counted in
-// shared memory (high-level additions commute) and never become entries.
+enum { HOT_NONE = 0, HOT_CALL = 1, HOT_OWN = 2 };
+
+// The whole block: the keys seen at least `least` times among 1,024 of the tile's, PER of each thread
+// (the first `cnt` of the tile are there), into their sets of hkey[PART_HOT]; tmp: 2,048 words.
+template <int THREADS, int PER, int KPT>
+__device__ __forceinline__ void sample_hot(const uint32_t (&e)[KPT], uint32_t cnt, uint32_t least, uint32_t* tmp,
+                                           uint32_t* hkey) {
+    constexpr uint32_t SLOTS = 1024;
+    static_assert(THREADS * PER == SLOTS, "a slot per sample");
+    const uint32_t tid = threadIdx.x;
+    uint32_t *key = tmp, *num = tmp + SLOTS;
+    for (uint32_t i = tid; i < SLOTS; i += THREADS) key[i] = HOT_EMPTY, num[i] = 0u;
+    for (uint32_t i = tid; i < PART_HOT; i += THREADS) hkey[i] = HOT_EMPTY;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint32_t k = e[j];
+        if (4 * tid + j >= cnt || k == HOT_EMPTY) continue;
+        const uint32_t h = mix32(k);
+        for (uint32_t p = 0; p < 8; ++p) {
+            const uint32_t i = (h + p) & (SLOTS - 1);
+            uint32_t seen = reinterpret_cast<volatile uint32_t*>(key)[i];
+            if (seen == HOT_EMPTY) seen = atomicCAS(key + i, HOT_EMPTY, k);
+            if (seen == HOT_EMPTY || seen == k) {
+                atomicAdd(num + i, 1u);
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < SLOTS; i += THREADS) {
+        if (num[i] < least) continue;
+        const uint32_t s = 2 * hot_set(key[i]);
+        if (atomicCAS(hkey + s, HOT_EMPTY, key[i]) != HOT_EMPTY) atomicCAS(hkey + s + 1, HOT_EMPTY, key[i]);
+    }
+    __syncthreads();
+}
+
+// HOT: keys of a hot table whose bucket is linked when the chunk begins are counted in shared memory
+// (high-level additions commute) and never become entries.  HOT_CALL: the table that k_part_hot (or
+// k_part_hot_batch) left for the call.  HOT_OWN, for calls too short for a launch of its own: each
+// block samples its first tile and finds the keys of about 4,096 entries and more, which would
+// otherwise pass through one block of the apply step, unit after unit: warm sketches, 10^6 equal
+// keys 476 -> 26 us, Zipf 1.1 107 -> 44 (0.5 MB) and 127 -> 52 (8 MB), exponent 0.9 75 -> 50, uniform
+// 30 -> 32 (sampling 1,024 keys of the whole chunk in every block 34: its sectors are the same for all).
 // TABLE (learned split): keys of the exact table count there (D.tbl_keys, D.tbl_counts) and never
 // become entries; four lookups of a thread are in flight at a time, and the table's heavy keys are
 // counted in shared memory with the others.
 // Bound by the random 32-byte sectors of the table in L2 (1 MB table, 2^24 keys: 263 us against 92
 // without); 8,192-key tiles and whole-warp probing of every key took 302 us.
-template <int PT_THREADS, int KPT, bool HOT, bool BATCH, bool TABLE>
+template <int PT_THREADS, int KPT, int HOT, bool BATCH, bool TABLE>
 __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(const uint32_t* __restrict__ keys, uint64_t n, MswsDev D,
                                                               PartDev Q, BatchDev B) {
     constexpr uint32_t R = PT_THREADS * KPT, HOTS = BATCH ? BATCH_HOT : PART_HOT;
@@ -277,13 +320,14 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
     PartView V = part_view<false>(D, Q, B, 0);
     // Learned chunks skip the lookups while no hot key is linked or in the table (0.45 -> 0.44 ms a pass);
     // for plain ones the branch costs Zipf streams more (1 %) than it gives uniform ones.
-    bool any_hot = !TABLE;
+    bool any_hot = !TABLE && HOT != HOT_OWN;
     auto load_hot = [&] {  // the hot keys whose buckets are linked
         bool mine = false;
         const uint32_t* hot = BATCH ? B.hot + (uint64_t)stream * BATCH_HOT : Q.hot;
         if (BATCH) hot_mul = __ldcg(B.hot_mul + stream);
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
-            uint32_t key = __ldcg(hot + i), id = 0;
+            uint32_t key = HOT == HOT_OWN ? s_hkey[i] : __ldcg(hot + i), id = 0;
+            if (HOT == HOT_OWN && key == HOT_EMPTY) continue;
             const int ts = TABLE && key != HOT_EMPTY ? table_find(D.tbl_keys, D.tbl_slots, key) : -1;
             if (ts >= 0) {
                 id = IN_TABLE | (uint32_t)ts;
@@ -296,10 +340,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             s_hid[i] = id;
             mine |= key != HOT_EMPTY;
         }
-        if (TABLE) any_hot = __syncthreads_or(mine);
+        if (TABLE || HOT == HOT_OWN) any_hot = __syncthreads_or(mine);
     };
     auto flush_hot = [&] {  // their counts: one add per counter
         for (uint32_t i = tid; i < HOTS; i += PT_THREADS) {
+            if (HOT == HOT_OWN && s_hkey[i] == HOT_EMPTY) continue;
             const uint32_t c = s_hcnt[i];
             if (!c) continue;
             if (TABLE && (s_hid[i] & IN_TABLE)) {
@@ -311,7 +356,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
                 atomicAdd(hb + (__ffs(m) - 1), c);
         }
     };
-    if (HOT && !BATCH) load_hot();
+    if (HOT == HOT_CALL && !BATCH) load_hot();
     if (BATCH) stream = NONE;
     for (uint32_t t = blockIdx.x; t < Q.tiles; t += gridDim.x) {
         if (BATCH) {
@@ -355,6 +400,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
             }
         }
         __syncthreads();
+        if (HOT == HOT_OWN && t == blockIdx.x) {
+            // about a unit's worth of entries in the chunk, and no chance repetition
+            const uint32_t least = max(4u, (uint32_t)((4096ull << 10) / n));
+            sample_hot<PT_THREADS, 1024 / PT_THREADS>(e, cnt, least, s_ent, s_hkey);
+            load_hot();
+        }
         uint32_t live = 0;  // bit j: key j goes to the sketch
 #pragma unroll
         for (int j = 0; j < KPT; ++j) {
@@ -490,7 +541,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1024 / PT_THREADS) k_part_split(co
         }
         __syncthreads();
     }
-    if (HOT && (!BATCH || stream != NONE)) flush_hot();
+    if (HOT && (HOT == HOT_OWN ? any_hot : !BATCH || stream != NONE)) flush_hot();
 }
 
 // ---- 2: one partition per block ------------------------------------------------------------
@@ -1384,22 +1435,20 @@ static size_t split_smem(uint32_t tile, uint32_t parts, uint32_t hot) {
 }
 
 // Kernel and threads of a split by tile size.
-static const void* split_fn(uint32_t tile, bool hot, bool batch, bool table) {
+template <int HOT, bool BATCH, bool TABLE>
+static const void* split_of(bool small) {
+    return small ? (const void*)k_part_split<512, 4, HOT, BATCH, TABLE> : (const void*)k_part_split<1024, 16, HOT, BATCH, TABLE>;
+}
+static const void* split_fn(uint32_t tile, int hot, bool batch, bool table) {
     const bool small = tile == PART_TILE_SMALL;
+    if (batch) return hot ? split_of<HOT_CALL, true, false>(small) : split_of<HOT_NONE, true, false>(small);
     if (table)
-        return small ? (hot ? (const void*)k_part_split<512, 4, true, false, true>
-                            : (const void*)k_part_split<512, 4, false, false, true>)
-                     : (hot ? (const void*)k_part_split<1024, 16, true, false, true>
-                            : (const void*)k_part_split<1024, 16, false, false, true>);
-    if (batch)
-        return small ? (hot ? (const void*)k_part_split<512, 4, true, true, false>
-                            : (const void*)k_part_split<512, 4, false, true, false>)
-                     : (hot ? (const void*)k_part_split<1024, 16, true, true, false>
-                            : (const void*)k_part_split<1024, 16, false, true, false>);
-    return small ? (hot ? (const void*)k_part_split<512, 4, true, false, false>
-                        : (const void*)k_part_split<512, 4, false, false, false>)
-                 : (hot ? (const void*)k_part_split<1024, 16, true, false, false>
-                        : (const void*)k_part_split<1024, 16, false, false, false>);
+        return hot == HOT_OWN    ? split_of<HOT_OWN, false, true>(small)
+               : hot == HOT_CALL ? split_of<HOT_CALL, false, true>(small)
+                                 : split_of<HOT_NONE, false, true>(small);
+    return hot == HOT_OWN    ? split_of<HOT_OWN, false, false>(small)
+           : hot == HOT_CALL ? split_of<HOT_CALL, false, false>(small)
+                             : split_of<HOT_NONE, false, false>(small);
 }
 
 static const void* apply_fn(bool wide, bool batch) {
@@ -1420,7 +1469,8 @@ cudaError_t part_configure(int num_sms, PartLaunch* L) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
     for (int batch = 0; batch < 2; ++batch) {
-        for (int i = 0; i < 8; ++i) cap(split_fn(i & 1 ? PART_TILE : PART_TILE_SMALL, i & 2, batch != 0, i & 4), split_max);
+        for (int hot = 0; hot < 3; ++hot)
+            for (int i = 0; i < 4; ++i) cap(split_fn(i & 1 ? PART_TILE : PART_TILE_SMALL, hot, batch != 0, i & 2), split_max);
         for (int wide = 0; wide < 2; ++wide) cap(apply_fn(wide != 0, batch != 0), apply_max);
     }
     cap((const void*)k_part_link<false>, link_max);
@@ -1437,7 +1487,7 @@ cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cu
 
 // Split, apply and link of a chunk (or a batch's window) whose tiles Q names.
 static cudaError_t part_steps(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& Q, const BatchDev& B,
-                              const PartLaunch& L, bool hot, uint32_t blocks, cudaStream_t st) {
+                              const PartLaunch& L, int hot, uint32_t blocks, cudaStream_t st) {
     MswsDev Dc = D;
     PartDev Qc = Q;
     BatchDev Bc = B;
@@ -1460,7 +1510,7 @@ static cudaError_t part_steps(const uint32_t* d_keys, uint64_t n, const MswsDev&
 }
 
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
-                        bool hot, cudaStream_t st) {
+                        int hot, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     PartDev Q = part;
     // small tiles while large ones would leave more than half of the SMs idle
