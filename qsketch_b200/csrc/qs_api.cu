@@ -551,13 +551,12 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, bool pa
                                p.first_chunk || (p.flags & QS_FLAG_NO_CHUNK_RAMP);
         sk->own_knobs = own_knobs;
         PartDev& P = sk->P;
-        P.shift = PART_MIN_SHIFT;
-        while (P.shift < PART_MAX_SHIFT && (n_low >> P.shift) >= 640) ++P.shift;
+        P.shift = part_shift(n_low);
         const uint64_t parts = (n_low + (1ull << P.shift) - 1) >> P.shift;
         // The tuner times pass 1 alone: a chunk size that it picked below the default's must not cut
         // the partitioned chunks, each of which streams the whole table (one above widens them).
         const uint64_t PB = p.max_batch ? B : std::max<uint64_t>(B, 1ull << 22);
-        if (!own_knobs && PB >= PART_TILE && parts >= 8 && parts <= PART_MAX_PARTS && H <= PART_MAX_MASKS &&
+        if (!own_knobs && PB >= PART_TILE && parts >= PART_MIN_PARTS && parts <= PART_MAX_PARTS && H <= PART_MAX_MASKS &&
             p.n_high < (1ull << 28))
             P.parts = (uint32_t)parts;
         // scratch words per chunk: the replay's records and their positions (24 B a key of B), or a

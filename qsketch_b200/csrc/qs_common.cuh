@@ -135,7 +135,20 @@ constexpr uint32_t PART_TILE = 16384, PART_TILE_SMALL = 2048;
 // Chunks below this many keys (half a large tile per SM) take small tiles.  Uniform calls of 2^20 keys
 // 34 us with small tiles, 36 with large ones; 1.3M 42 / 36; 2.4M 83 / 65.
 constexpr uint64_t PART_SMALL_MAX = 74ull * PART_TILE;
-constexpr uint32_t PART_MAX_PARTS = 2048, PART_MIN_SHIFT = 6, PART_MAX_SHIFT = 11;
+constexpr uint32_t PART_MAX_PARTS = 2048, PART_MAX_SHIFT = 11;
+// Buckets of a partition, as a shift: 64, more while that makes 640 partitions, and down to 16 for small
+// tables while that makes fewer than 256, because a partition is one block's (2^24 uniform keys, warm:
+// 1,021 buckets in 16 partitions 1049 us, in 64 306; 2,039 527 -> 216; 4,093 332 -> 204; 8,191 306 -> 268;
+// but 16,381 in 512 instead of 256 314 -> 348).
+__host__ __device__ constexpr uint32_t part_shift(uint64_t n_low) {
+    uint32_t s = 4;
+    while (s < 6 && (n_low >> s) >= 256) ++s;
+    while (s < PART_MAX_SHIFT && (n_low >> s) >= 640) ++s;
+    return s;
+}
+// Tables of fewer partitions stay with pass 1: at 509 buckets 2^24 uniform keys 407 us through pass 1, 525
+// in 32 partitions (cleared 655 / 579; Zipf 1.4 417 / 155, cleared 854 / 297), 1980 in eight of 64 buckets.
+constexpr uint64_t PART_MIN_PARTS = 32;
 constexpr uint32_t PART_MAX_MASKS = 2048;         // mask tables the apply step keeps in shared memory
 constexpr uint64_t PART_MAX_CHUNK = 1ull << 26;
 constexpr uint32_t PART_HOT = 2048;               // heavy keys of a call
