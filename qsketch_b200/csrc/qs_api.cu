@@ -1812,7 +1812,8 @@ struct qs_batch {
     std::vector<uint32_t> grp_class;   // size class of each grouped position
     // partitioned insert of the streams with enough keys (batch_dense)
     bool own_knobs = false;            // the caller fixed a pass-1 knob: every stream goes through pass 1
-    std::vector<uint32_t> part_off;    // [S + 1] prefix of the streams' partitions (empty: not used)
+    std::vector<uint32_t> part_shift;  // [S] the streams' smallest partitions (empty: not used)
+    std::vector<uint32_t> parts;       // [S] and how many (0: not for the stream)
     std::vector<uint32_t> n_low;       // [S]
     PartDev P{};
     uint64_t run_cap = 0;              // run bounds a window can have
@@ -1883,57 +1884,66 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
     qs_sketch* sk = b->sk;
     BatchDev B = b->B;
     B.key_off = d_offsets;
-    // (2^14: 11.8 ms a pass over 512 streams, 2^16 11.2, 2^17 11.0)
-    const uint64_t first = std::min<uint64_t>(1ull << 17, sk->part_cap / 4);
+    // Rounds: each stream's first keys (2^14: 11.8 ms a pass over 512 streams, 2^16 11.2, 2^17 11.0), in
+    // tiles of 2048 keys (a heavy key's run of a tile stays within a unit), then the rest, with
+    // the heavy keys counted in the split.  A rest of at most `fold` keys goes with the first: it is not
+    // worth streaming the stream's table again.
+    const uint64_t first = std::min<uint64_t>(1ull << 17, sk->part_cap / 4), fold = first / 4;
+    auto cut = [&](uint64_t len, uint64_t rel, uint64_t tail) {  // as k_part_plan
+        return rel && len - std::min(len, rel) <= tail ? len : std::min(len, rel);
+    };
+    auto parts_of = [&](uint32_t i, uint64_t part) -> uint64_t {
+        return part ? batch_parts(batch_shift(b->part_shift[i], b->n_low[i], part), b->n_low[i]) : 0;
+    };
+    auto length = [&](uint32_t i) -> uint64_t { return dense[i] ? off[i + 1] - off[i] : 0; };
     // one window: the streams [s_lo, s_hi), each stream's keys [r0, r1)
-    auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1, bool small,
-                   bool hot) -> qs_status {
-        const uint64_t tile = small ? PART_TILE_SMALL : PART_TILE;
-        uint64_t tiles = 0;
+    auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1, uint64_t tail, bool hot) -> qs_status {
+        const uint64_t tile = hot ? PART_TILE : PART_TILE_SMALL;
+        uint64_t tiles = 0, parts = 0;
         for (uint32_t i = s_lo; i < s_hi; ++i) {
-            const uint64_t len = dense[i] ? off[i + 1] - off[i] : 0;
-            tiles += (std::min(len, r1) - std::min(len, r0) + tile - 1) / tile;
+            const uint64_t part = cut(length(i), r1, tail) - cut(length(i), r0, tail);
+            tiles += (part + tile - 1) / tile;
+            parts += parts_of(i, part);
         }
         BatchWindow W{};
         W.s_lo = s_lo;
         W.s_hi = s_hi;
         W.rel_lo = r0;
         W.rel_hi = r1;
+        W.fold = tail;
         W.which = STREAMS_DENSE;
         CK(sk->prof_begin(0, st), "profile");
-        CK(part_insert_batch(d_keys, sk->D, b->P, B, sk->PL, W, (uint32_t)tiles, b->part_off[s_lo], b->part_off[s_hi],
-                             small, hot, st),
+        CK(part_insert_batch(d_keys, sk->D, b->P, B, sk->PL, W, (uint32_t)tiles, (uint32_t)parts, hot, st),
            "partitioned batch insert");
         CK(sk->prof_end(0, st), "profile");
         b->info.launches += 4;
         return QS_OK;
     };
+    uint64_t longest = 0;
+    for (uint32_t i = 0; i < b->S; ++i) longest = std::max(longest, length(i));
     for (int round = 0; round < 2; ++round) {
-        const uint64_t r0 = round ? first : 0, r1 = round ? ~0ull : first;
-        if (round) {
-            CK(part_hot_batch(d_keys, B, first, st), "heavy keys");
+        const bool hot = round != 0;
+        const uint64_t r0 = hot ? first : 0, r1 = hot ? ~0ull : first, tile = hot ? PART_TILE : PART_TILE_SMALL;
+        if (hot) {
+            if (longest <= first + fold) break;
+            CK(part_hot_batch(d_keys, B, first, fold, st), "heavy keys");
             ++b->info.launches;
         }
         uint64_t slots = 0, keys = 0, runs = 0;
         uint32_t lo = 0;
         auto close = [&](uint32_t hi) -> qs_status {
-            qs_status s = QS_OK;
-            // tiles of 2048 keys in the first round (a heavy key's run of a tile stays within a
-            // unit), and while larger ones would leave SMs idle
-            if (keys) s = run(lo, hi, r0, r1, !round, round != 0);
+            const qs_status s = keys ? run(lo, hi, r0, r1, fold, hot) : QS_OK;
             slots = keys = runs = 0;
             lo = hi;
             return s;
         };
-        const uint64_t tile = round ? PART_TILE : PART_TILE_SMALL;
         for (uint32_t i = 0; i < b->S; ++i) {
-            const uint64_t len = dense[i] ? off[i + 1] - off[i] : 0, part = std::min(len, r1) - std::min(len, r0);
-            const uint64_t parts = b->part_off[i + 1] - b->part_off[i];
-            if (part > sk->part_cap) {  // one stream's slice alone exceeds a window: split it
+            const uint64_t len = length(i), part = cut(len, r1, fold) - cut(len, r0, fold), parts = parts_of(i, part);
+            if (part > sk->part_cap) {  // one stream's rest alone exceeds a window: split it
                 qs_status s = close(i);
                 if (s != QS_OK) return s;
-                for (uint64_t a = r0; a < std::min(len, r1); a += sk->part_cap) {
-                    s = run(i, i + 1, a, std::min(std::min(len, r1), a + sk->part_cap), false, round != 0);
+                for (uint64_t a = r0; a < len; a += sk->part_cap) {
+                    s = run(i, i + 1, a, std::min(len, a + sk->part_cap), 0, hot);
                     if (s != QS_OK) return s;
                 }
                 lo = i + 1;
@@ -2093,9 +2103,11 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
         hb += p->n_high[i];
     }
     if (part) {
-        // 64 partitions of a stream's sketch where that leaves 16 buckets to each (several
-        // blocks then share even a small sketch's keys), 2048 buckets to each of a large one
-        b->part_off.assign(S + 1, 0);
+        // at most 64 partitions of a stream's sketch where that leaves 16 buckets to each (several
+        // blocks then share even a small sketch's keys), 2048 buckets to each of a large one;
+        // fewer where a window has few keys for it (batch_shift)
+        b->part_shift.resize(S);
+        b->parts.resize(S);
         b->n_low.resize(S);
         size_t smem = 0;
         for (uint32_t i = 0; i < S; ++i) {
@@ -2105,8 +2117,10 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
             desc[i].shift = sh;
             desc[i].parts = parts >= 4 && parts <= PART_MAX_PARTS ? (uint32_t)parts : 0u;
             b->n_low[i] = (uint32_t)p->n_low[i];
-            b->part_off[i + 1] = b->part_off[i] + desc[i].parts;
-            if (desc[i].parts) smem = std::max(smem, part_apply_smem(sh, p->hash_mask_table_sz));
+            b->part_shift[i] = sh;
+            b->parts[i] = desc[i].parts;
+            for (uint32_t x = sh; desc[i].parts && x <= batch_shift(sh, b->n_low[i], 0); ++x)  // (units halve with shift)
+                smem = std::max(smem, part_apply_smem(x, p->hash_mask_table_sz));
         }
         sk->PL.apply_smem = smem;
         b->P = sk->P;
@@ -2117,10 +2131,8 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
     BatchDev& B = b->B;
     B.n_streams = S;
     if (part) {
-        uint32_t* d_off = nullptr;
-        CKB(sk->alloc(&d_off, (uint64_t)S + 1), "alloc partitions");
-        CKB(cudaMemcpy(d_off, b->part_off.data(), ((size_t)S + 1) * 4, cudaMemcpyHostToDevice), "upload partitions");
-        B.part_off = d_off;
+        CKB(sk->alloc(&B.part_off, (uint64_t)S + 1), "alloc partitions");
+        CKB(sk->alloc(&B.part_shift, S), "alloc partitions");
         CKB(sk->alloc(&B.run_off, (uint64_t)S + 1), "alloc run prefix");
         CKB(sk->alloc(&B.base_id, S), "alloc allocators");
         CKB(sk->alloc(&B.hot, (uint64_t)S * BATCH_HOT), "alloc heavy keys");
@@ -2231,8 +2243,7 @@ qs_status qs_batch_insert(qs_batch* b, const uint32_t* d_keys, const uint64_t* d
     std::vector<char> dense(S, 0);
     bool any_dense = false, any_sparse = false;
     for (uint32_t i = 0; i < S; ++i) {
-        dense[i] = !b->part_off.empty() &&
-                   batch_dense(off[i + 1] - off[i], b->n_low[i], b->part_off[i + 1] - b->part_off[i]);
+        dense[i] = !b->parts.empty() && batch_dense(off[i + 1] - off[i], b->n_low[i], b->parts[i]);
         (dense[i] ? any_dense : any_sparse) = true;
     }
     if (any_dense) {

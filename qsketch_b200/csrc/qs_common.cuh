@@ -129,7 +129,6 @@ struct PartDev {
     uint32_t parts;
     uint32_t tiles;   // this chunk's tiles, of `tile` keys
     uint32_t tile;
-    uint32_t part0;   // batch: the window's first partition among all streams'
 };
 constexpr uint32_t PART_TILE = 16384, PART_TILE_SMALL = 2048;
 // Chunks below this many keys (half a large tile per SM) take small tiles.  Uniform calls of 2^20 keys
@@ -169,8 +168,8 @@ struct StreamDesc {
     uint32_t low_base;   // first bucket of the stream's sketch in the low arena
     uint32_t high_base;  // global high id = high_base + the stream's own id (from FIRST_ID)
     uint32_t n_high;     // the stream's pool size in buckets (own ids < START + n_high)
-    uint32_t shift;      // partitioned insert: 2^shift buckets to a partition
-    uint32_t parts;      // and the stream's partitions
+    uint32_t shift;      // partitioned insert: 2^shift buckets to the smallest partition
+    uint32_t parts;      // and the partitions then (0: not for this stream)
 };
 
 struct BatchDev {
@@ -190,7 +189,8 @@ struct BatchDev {
     unsigned long long* first;// [n_streams] (repair generation << 32) | ~(lowest rank of the
                               // stream's links in that repair): ranks within each stream
     // partitioned insert (its plan fills item_off with its own tiles)
-    const uint32_t* part_off; // [n_streams + 1] prefix of the streams' partitions
+    uint32_t* part_shift;     // [n_streams] buckets of a partition in this window (batch_shift)
+    uint32_t* part_off;       // [n_streams + 1] prefix of the streams' partitions in this window
     uint32_t* run_off;        // [n_streams + 1] prefix of the streams' run bounds in PartDev::off
     uint32_t* base_id;        // [n_streams] next_id when the window began
     uint32_t* hot;            // [n_streams][BATCH_HOT] heavy keys of each stream in this call
@@ -208,15 +208,30 @@ struct BatchWindow {
     uint64_t rel_lo, rel_hi;
     uint32_t s_lo, s_hi;
     uint32_t flat;
+    uint64_t fold;   // dense streams: one with at most this many keys from rel_hi on has them in the window
+                     // that ends at rel_hi, and none in the one that begins there
     uint32_t which;  // all streams, or only the dense or the sparse ones (batch_dense), or (flat)
                      // work items only for the slices of more than SMALL_STREAM keys
 };
 enum { STREAMS_ALL = 0, STREAMS_DENSE = 1, STREAMS_SPARSE = 2, STREAMS_LONG = 3 };
 // Keys of a stream in one call that one block takes by itself (k_msws_small).
 constexpr uint64_t SMALL_STREAM = 4096;
+// Buckets of a partition of such a stream, of `keys` keys in the window, as a shift: as many as it takes
+// for 2,048 keys to a partition, down to eight of them.  A block per partition is 20 to 30 ns of the
+// chip, whatever its keys: 512 streams of 33,000 keys, 1,024 to 8,192 buckets, cleared / warm, in 32 to 64
+// partitions each 0.89 / 0.96 ms uniform and 1.60 / 1.13 Zipf 1.2; so 0.54 / 0.58 and 1.51 / 0.71 (pass 1
+// 0.64 / 0.94 and 1.23 / 0.88).
+__host__ __device__ __forceinline__ uint32_t batch_shift(uint32_t shift, uint32_t n_low, uint64_t keys) {
+    while (shift < PART_MAX_SHIFT && (n_low >> shift) > 8 && (n_low >> shift) > (keys >> 11)) ++shift;
+    return shift;
+}
+__host__ __device__ __forceinline__ uint32_t batch_parts(uint32_t shift, uint32_t n_low) {
+    return (uint32_t)(((uint64_t)n_low + (1ull << shift) - 1) >> shift);
+}
 // Streams whose keys go through the partitioned insert: at least a key to a bucket and 2^15 keys in
 // the call.  The partitioned insert streams a sketch's table twice (about 46 ps a bucket) and takes
-// 20-30 ps a key; pass 1 and the replay take 66 ps a key.
+// 20-30 ps a key; pass 1 and the replay take 66 ps a key.  (From 1.5 keys a bucket on only: 64 streams of
+// 135,000 keys, up to 262,144 buckets, warm, 503 -> 489 us uniform, but 667 -> 682 at exponent 0.6.)
 __host__ __device__ __forceinline__ bool batch_dense(uint64_t keys, uint32_t n_low, uint32_t parts) {
     return parts && keys >= (1ull << 15) && keys >= n_low;
 }

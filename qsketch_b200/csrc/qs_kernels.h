@@ -59,13 +59,13 @@ size_t part_apply_smem(uint32_t shift, uint32_t n_masks);
 cudaError_t part_hot(const uint32_t* d_keys, uint64_t n, const PartDev& part, cudaStream_t st);
 cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, const PartDev& part, const PartLaunch& L,
                         int hot, cudaStream_t st);
-// The same for a window of a batch: `tiles` tiles (small or large) of the streams W names, whose
-// partitions are [part_lo, part_hi) of all streams'; hot: the heavy keys that part_hot_batch left
-// for each stream (from its keys at `first` on) are counted in the split.
-cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, cudaStream_t st);
+// The same for a window of a batch: `tiles` tiles of the streams W names, `parts` partitions in all; hot:
+// large tiles, and the heavy keys that part_hot_batch left for each stream (from its keys at
+// `first` on, where there are more than `fold`) are counted in the split; else small tiles.
+cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, uint64_t fold, cudaStream_t st);
 cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const PartDev& part, const BatchDev& B,
-                              const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t part_lo,
-                              uint32_t part_hi, bool small, bool hot, cudaStream_t st);
+                              const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t parts, bool hot,
+                              cudaStream_t st);
 
 cudaError_t cm_insert(const uint32_t* d_keys, uint64_t n, const CmDev& D, int agg, int grid, cudaStream_t st);
 // REMOVE (qs_remove.cu): one occurrence of each key out, counters floored at 0.  below_2_31: no u32

@@ -134,7 +134,7 @@ __device__ __forceinline__ PartView part_view(const MswsDev& D, const PartDev& Q
     const StreamDesc* sd = B.desc + s;
     V.fm = FastMod{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d)};
     V.seed = __ldg(&sd->seed), V.low_base = __ldg(&sd->low_base);
-    V.shift = __ldg(&sd->shift), V.parts = __ldg(&sd->parts);
+    V.shift = __ldcg(B.part_shift + s), V.parts = batch_parts(V.shift, V.fm.d);
     V.tile0 = __ldcg(B.item_off + s), V.tiles = __ldcg(B.item_off + s + 1) - V.tile0;
     V.off = Q.off + __ldcg(B.run_off + s), V.stride = V.tiles;
     return V;
@@ -147,17 +147,24 @@ __global__ void __launch_bounds__(1024) k_part_plan(BatchDev B, BatchWindow W, u
     for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
         const uint64_t o0 = __ldcg(B.key_off + s), len = __ldcg(B.key_off + s + 1) - o0;
         const bool in = s >= W.s_lo && s < W.s_hi && in_window(B, W, s, len);
-        const uint64_t lo = in ? o0 + umin64(W.rel_lo, len) : o0, hi = in ? o0 + umin64(W.rel_hi, len) : o0;
+        auto cut = [&](uint64_t rel) { return rel && len - umin64(rel, len) <= W.fold ? len : umin64(rel, len); };
+        const uint64_t lo = in ? o0 + cut(W.rel_lo) : o0, hi = in ? o0 + cut(W.rel_hi) : o0;
         const uint32_t t = (uint32_t)((hi - lo + tile - 1) / tile);
         B.lo[s] = lo;
         B.hi[s] = hi;
         B.item_off[s] = t;
-        B.run_off[s] = t * (B.desc[s].parts + 1u);
+        const uint32_t n_low = B.desc[s].fm_low.d, shift = batch_shift(B.desc[s].shift, n_low, hi - lo);
+        const uint32_t parts = t ? batch_parts(shift, n_low) : 0u;
+        B.part_shift[s] = shift;
+        B.part_off[s] = parts;
+        B.run_off[s] = t * (parts + 1u);
         B.base_id[s] = __ldcg(B.next_id + s);
     }
     __syncthreads();
     const uint32_t tiles = block_scan_array(B.item_off, S), runs = block_scan_array(B.run_off, S);
+    const uint32_t parts = block_scan_array(B.part_off, S);
     if (threadIdx.x == 0) {
+        B.part_off[S] = parts;
         B.item_off[S] = tiles;
         B.run_off[S] = runs;
         ctl->n_switch = 0;
@@ -172,12 +179,13 @@ static_assert(BATCH_HOT == 2 * 64, "batch_hot_set yields 6 bits, two keys per se
 // (short streams: none).  Sets are few, and a heavy key that finds its set full would go through
 // one block entry by entry (0.5 M of them, 0.9 ms), so each of the eight warps tries a multiplier
 // and the one that leaves the least weight out is kept with the stream.
-__global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restrict__ keys, BatchDev B, uint64_t first) {
+__global__ void __launch_bounds__(256) k_part_hot_batch(const uint32_t* __restrict__ keys, BatchDev B, uint64_t first,
+                                                        uint64_t fold) {
     constexpr uint32_t N = 4096, SLOTS = 4096, LIST = 512;
     __shared__ uint32_t s_key[SLOTS], s_cnt[SLOTS], s_hot[BATCH_HOT];
     const uint32_t tid = threadIdx.x, s = blockIdx.x;
     const uint64_t o0 = __ldcg(B.key_off + s), all = __ldcg(B.key_off + s + 1) - o0;
-    if (!batch_dense(all, B.desc[s].fm_low.d, B.desc[s].parts) || all <= first) return;
+    if (!batch_dense(all, B.desc[s].fm_low.d, B.desc[s].parts) || all <= first + fold) return;
     const uint64_t lo = o0 + first, len = all - first;
     for (uint32_t i = tid; i < BATCH_HOT; i += 256) s_hot[i] = HOT_EMPTY;
     if (len >= 8 * N) {
@@ -939,20 +947,20 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
     return true;
 }
 
-// The partition `p` (batch: of all streams') that a block works on.
+// The partition `p` (batch: of the window's) that a block works on.
 template <bool BATCH>
 __device__ __forceinline__ PartView part_of_block(const MswsDev& D, const PartDev& Q, const BatchDev& B, uint32_t& p,
                                                   uint32_t& stream) {
     stream = 0;
     if (BATCH) {
-        uint32_t lo = 0, hi = B.n_streams;  // part_off[lo] <= p < part_off[hi]
+        uint32_t lo = 0, hi = B.n_streams;  // part_off[lo] <= p < part_off[hi]: the last such lo has partitions
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(B.part_off + mid) <= p) lo = mid;
+            if (__ldcg(B.part_off + mid) <= p) lo = mid;
             else hi = mid;
         }
         stream = lo;
-        p -= __ldg(B.part_off + lo);
+        p -= __ldcg(B.part_off + lo);
     }
     return part_view<BATCH>(D, Q, B, stream);
 }
@@ -960,7 +968,7 @@ __device__ __forceinline__ PartView part_of_block(const MswsDev& D, const PartDe
 template <bool WIDE, bool BATCH>
 __global__ void __launch_bounds__(AP_THREADS, 2) k_part_apply(MswsDev D, PartDev Q, BatchDev B) {
     extern __shared__ __align__(128) uint8_t smem[];
-    uint32_t p = BATCH ? Q.part0 + blockIdx.x : blockIdx.x, stream;
+    uint32_t p = blockIdx.x, stream;
     const PartView V = part_of_block<BATCH>(D, Q, B, p, stream);
     if (V.tiles == 0) return;
     ApShared S = ap_carve(smem, V.shift, D.n_masks);
@@ -1343,7 +1351,7 @@ __device__ __forceinline__ void part_link_rest(const MswsDev& D, const PartDev& 
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     bool full = false;  // a bucket found the pool exhausted
     for (uint32_t q = blockIdx.x; q < parts; q += gridDim.x) {
-        uint32_t p = BATCH ? Q.part0 + q : q, stream;
+        uint32_t p = q, stream;
         const PartView V = part_of_block<BATCH>(D, Q, B, p, stream);
         if (V.tiles == 0) continue;
         const uint64_t b0 = V.low_base + ((uint64_t)p << V.shift);
@@ -1519,23 +1527,22 @@ cudaError_t part_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, co
     return part_steps(d_keys, n, D, Q, BatchDev{}, L, hot, Q.parts, st);
 }
 
-cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, cudaStream_t st) {
-    k_part_hot_batch<<<B.n_streams, 256, 0, st>>>(d_keys, B, first);
+cudaError_t part_hot_batch(const uint32_t* d_keys, const BatchDev& B, uint64_t first, uint64_t fold, cudaStream_t st) {
+    k_part_hot_batch<<<B.n_streams, 256, 0, st>>>(d_keys, B, first, fold);
     return cudaGetLastError();
 }
 
 cudaError_t part_insert_batch(const uint32_t* d_keys, const MswsDev& D, const PartDev& part, const BatchDev& B,
-                              const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t part_lo,
-                              uint32_t part_hi, bool small, bool hot, cudaStream_t st) {
+                              const PartLaunch& L, const BatchWindow& W, uint32_t tiles, uint32_t parts, bool hot,
+                              cudaStream_t st) {
     if (tiles == 0) return cudaSuccess;
     PartDev Q = part;
-    Q.tile = small ? PART_TILE_SMALL : PART_TILE;
+    Q.tile = hot ? PART_TILE : PART_TILE_SMALL;
     Q.tiles = tiles;
-    Q.part0 = part_lo;
     k_part_plan<<<1, 1024, 0, st>>>(B, W, Q.tile, D.ctl);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return part_steps(d_keys, 0, D, Q, B, L, hot, part_hi - part_lo, st);
+    return part_steps(d_keys, 0, D, Q, B, L, hot, parts, st);
 }
 
 }  // namespace qsb
