@@ -582,7 +582,7 @@ __device__ __forceinline__ ApShared ap_carve(uint8_t* p, uint32_t shift, uint32_
     S.tab = reinterpret_cast<uint32_t*>(p);
     p += pb * 32;
     S.mk = reinterpret_cast<uint32_t*>(p);
-    p += (size_t)((n_masks + 1) & ~1u) * 4;  // what follows stays 8-byte aligned (replay_few uses the run map's memory)
+    p += (size_t)((n_masks + 1) & ~1u) * 4;  // what follows stays 8-byte aligned (replay_warp uses the run map's memory)
     S.acc = reinterpret_cast<uint32_t*>(p);
     p += ap_accs(shift) * ACC_WORDS * 4;
     S.accid = reinterpret_cast<uint32_t*>(p);
@@ -757,7 +757,7 @@ __device__ __forceinline__ void part_write_low(uint32_t* bw, uint32_t cur) {
     if (lane < 7) bw[lane] = word;
 }
 
-// Ascending sort of recs[0, K) (at most ap_recs) by the whole block: bitonic over the next power
+// Ascending sort of recs[0, K) (at most ap_unit) by the whole block: bitonic over the next power
 // of two, padded with all ones.
 __device__ __forceinline__ void block_sort(unsigned long long* recs, uint32_t K) {
     uint32_t N = 32;
@@ -1449,7 +1449,8 @@ static const void* split_of(bool small) {
 }
 static const void* split_fn(uint32_t tile, int hot, bool batch, bool table) {
     const bool small = tile == PART_TILE_SMALL;
-    if (batch) return hot ? split_of<HOT_CALL, true, false>(small) : split_of<HOT_NONE, true, false>(small);
+    if (batch)  // small tiles without, large ones with heavy keys
+        return small ? (const void*)k_part_split<512, 4, HOT_NONE, true, false> : (const void*)k_part_split<1024, 16, HOT_CALL, true, false>;
     if (table)
         return hot == HOT_OWN    ? split_of<HOT_OWN, false, true>(small)
                : hot == HOT_CALL ? split_of<HOT_CALL, false, true>(small)
