@@ -253,7 +253,7 @@ void count_seen(qs_sketch* sk, uint64_t n, bool cleared, cudaStream_t st) {
 qs_status clear_msws(qs_sketch* sk, const BatchDev& B, cudaStream_t st) {
     count_seen(sk, 0, true, st);
     sk->fresh = 0;
-    CK(msws_clear(sk->D, ctl_init(), B, sk->L.num_sms, st), "clear");
+    CK(msws_clear(sk->D, ctl_init(), B, st), "clear");
     return QS_OK;
 }
 

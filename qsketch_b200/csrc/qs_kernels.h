@@ -41,7 +41,7 @@ cudaError_t msws_query(const uint32_t* d_keys, uint64_t n, uint32_t* d_out, cons
                        cudaStream_t st);
 
 // Empty tables, `init` as the control block and (n_streams > 0) the batch's allocators reset.
-cudaError_t msws_clear(const MswsDev& D, const Ctl& init, const BatchDev& B, int num_sms, cudaStream_t st);
+cudaError_t msws_clear(const MswsDev& D, const Ctl& init, const BatchDev& B, cudaStream_t st);
 // Few keys (qs_small.cu): one block, start to end; a batch's slices of at most SMALL_STREAM keys (their
 // bounds from batch_plan), a block each.
 cudaError_t small_insert(const uint32_t* d_keys, uint64_t n, const MswsDev& D, cudaStream_t st);
