@@ -77,7 +77,8 @@ CONFIGS = {
     "zipf_prof": dict(workload="zipf1.1_2^25keys_2^22ranks_low16MB_high4MB_query2^22", kind=1, n_keys=1 << 25,
                       n_ranks=1 << 22, s=1.1, n_low=524287, n_high=1 << 15, n_query=1 << 22),
 }
-INSERT_BYTES_PER_KEY = 68  # 4 B key + 32 B bucket sector read + 32 B write-back
+INSERT_BYTES_PER_KEY = 68  # pass 1: 4 B key + 32 B bucket sector read + 32 B write-back
+PART_BYTES_PER_KEY = 16    # partitioned: 4 B key + its 6 B entry written and read (the table streams once a chunk)
 L2_BYTES = 126 << 20      # B200 L2: tables above this live in HBM
 QUERY_BYTES_PER_KEY = 40   # 4 B key + 32 B bucket sector + 4 B result
 
@@ -382,7 +383,10 @@ def run_ours(args, cfg):
     prof = sk.profile()
     sk.set_profiling(False)
     hbm, peak_kind = peaks()
-    kern = {"insert": (prof["insert_ms"], prof["insert_timed"], n_ins, INSERT_BYTES_PER_KEY),
+    # large calls with default knobs are partitioned: no replay launches
+    parted = prof["repair_launches"] == 0
+    insert_bytes = PART_BYTES_PER_KEY if parted else INSERT_BYTES_PER_KEY
+    kern = {"insert": (prof["insert_ms"], prof["insert_timed"], n_ins, insert_bytes),
             "query": (prof["query_ms"], prof["query_timed"], n_q, QUERY_BYTES_PER_KEY)}
     dom = max(kern, key=lambda k: kern[k][0])
     ms_k, launches_k, units, bpu = kern[dom]
@@ -398,18 +402,18 @@ def run_ours(args, cfg):
         q_ms = prof["query_ms"]
     insert_step_ms = prof["insert_ms"] + prof["repair_ms"]  # pass 1 + ordered replay of the step
     keys_per_s = n_ins / (insert_step_ms * 1e-3)
-    # large calls with default knobs are partitioned: no replay launches
-    parted = prof["repair_launches"] == 0
     ins_kernel = "k_part_split + k_part_apply + k_part_link" if parted else "k_msws_insert"
     hbm_line = {"bound": "hbm", "kernel": ins_kernel if dom == "insert" else "k_msws_query",
                 "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
                 "traffic": dram_per_key * per_launch_units if dram_per_key else None, "peak_source": peak_kind,
                 "bytes_per_unit": bpu, "units_per_launch": per_launch_units, "avg_launch_ms": round(avg_ms, 5)}
-    if table_bytes > L2_BYTES:  # the tables live in HBM: bucket sectors cost DRAM traffic
+    if parted:  # counters live in shared memory: no L2 atomics, and far from DRAM
+        roofline = dict(hbm_line, note="against DRAM; the kernels are bound by instruction issue and the shared-memory "
+                                       "pipe, each about half busy between block barriers (profiles/k_part_insert_2^24.md)")
+    elif table_bytes > L2_BYTES:  # the tables live in HBM: bucket sectors cost DRAM traffic
         roofline = hbm_line
     else:  # L2-resident tables: the L2's atomic units bound the insert
         roofline = l2_atomic_roofline(probes, keys_per_s, MSWS_WORD_OPS_PER_KEY,
-                                      ins_kernel if parted else
                                       "k_msws_insert + k_msws_repair (pass 1 + ordered replay)",
                                       "each key adds 1 to 3 of its bucket's 28 packed 8-bit counters: "
                                       f"{MSWS_WORD_OPS_PER_KEY:.4f} 32-bit words on average (the expected number "
@@ -466,7 +470,7 @@ def run_ours(args, cfg):
             "insert_gkeys_per_s": round(world * n_ins / (ins_ms * 1e6), 4),
             "query_gkeys_per_s": round(world * n_q / (q_ms * 1e6), 4),
             "avg_rel_error": rel, "mean_est_over_exact": ratio,
-            "hbm_gbs_algorithmic": round((n_ins * INSERT_BYTES_PER_KEY + n_q * QUERY_BYTES_PER_KEY) /
+            "hbm_gbs_algorithmic": round((n_ins * insert_bytes + n_q * QUERY_BYTES_PER_KEY) /
                                          (ms_per_step * 1e-3) / 1e9, 1),
             "e2e": {"value": round(world * (n_ins + n_q) / (e2e_ms * 1e6), 4), "unit": "Gkeys/s",
                     "h2d_bytes_per_step": (n_ins + n_q) * 4, "d2h_bytes_per_step": n_q * 4,
@@ -474,7 +478,8 @@ def run_ours(args, cfg):
             "gpu_launches": int(launches),
             "roofline": roofline,
             "hbm_roofline": hbm_line,
-            "pass1_atomic_roofline": {"kernel": ins_kernel + " alone", "achieved_gsectors": round(ins_rate / 1e9, 3),
+            "pass1_atomic_roofline": None if parted else {
+                                      "kernel": ins_kernel + " alone", "achieved_gsectors": round(ins_rate / 1e9, 3),
                                       "peak_gsectors": round(atomic_peak / 1e9, 3) if atomic_peak else None,
                                       "frac": round(ins_rate / atomic_peak, 4) if atomic_peak else None,
                                       "probe": "random 32 B sectors, 3 red.add.u32 words per sector, sub-warp "
@@ -892,7 +897,7 @@ def run_learned(args, cfg):
     lo.close()
 
     rest_keys = n - warm
-    achieved = rest_keys * INSERT_BYTES_PER_KEY / (rest_ms * 1e-3) / 1e9
+    achieved = rest_keys * PART_BYTES_PER_KEY / (rest_ms * 1e-3) / 1e9
     hbm, peak_kind = peaks()
     if rank == 0:
         line = {
@@ -929,7 +934,7 @@ def run_learned(args, cfg):
             "roofline": {"bound": "hbm", "kernel": "routed insert (k_route, k_part_split + k_part_apply + k_part_link)",
                          "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                          "frac": round(achieved / hbm, 4), "traffic": None, "peak_source": peak_kind,
-                         "bytes_per_unit": INSERT_BYTES_PER_KEY, "units": rest_keys},
+                         "bytes_per_unit": PART_BYTES_PER_KEY, "units": rest_keys},
             "clocks": clk.summary(),
         }
         print(json.dumps(line), flush=True)
@@ -1011,7 +1016,7 @@ def run_batched(args, cfg):
     hbm, peak_kind = peaks()
     avg_ins = prof["insert_ms"] / max(1, prof["insert_timed"])
     per_launch = total / max(1, prof["insert_timed"])
-    achieved = per_launch * INSERT_BYTES_PER_KEY / (avg_ins * 1e-3) / 1e9
+    achieved = per_launch * PART_BYTES_PER_KEY / (avg_ins * 1e-3) / 1e9
 
     # the same streams through separate sketches, one call after another (one pass)
     alone = [qs.Sketch_GPU_Sub_Warp_Level(int(w["n_low"][s]), 8, int(w["n_high"][s]), 32,
@@ -1109,9 +1114,11 @@ def run_batched(args, cfg):
                     "h2d_bytes_per_step": total * 4 + (S + 1) * 8, "d2h_bytes_per_step": total * 4,
                     "ms_per_step": round(e2e_ms, 3), "api": "qs_batch_insert + qs_batch_query"},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "hbm", "kernel": "k_part_split + k_part_apply + k_part_link (dense streams), k_batch_insert (the rest)", "achieved": round(achieved, 1), "peak": hbm,
+            "roofline": {"bound": "hbm",
+                         "kernel": "k_part_split + k_part_apply + k_part_link (dense streams), k_batch_insert (the rest)",
+                         "achieved": round(achieved, 1), "peak": hbm,
                          "unit": "GB/s", "frac": round(achieved / hbm, 4), "traffic": None,
-                         "peak_source": peak_kind, "bytes_per_unit": INSERT_BYTES_PER_KEY,
+                         "peak_source": peak_kind, "bytes_per_unit": PART_BYTES_PER_KEY,
                          "units_per_launch": per_launch, "avg_launch_ms": round(avg_ins, 5)},
             "kernel_ms_per_step": {"insert": round(prof["insert_ms"], 4), "repair": round(prof["repair_ms"], 4),
                                    "query": round(prof["query_ms"], 4)},
