@@ -1680,18 +1680,19 @@ template <bool WIDE>
 __global__ void __launch_bounds__(QRY_THREADS) k_msws_query(const uint32_t* __restrict__ keys, uint64_t n,
                                                             uint32_t* __restrict__ out, MswsDev D) {
     extern __shared__ __align__(16) uint32_t s_codes[];
-    griddep_wait();  // the previous kernel (an insert or its replay) has ended
+    // No kernel writes the codes, and between queries of a table beyond the L2 they are evicted: they
+    // are read while the previous kernel (an insert or its replay) ends.
+    stage_codes<WIDE>(D, s_codes);
+    griddep_wait();
     griddep_launch_dependents();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t base = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t k[QRY_KPT], r[QRY_KPT];
-    // the first keys are loaded while the mask table is staged
 #pragma unroll
     for (int j = 0; j < QRY_KPT; ++j) {
         const uint64_t i = base + j * stride;
         k[j] = i < n ? __ldcs(keys + i) : 0u;
     }
-    stage_codes<WIDE>(D, s_codes);
     __syncthreads();
     for (; base < n; base += stride * QRY_KPT) {
         if (base != (uint64_t)blockIdx.x * blockDim.x + threadIdx.x) {
