@@ -1892,20 +1892,23 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
     auto cut = [&](uint64_t len, uint64_t rel, uint64_t tail) {  // as k_part_plan
         return rel && len - std::min(len, rel) <= tail ? len : std::min(len, rel);
     };
-    auto parts_of = [&](uint32_t i, uint64_t part) -> uint64_t {
-        return part ? batch_parts(batch_shift(b->part_shift[i], b->n_low[i], part), b->n_low[i]) : 0;
+    auto parts_of = [&](uint32_t i, uint64_t part, bool coarse) -> uint64_t {
+        return part ? batch_parts(batch_shift(b->part_shift[i], b->n_low[i], part, coarse), b->n_low[i]) : 0;
     };
     auto length = [&](uint32_t i) -> uint64_t { return dense[i] ? off[i + 1] - off[i] : 0; };
     // one window: the streams [s_lo, s_hi), each stream's keys [r0, r1)
     auto run = [&](uint32_t s_lo, uint32_t s_hi, uint64_t r0, uint64_t r1, uint64_t tail, bool hot) -> qs_status {
         const uint64_t tile = hot ? PART_TILE : PART_TILE_SMALL;
-        uint64_t tiles = 0, parts = 0;
+        uint64_t tiles = 0, fine = 0, coarse = 0;
         for (uint32_t i = s_lo; i < s_hi; ++i) {
             const uint64_t part = cut(length(i), r1, tail) - cut(length(i), r0, tail);
             tiles += (part + tile - 1) / tile;
-            parts += parts_of(i, part);
+            fine += parts_of(i, part, false);
+            coarse += parts_of(i, part, true);
         }
         BatchWindow W{};
+        W.coarse = fine > BATCH_PARTS;
+        const uint64_t parts = W.coarse ? coarse : fine;
         W.s_lo = s_lo;
         W.s_hi = s_hi;
         W.rel_lo = r0;
@@ -1938,7 +1941,7 @@ qs_status batch_insert_dense(qs_batch* b, const uint32_t* d_keys, const uint64_t
             return s;
         };
         for (uint32_t i = 0; i < b->S; ++i) {
-            const uint64_t len = length(i), part = cut(len, r1, fold) - cut(len, r0, fold), parts = parts_of(i, part);
+            const uint64_t len = length(i), part = cut(len, r1, fold) - cut(len, r0, fold), parts = parts_of(i, part, false);
             if (part > sk->part_cap) {  // one stream's rest alone exceeds a window: split it
                 qs_status s = close(i);
                 if (s != QS_OK) return s;
@@ -2119,7 +2122,7 @@ qs_status qs_batch_create(const qs_batch_params* p, qs_batch** out) {
             b->n_low[i] = (uint32_t)p->n_low[i];
             b->part_shift[i] = sh;
             b->parts[i] = desc[i].parts;
-            for (uint32_t x = sh; desc[i].parts && x <= batch_shift(sh, b->n_low[i], 0); ++x)  // (units halve with shift)
+            for (uint32_t x = sh; desc[i].parts && x <= batch_shift(sh, b->n_low[i], 0, true); ++x)  // (units halve with shift)
                 smem = std::max(smem, part_apply_smem(x, p->hash_mask_table_sz));
         }
         sk->PL.apply_smem = smem;

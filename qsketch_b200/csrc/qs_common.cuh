@@ -210,6 +210,7 @@ struct BatchWindow {
     uint32_t flat;
     uint64_t fold;   // dense streams: one with at most this many keys from rel_hi on has them in the window
                      // that ends at rel_hi, and none in the one that begins there
+    uint32_t coarse; // dense streams: partitions of at least about 2,048 keys (batch_shift)
     uint32_t which;  // all streams, or only the dense or the sparse ones (batch_dense), or (flat)
                      // work items only for the slices of more than SMALL_STREAM keys
 };
@@ -217,12 +218,14 @@ enum { STREAMS_ALL = 0, STREAMS_DENSE = 1, STREAMS_SPARSE = 2, STREAMS_LONG = 3 
 // Keys of a stream in one call that one block takes by itself (k_msws_small).
 constexpr uint64_t SMALL_STREAM = 4096;
 // Buckets of a partition of such a stream, of `keys` keys in the window, as a shift: as many as it takes
-// for 2,048 keys to a partition, down to eight of them.  A block per partition is 20 to 30 ns of the
+// for 2,048 keys to a partition, down to eight of them, in windows of more than BATCH_PARTS partitions (few
+// would leave the chip idle: 44 streams of up to 84,000 keys 409 -> 423 us).  A block per partition is 20 to 30 ns of the
 // chip, whatever its keys: 512 streams of 33,000 keys, 1,024 to 8,192 buckets, cleared / warm, in 32 to 64
 // partitions each 0.89 / 0.96 ms uniform and 1.60 / 1.13 Zipf 1.2; so 0.54 / 0.58 and 1.51 / 0.71 (pass 1
 // 0.64 / 0.94 and 1.23 / 0.88).
-__host__ __device__ __forceinline__ uint32_t batch_shift(uint32_t shift, uint32_t n_low, uint64_t keys) {
-    while (shift < PART_MAX_SHIFT && (n_low >> shift) > 8 && (n_low >> shift) > (keys >> 11)) ++shift;
+constexpr uint64_t BATCH_PARTS = 2560;  // eight or nine waves of blocks
+__host__ __device__ __forceinline__ uint32_t batch_shift(uint32_t shift, uint32_t n_low, uint64_t keys, bool coarse) {
+    while (coarse && shift < PART_MAX_SHIFT && (n_low >> shift) > 8 && (n_low >> shift) > (keys >> 11)) ++shift;
     return shift;
 }
 __host__ __device__ __forceinline__ uint32_t batch_parts(uint32_t shift, uint32_t n_low) {

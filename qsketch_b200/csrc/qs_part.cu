@@ -134,7 +134,7 @@ __device__ __forceinline__ PartView part_view(const MswsDev& D, const PartDev& Q
     const StreamDesc* sd = B.desc + s;
     V.fm = FastMod{__ldg(&sd->fm_low.M), __ldg(&sd->fm_low.d)};
     V.seed = __ldg(&sd->seed), V.low_base = __ldg(&sd->low_base);
-    V.shift = __ldcg(B.part_shift + s), V.parts = batch_parts(V.shift, V.fm.d);
+    V.shift = __ldg(B.part_shift + s), V.parts = batch_parts(V.shift, V.fm.d);
     V.tile0 = __ldcg(B.item_off + s), V.tiles = __ldcg(B.item_off + s + 1) - V.tile0;
     V.off = Q.off + __ldcg(B.run_off + s), V.stride = V.tiles;
     return V;
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(1024) k_part_plan(BatchDev B, BatchWindow W, u
         B.lo[s] = lo;
         B.hi[s] = hi;
         B.item_off[s] = t;
-        const uint32_t n_low = B.desc[s].fm_low.d, shift = batch_shift(B.desc[s].shift, n_low, hi - lo);
+        const uint32_t n_low = B.desc[s].fm_low.d, shift = batch_shift(B.desc[s].shift, n_low, hi - lo, W.coarse);
         const uint32_t parts = t ? batch_parts(shift, n_low) : 0u;
         B.part_shift[s] = shift;
         B.part_off[s] = parts;
@@ -947,7 +947,8 @@ __device__ __forceinline__ bool replay_warp(const MswsDev& D, const PartDev& Q, 
     return true;
 }
 
-// The partition `p` (batch: of the window's) that a block works on.
+// The partition `p` (batch: of the window's) that a block works on.  (The plan wrote the offsets in an
+// earlier kernel: the search goes through the L1.)
 template <bool BATCH>
 __device__ __forceinline__ PartView part_of_block(const MswsDev& D, const PartDev& Q, const BatchDev& B, uint32_t& p,
                                                   uint32_t& stream) {
@@ -956,11 +957,11 @@ __device__ __forceinline__ PartView part_of_block(const MswsDev& D, const PartDe
         uint32_t lo = 0, hi = B.n_streams;  // part_off[lo] <= p < part_off[hi]: the last such lo has partitions
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (__ldcg(B.part_off + mid) <= p) lo = mid;
+            if (__ldg(B.part_off + mid) <= p) lo = mid;
             else hi = mid;
         }
         stream = lo;
-        p -= __ldcg(B.part_off + lo);
+        p -= __ldg(B.part_off + lo);
     }
     return part_view<BATCH>(D, Q, B, stream);
 }
