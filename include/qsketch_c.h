@@ -102,9 +102,9 @@ typedef struct qs_params {
     int32_t device;              /* CUDA device ordinal; -1 = current */
     /* Insert-kernel knobs; none changes any result.  They shape pass 1, which takes the calls
      * that are small against the table.  With all of them (and QS_FLAG_NO_CHUNK_RAMP) left at 0,
-     * calls of at least max(2^18, 1.5 n_low) keys are partitioned by bucket range and applied in
-     * shared memory instead, in chunks of up to 4 * max_batch keys, and calls of at most 4096
-     * keys run in one kernel of one block.  When lanes_per_key, aggregate, route and ctas_per_sm
+     * calls of at least max(2^18, 1.5 n_low) keys into tables of about 500 to 2^22 buckets are
+     * partitioned by bucket range and applied in shared memory instead, in chunks of up to
+     * 4 * max_batch keys, and calls of at most 4096 keys run in one kernel of one block.  When lanes_per_key, aggregate, route and ctas_per_sm
      * are all 0, qs_create takes them (and max_batch, if 0) from the autotuner's entry for the
      * sketch's size class (qs_autotune), else the defaults 4 / 3 / 1 / 0. */
     uint32_t lanes_per_key;      /* lanes serving one key in pass 1: 1, 2, 4, 8 (one lane
