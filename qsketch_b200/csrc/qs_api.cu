@@ -565,7 +565,7 @@ static qs_status create_sketch(const qs_params* params, qs_sketch** out, bool pa
         // partitioned chunk's entries and key indices (6 B a key); every partitioned chunk or
         // window of this sketch, or of the batch whose arena it is, goes by part_cap
         sk->part_cap = PB >= PART_TILE ? std::min<uint64_t>(PB * 4, PART_MAX_CHUNK) / PART_TILE * PART_TILE : 0;
-        const uint64_t record_words = std::max(B * 6, (sk->part_cap * 6 + 3) / 4);
+        const uint64_t record_words = P.parts || part_arena ? std::max(B * 6, (sk->part_cap * 6 + 3) / 4) : B * 6;
         // A partitioned chunk streams the whole table through shared memory (64 MB: 45 us), pass 1
         // touches the buckets of its keys only.  Per call, measured: 2^18 Zipf 1.1 keys into a 4 MB
         // table 48 us against 80 (uniform 22 against 19), 2^20 117 against 137 (38 / 45), 2^22 136
